@@ -365,7 +365,7 @@ def work(case):
         return {"bytes": b, "flops": f}
     if kind == "cg":
         # about this many steps at this mass and tolerance; each is M^dag M and the vector updates
-        steps = 130 if case["system"] == "eo" else 330
+        steps = 200 if case["system"] == "eo" else 340
         inner = "f32" if case["inner"] == "plain" else case["inner"]
         hb, hf = _hop_work(inner, V, Ls)
         vec = 5 * 192 if case["inner"] == "plain" else 2 * 96 + 4 * SPINOR[inner]
