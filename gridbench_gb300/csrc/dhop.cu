@@ -53,6 +53,18 @@ bool blocked_ok(const gbdw_lattice* lat, const gbdw_field* in) {
   return true;
 }
 
+int sweep_extent(const gbdw_gauge* g, const gbdw_field* in, int epi, int spt) {
+  const gbdw_lattice* lat = g->lat;
+  if (in->prec != GBDW_F32 || g->prec != GBDW_F32 || spt != 2 || in->LsE != in->LsP || !lat->fast) return 0;
+  const int* d = lat->parity >= 0 ? lat->parent->dims : lat->dims;
+  for (int k = 0; k < 3; ++k)
+    if (d[k] <= 0 || d[k] % (k == 0 && lat->parity >= 0 ? 4 : 2)) return 0;
+  if (d[3] <= 0) return 0;
+  for (int te : {16, 12, 8})
+    if (epi ? in->LsE == te && in->nrhs == 1 : in->LsE % te == 0) return te;
+  return 0;
+}
+
 int tile_extent(int LsE, const DhopLaunch& L, bool whole_sites) {
   if (L.split <= 1 || whole_sites || (L.mode != 0 && L.mode != 3) || LsE % L.split) return 0;
   const int TE = LsE / L.split;
@@ -162,6 +174,11 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
   const bool staged = L.mode == 1 || L.mode == 2;
   if (staged && !tma_shape(in->prec, in->LsE, L, &NS, &tthreads, &smem)) L.mode = 0;
   // fall back before fixing the CTA size: the block count below must match the launch
+  const int sweep = L.mode == 5 ? sweep_extent(g, in, epi, L.spt) : 0;
+  if (L.mode == 5 && (!sweep || (p.mob && (sweep == 12 || (epi == 6 && g->lat->parity >= 0))))) {
+    L.mode = 3;
+    L.brick = 1;
+  }
   if (L.mode == 4 && !blocked_ok(g->lat, in)) L.mode = 3;
   if (L.mode == 3 && !form3_ok(in, epi, L.spt)) L.mode = 0;
   if (L.mode == 3) L.threads = 64;
@@ -169,7 +186,21 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
   p.TE = tile_extent(in->LsE, L, p.mob != 0);
   p.brick = brick_extent(g->lat, L);
   const int64_t nthreads = p.nsite * (p.LsE / L.spt);
-  const int64_t blocks = staged ? (p.nsite + NS - 1) / NS : (nthreads + L.threads - 1) / L.threads;
+  int64_t blocks = staged ? (p.nsite + NS - 1) / NS : (nthreads + L.threads - 1) / L.threads;
+  SweepParams sw;
+  if (L.mode == 5) {
+    const gbdw_lattice* lat = g->lat;
+    const int* d = lat->parity >= 0 ? lat->parent->dims : lat->dims;
+    for (int k = 0; k < 4; ++k) sw.L[k] = d[k];
+    if (lat->parity >= 0) sw.L[0] /= 2;
+    sw.parity = lat->parity;
+    sw.nbx = sw.L[0] / 2;
+    sw.nby = sw.L[1] / 2;
+    sw.nbz = sw.L[2] / 2;
+    sw.ntile = p.LsE / sweep;
+    sw.nt = L.brick > 1 ? L.brick : 8;
+    blocks = int64_t(sw.nbx) * sw.nby * sw.nbz * sw.ntile * ((sw.L[3] + sw.nt - 1) / sw.nt);
+  }
   Reduce red;
   const bool reduce = norm2 || (ex && ex->sum_to);
   if (reduce) {
@@ -204,6 +235,8 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
     return GBDW_OK;
   }
   if (in->prec == GBDW_F64) st = launch_dhop_f64(p, dag, epi, L);
+  else if (L.mode == 5)
+    st = (sweep == 16 ? launch_dhop_sweep16 : sweep == 12 ? launch_dhop_sweep12 : launch_dhop_sweep8)(p, sw, unsigned(blocks), dag, epi);
   else if (in->prec == GBDW_F32) st = launch_dhop_f32(p, dag, epi, L);
   else st = launch_dhop_f16(p, g->prec, dag, epi, L);
   if (st) return st;
@@ -223,7 +256,7 @@ bool tma_shape(int prec, int LsE, DhopLaunch L, int* NS, int* threads, size_t* s
   const size_t esz = spinor_elem_bytes(prec);
   const size_t blk = 12 * size_t(padded_slices(prec, LsE)) * esz + (prec == GBDW_F16 ? 4 * size_t(LsE) : 0);
   const size_t lb = 8 * link_bytes(prec);
-  if (L.mode == 3 || L.mode == 4) return false;  // direct forms: no staging shape
+  if (L.mode >= 3) return false;  // direct forms and the t-sweep: no staging shape
   if (L.mode == 2) {
     // one ring per warp: a warp owns 32/Tps whole sites
     if (Tps > 32 || L.threads % 32 != 0 || L.threads > 256) return false;

@@ -870,15 +870,30 @@ struct DhopLaunch {
   int mode = 0;    // 0: direct loads, 1: TMA-staged (CTA ring), 2: TMA-staged (one ring per warp),
                    // 3: direct, FP32/FP16 Ls = 16 at compile time, registers balanced for 6 CTAs/SM
                    // 4: form 3 on 2x2x2x2 site blocks per 128-thread CTA (periodic, even extents)
+                   // 5: t-sweep over 2x2x2 columns (FP32, periodic, even x, y and z); brick = slices of t
+                   //    per CTA
   int stages = 4;  // staged kernels: depth of the leg ring
   int split = 1;   // forms 0 and 3: each site's Ls*nrhs slices cut into this many tiles
   int brick = 1;   // forms 0 and 3 on periodic lattices: t-brick sweep order (1: natural order)
+};
+
+// The t-sweep form's geometry (dhop_sweep.cuh).
+struct SweepParams {
+  int L[4];          // extents in site-index space (x halved on a half lattice)
+  int parity;        // parity of the output half lattice, -1 on a full lattice
+  int nbx, nby, nbz; // column blocks per direction
+  int ntile;         // slice tiles per site
+  int nt;            // t-slices per CTA
 };
 
 // Implemented per precision family in dhop_f64.cu / dhop_f32.cu / dhop_f16.cu.
 int launch_dhop_f64(const DhopParams& p, int dag, int epi, DhopLaunch L);
 int launch_dhop_f32(const DhopParams& p, int dag, int epi, DhopLaunch L);
 int launch_dhop_f16(const DhopParams& p, int gprec, int dag, int epi, DhopLaunch L);
+int launch_dhop_bf16(const DhopParams& p, int dag, int epi, DhopLaunch L);
+int launch_dhop_sweep8(const DhopParams& p, const SweepParams& q, unsigned blocks, int dag, int epi);
+int launch_dhop_sweep12(const DhopParams& p, const SweepParams& q, unsigned blocks, int dag, int epi);
+int launch_dhop_sweep16(const DhopParams& p, const SweepParams& q, unsigned blocks, int dag, int epi);
 int launch_dhop_general(const DhopParams& p, int prec, int dag);
 // The double-single form of the FP64 operator (dhop_ds.cu): direct loads, one slice per thread in
 // CTAs of DS_THREADS with registers capped for minb (3 or 4) CTAs per SM, Dhop and M; p.U must be

@@ -149,6 +149,11 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
       }
   }
   if (blocked_ok(g->lat, in)) cands.push_back(DhopLaunch{128, 2, 4, 4});
+  // the t-sweep with 4, 8 or 16 slices of t per CTA: more slices reread fewer planes, fewer fill the
+  // last wave better (measured best 4 to 8 on lattices from 16^4 to 32^4)
+  if (sweep_extent(g, in, 0, 2))
+    for (int nt : {4, 8, 16})
+      if (nt <= 4 || nt <= (g->lat->parity >= 0 ? g->lat->parent : g->lat)->dims[3]) cands.push_back(DhopLaunch{64, 2, 5, 4, 1, nt});
   // FP64 fields whose operator calls run the double-single form (gbdw_set_fp64_arith): only that
   // form's shapes are timed
   const bool ds_only = in->prec == GBDW_F64 && g->prec == GBDW_F64 && !eo && fp64_double_single();
@@ -259,9 +264,9 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
       shortlist.push_back(L);
     };
     for (size_t i = 0; i < m_times.size() && i < 4; ++i) add(m_times[i].second);
-    for (int form = 0; form <= 4; ++form)
+    for (int form = 0; form <= 5; ++form)
       for (const auto& mt : m_times)
-        if (mt.second.mode == form && mt.second.split == 1 && mt.second.brick == 1) {
+        if (mt.second.mode == form && mt.second.split == 1 && (mt.second.brick == 1 || form == 5)) {
           add(mt.second);
           break;
         }
@@ -465,7 +470,7 @@ int gbdw_tune_load(const char* path) {
     if (lb == std::string::npos) break;
     if (sscanf(key.c_str(), "g%d_s%d_L%d_e%d", &gp, &sp, &LsE, &epi) == 4 &&
         sscanf(text.c_str() + lb, "[%d , %d , %d , %d , %d , %d]", &th, &spt, &mode, &stages, &split, &brick) >= 2 &&
-        th > 0 && th <= 256 && th % 32 == 0 && (spt == 1 || spt == 2 || spt == 4) && mode >= 0 && mode <= 4 &&
+        th > 0 && th <= 256 && th % 32 == 0 && (spt == 1 || spt == 2 || spt == 4) && mode >= 0 && mode <= 5 &&
         // the double-single keys hold their register cap (CTAs per SM, 3 or 4) in `stages`
         (stages == 2 || stages == 4 || (epi >= DS_KEY && stages == 3)) && split >= 1 && split <= 64 && brick >= 1 &&
         brick <= 64) {
