@@ -47,7 +47,7 @@ bool form3_ok(const gbdw_field* in, int epi, int spt) {
 }
 
 bool blocked_ok(const gbdw_lattice* lat, const gbdw_field* in) {
-  if (in->prec == GBDW_F64 || in->LsE != 16 || in->LsP != 16 || lat->parity >= 0 || !lat->fast) return false;
+  if (in->prec != GBDW_F16 || in->LsE != 16 || in->LsP != 16 || lat->parity >= 0 || !lat->fast) return false;
   for (int d = 0; d < 4; ++d)
     if (lat->dims[d] <= 0 || lat->dims[d] % 2) return false;
   return true;
@@ -174,12 +174,13 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
   const bool staged = L.mode == 1 || L.mode == 2;
   if (staged && !tma_shape(in->prec, in->LsE, L, &NS, &tthreads, &smem)) L.mode = 0;
   // fall back before fixing the CTA size: the block count below must match the launch
-  const int sweep = L.mode == 5 ? sweep_extent(g, in, epi, L.spt) : 0;
-  if (L.mode == 5 && (!sweep || (p.mob && (sweep == 12 || (epi == 6 && g->lat->parity >= 0))))) {
+  // form 4: the t-sweep for FP32, the 2x2x2x2 blocks for FP16
+  int sweep = L.mode == 4 && in->prec == GBDW_F32 ? sweep_extent(g, in, epi, L.spt) : 0;
+  if (p.mob && (sweep == 12 || (epi == 6 && g->lat->parity >= 0))) sweep = 0;
+  if (L.mode == 4 && !sweep && (in->prec == GBDW_F32 || !blocked_ok(g->lat, in))) {
     L.mode = 3;
-    L.brick = 1;
+    L.brick = 1;  // a sweep's brick is its slices of t
   }
-  if (L.mode == 4 && !blocked_ok(g->lat, in)) L.mode = 3;
   if (L.mode == 3 && !form3_ok(in, epi, L.spt)) L.mode = 0;
   if (L.mode == 3) L.threads = 64;
   if (L.mode == 4) L.threads = 128;
@@ -188,7 +189,7 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
   const int64_t nthreads = p.nsite * (p.LsE / L.spt);
   int64_t blocks = staged ? (p.nsite + NS - 1) / NS : (nthreads + L.threads - 1) / L.threads;
   SweepParams sw;
-  if (L.mode == 5) {
+  if (sweep) {
     const gbdw_lattice* lat = g->lat;
     const int* d = lat->parity >= 0 ? lat->parent->dims : lat->dims;
     for (int k = 0; k < 4; ++k) sw.L[k] = d[k];
@@ -235,7 +236,7 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
     return GBDW_OK;
   }
   if (in->prec == GBDW_F64) st = launch_dhop_f64(p, dag, epi, L);
-  else if (L.mode == 5)
+  else if (sweep)
     st = (sweep == 16 ? launch_dhop_sweep16 : sweep == 12 ? launch_dhop_sweep12 : launch_dhop_sweep8)(p, sw, unsigned(blocks), dag, epi);
   else if (in->prec == GBDW_F32) st = launch_dhop_f32(p, dag, epi, L);
   else st = launch_dhop_f16(p, g->prec, dag, epi, L);

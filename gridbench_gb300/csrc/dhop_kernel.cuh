@@ -577,19 +577,21 @@ __device__ __forceinline__ double sumsq(const cpx<dsf> (&v)[N][12]) {
 // out(s) = a5 psi(s) - k D(s) - [P+ psi(s+1) + P- psi(s-1)]       (dag = 1)
 // P+ keeps spins 0,1 and P- spins 2,3 (gamma5 = diag(1,1,-1,-1)); a step across the
 // s boundary picks up -mf.  k = p.khop (1/2 for M) and psi is p.cen when set, else the
-// hopping input.  Requires nrhs == 1 (LsE == Ls).
-template <int PIN, int DAG, int N, class T>
-__device__ __forceinline__ void dwf_epilogue(const DhopParams& p, int64_t site, int s0, cpx<T> (&acc)[N][12]) {
+// hopping input.  Requires nrhs == 1 (LsE == Ls).  SMEM: psi's rows of this site lie in shared memory
+// at `rows` (FP32, without norms).
+template <int PIN, int DAG, int N, bool SMEM = false, class T>
+__device__ __forceinline__ void dwf_epilogue(const DhopParams& p, int64_t site, int s0, cpx<T> (&acc)[N][12],
+                                             const void* rows = nullptr) {
   const int Ls = p.Ls;
   const int LsP = p.LsP;
-  const int64_t row0 = site * 12;
-  const void* cin = p.cen ? p.cen : p.in;
+  const int64_t row0 = SMEM ? 0 : site * 12;
+  const void* cin = SMEM ? rows : p.cen ? p.cen : p.in;
   const float* cnorm = p.cen ? p.cen_norm : p.in_norm;
   cpx<T> cen[N][12];
 #pragma unroll
   for (int k = 0; k < 12; ++k) {
     cpx<T> x[N];
-    Vec<PIN, N>::load(cin, row0 + k, s0, LsP, x);
+    Vec<PIN, N, SMEM>::load(cin, row0 + k, s0, LsP, x);
 #pragma unroll
     for (int j = 0; j < N; ++j) cen[j][k] = x[j];
   }
@@ -602,8 +604,8 @@ __device__ __forceinline__ void dwf_epilogue(const DhopParams& p, int64_t site, 
   cpx<T> lo[6], hi[6];
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
-    lo[k] = Elem<PIN>::ld(cin, row0 + LO0 * 3 + k, slo, LsP);
-    hi[k] = Elem<PIN>::ld(cin, row0 + HI0 * 3 + k, shi, LsP);
+    lo[k] = Vec<PIN, N, SMEM>::one(cin, row0 + LO0 * 3 + k, slo, 1, LsP);
+    hi[k] = Vec<PIN, N, SMEM>::one(cin, row0 + HI0 * 3 + k, shi, 0, LsP);
   }
   T nlo = flo, nhi = fhi;
   if constexpr (PIN == GBDW_F16) {
@@ -684,13 +686,14 @@ __device__ __forceinline__ void mobius_adj_hop(const DhopParams& p, int s0, cpx<
 // FP16 (the CG residual update fused into the operator's second pass; M(in) is not stored);
 // EPI 6: store the Mobius M(in), A(b, c) applied to the neighbours as they are loaded.
 // Returns |what was stored|^2 in part (FP32 outputs) or dpart (FP64 outputs and EPI 2-4).
-template <int PIN, int POUT, int DAG, int N, int EPI, class T>
+template <int PIN, int POUT, int DAG, int N, int EPI, bool SMEM = false, class T>
 __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, int s0, int LsE, int LsP,
-                                            cpx<T> (&v)[N][12], float& part, double& dpart) {
+                                            cpx<T> (&v)[N][12], float& part, double& dpart,
+                                            const void* rows = nullptr) {
   if constexpr (EPI == 1 && DAG == 1 && N == 2 && PIN != GBDW_DS) {
     if (p.mob) mobius_adj_hop(p, s0, v);
   }
-  if constexpr (EPI >= 1) dwf_epilogue<PIN, DAG, N>(p, site, s0, v);
+  if constexpr (EPI >= 1) dwf_epilogue<PIN, DAG, N, SMEM>(p, site, s0, v, rows);
   if constexpr (EPI == 4) {
     // FP16 r: dequantise with its per-slice norms, update in FP32, store with new norms
     const float al = float(*p.alpha);
@@ -869,9 +872,9 @@ struct DhopLaunch {
   int spt;         // slices per thread
   int mode = 0;    // 0: direct loads, 1: TMA-staged (CTA ring), 2: TMA-staged (one ring per warp),
                    // 3: direct, FP32/FP16 Ls = 16 at compile time, registers balanced for 6 CTAs/SM
-                   // 4: form 3 on 2x2x2x2 site blocks per 128-thread CTA (periodic, even extents)
-                   // 5: t-sweep over 2x2x2 columns (FP32, periodic, even x, y and z); brick = slices of t
-                   //    per CTA
+                   // 4: site blocks on a periodic lattice: FP32 the t-sweep over 2x2x2 columns (even x,
+                   //    y and z; brick = slices of t per CTA), FP16 form 3 on 2x2x2x2 blocks per
+                   //    128-thread CTA (even extents)
   int stages = 4;  // staged kernels: depth of the leg ring
   int split = 1;   // forms 0 and 3: each site's Ls*nrhs slices cut into this many tiles
   int brick = 1;   // forms 0 and 3 on periodic lattices: t-brick sweep order (1: natural order)

@@ -106,7 +106,8 @@ int by_shape(const DhopParams& p, DhopLaunch L) {
       }
     }
   } else if (L.mode == 4) {
-    if constexpr (PIN == GBDW_F32 || PIN == GBDW_F16) {
+    // FP16 (FP32 runs the t-sweep there, dhop_sweep.cuh)
+    if constexpr (PIN == GBDW_F16) {
       if (L.spt == 2 && p.LsE == 16 && p.LsP == 16 && p.nsite % 16 == 0) {
         k_dhop<PIN, POUT, GP, DAG, 2, EPI, 3, 16, 128, 1><<<unsigned(p.nsite / 16), 128, 0, stream()>>>(p);
         GBDW_LAUNCHED();

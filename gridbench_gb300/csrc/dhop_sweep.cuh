@@ -1,4 +1,4 @@
-// The t-sweep form of the FP32 hopping kernel.
+// The t-sweep form of the FP32 hopping kernel (form 4).
 //
 // What bounds the other forms is the L2 -> SM path: each of a site's eight neighbour spinors comes
 // from L2, 834 MB per launch at 16^4 x 16 where DRAM moves 239 MB.  Here a CTA owns a column of
@@ -235,7 +235,11 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
       acc.unpack(v);
       float pt = 0.f;
       double dt = 0.0;
-      finish_site<GBDW_F32, GBDW_F32, DAG, 2, EPI>(p, int64_t(t) * vol3 + col, e0, p.LsE, p.LsP, v, pt, dt);
+      const int64_t site = int64_t(t) * vol3 + col;
+      if (!EO && EPI >= 1 && !p.cen)  // the diagonal part reads this site's plane t, in shared memory
+        finish_site<GBDW_F32, GBDW_F32, DAG, 2, EPI, !EO && EPI >= 1>(p, site, e0, p.LsE, p.LsP, v, pt, dt, sc - lg * 16);
+      else
+        finish_site<GBDW_F32, GBDW_F32, DAG, 2, EPI>(p, site, e0, p.LsE, p.LsP, v, pt, dt);
       part += pt;
       dpart += dt;
     }

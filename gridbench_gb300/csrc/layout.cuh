@@ -1,7 +1,8 @@
 // Spinor storage of the GB300 layout and its element access.
 //
 // A row is one spin-colour component of one 4D site: row = site*12 + sc, holding the
-// LsE = Ls*nrhs fifth-dimension slices (rhs innermost).
+// LsE = Ls*nrhs fifth-dimension slices, one right-hand side after the other (e = rhs*Ls + s), so that
+// importing or exporting one of them touches its own bytes only.
 //   F64     : double2 per slice; slice e at double2 index row*LsP + e (LsP = LsE).
 //   F32/F16 : slices grouped in pairs, each pair stored as (Re s, Re s+1, Im s, Im s+1);
 //             rows padded to an even slice count LsP.  Re of slice e sits at real index
@@ -120,6 +121,18 @@ struct Vec {
         v[2 * k] = {q[k].r.x, q[k].i.x};
         v[2 * k + 1] = {q[k].r.y, q[k].i.y};
       }
+    }
+  }
+  // Slice e alone, which is the `second` (or first) of its pair when a thread's slices come in pairs.
+  // From shared memory the pair is loaded whole, one access instead of two; from global memory, where
+  // the line is in L1, the wider access costs more (M at 16^4 x 16 in form 3: 64.3 -> 66.6 us).
+  __device__ static cpx<T> one(const void* b, int64_t row, int e, int second, int LsP) {
+    if constexpr (P == GBDW_F64 || P == GBDW_DS || N == 1 || !SMEM) {
+      return Elem<P>::template ld<SMEM>(b, row, e, LsP);
+    } else {
+      cp2 q[1];
+      Vec<P, 2, SMEM>::load_pairs(b, row, e - second, LsP, q);
+      return second ? cpx<T>{q[0].r.y, q[0].i.y} : cpx<T>{q[0].r.x, q[0].i.x};
     }
   }
   // F32/F16, N even: the pairs themselves

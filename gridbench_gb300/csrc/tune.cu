@@ -153,7 +153,7 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
   // last wave better (measured best 4 to 8 on lattices from 16^4 to 32^4)
   if (sweep_extent(g, in, 0, 2))
     for (int nt : {4, 8, 16})
-      if (nt <= 4 || nt <= (g->lat->parity >= 0 ? g->lat->parent : g->lat)->dims[3]) cands.push_back(DhopLaunch{64, 2, 5, 4, 1, nt});
+      if (nt <= 4 || nt <= (g->lat->parity >= 0 ? g->lat->parent : g->lat)->dims[3]) cands.push_back(DhopLaunch{64, 2, 4, 4, 1, nt});
   // FP64 fields whose operator calls run the double-single form (gbdw_set_fp64_arith): only that
   // form's shapes are timed
   const bool ds_only = in->prec == GBDW_F64 && g->prec == GBDW_F64 && !eo && fp64_double_single();
@@ -264,9 +264,9 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
       shortlist.push_back(L);
     };
     for (size_t i = 0; i < m_times.size() && i < 4; ++i) add(m_times[i].second);
-    for (int form = 0; form <= 5; ++form)
+    for (int form = 0; form <= 4; ++form)
       for (const auto& mt : m_times)
-        if (mt.second.mode == form && mt.second.split == 1 && (mt.second.brick == 1 || form == 5)) {
+        if (mt.second.mode == form && mt.second.split == 1 && (mt.second.brick == 1 || (form == 4 && in->prec == GBDW_F32))) {
           add(mt.second);
           break;
         }
@@ -369,9 +369,9 @@ int gbdw_tune_set(const gbdw_gauge* g, const gbdw_field* in, int threads, int sp
               "12 / 144 (FP32)");
     return GBDW_ERR_INVALID;
   }
-  if (form == 4 && (spt != 2 || !blocked_ok(g->lat, in))) {
-    set_error("gbdw_tune_set: form 4 needs FP32/FP16, Ls*nrhs = 16, 2 slices per thread and a periodic lattice "
-              "with even extents");
+  if (form == 4 && !(in->prec == GBDW_F32 ? sweep_extent(g, in, 0, spt) > 0 : spt == 2 && blocked_ok(g->lat, in))) {
+    set_error("gbdw_tune_set: form 4 needs 2 slices per thread and a periodic lattice: FP32 with Ls*nrhs a multiple "
+              "of 8 or 12 and even x, y and z, or FP16 with Ls*nrhs = 16 and even extents");
     return GBDW_ERR_INVALID;
   }
   if (form == 1 || form == 2) {
@@ -416,7 +416,7 @@ int gbdw_tune_set_brick(const gbdw_gauge* g, const gbdw_field* in, int brick) {
   if (!g || !in) return GBDW_ERR_INVALID;
   DhopLaunch L = lookup(g, in, 0);
   L.brick = brick;
-  if (brick < 1 || (brick > 1 && brick_extent(g->lat, L) == 0)) {
+  if (brick < 1 || (L.mode == 4 && in->prec == GBDW_F32 ? brick > 64 : brick > 1 && brick_extent(g->lat, L) == 0)) {
     set_error("gbdw_tune_set_brick: the chosen form must be direct (0 or 3) on a periodic lattice whose Lt the "
               "brick divides");
     return GBDW_ERR_INVALID;
@@ -470,7 +470,7 @@ int gbdw_tune_load(const char* path) {
     if (lb == std::string::npos) break;
     if (sscanf(key.c_str(), "g%d_s%d_L%d_e%d", &gp, &sp, &LsE, &epi) == 4 &&
         sscanf(text.c_str() + lb, "[%d , %d , %d , %d , %d , %d]", &th, &spt, &mode, &stages, &split, &brick) >= 2 &&
-        th > 0 && th <= 256 && th % 32 == 0 && (spt == 1 || spt == 2 || spt == 4) && mode >= 0 && mode <= 5 &&
+        th > 0 && th <= 256 && th % 32 == 0 && (spt == 1 || spt == 2 || spt == 4) && mode >= 0 && mode <= 4 &&
         // the double-single keys hold their register cap (CTAs per SM, 3 or 4) in `stages`
         (stages == 2 || stages == 4 || (epi >= DS_KEY && stages == 3)) && split >= 1 && split <= 64 && brick >= 1 &&
         brick <= 64) {

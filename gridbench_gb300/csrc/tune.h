@@ -43,9 +43,9 @@ DhopParams make_params(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* i
 // form 3 (specialised direct) applies: slice pairs, Ls*nrhs = 16 (FP32/FP16) or 12 / 144 (FP32
 // Dhop and M)
 bool form3_ok(const gbdw_field* in, int epi, int spt);
-// form 4 (blocked site order) applies: FP32/FP16, Ls*nrhs = 16, periodic lattice, even extents
+// form 4 for FP16 (blocked site order) applies: Ls*nrhs = 16, periodic lattice, even extents
 bool blocked_ok(const gbdw_lattice* lat, const gbdw_field* in);
-// form 5 (t-sweep over 2x2x2 columns) applies to these operands: slices per tile (16, 12 or 8; the
+// form 4 for FP32 (t-sweep over 2x2x2 columns) applies to these operands: slices per tile (16, 12 or 8; the
 // whole row for M and its variants), or 0
 int sweep_extent(const gbdw_gauge* g, const gbdw_field* in, int epi, int spt);
 // slices per tile of a direct launch with L.split tiles per site, or 0 (one tile: the split does

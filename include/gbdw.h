@@ -121,7 +121,7 @@ int gbdw_gauge_create(gbdw_gauge** g, const gbdw_lattice* lat, int prec, const v
                       int src_prec);
 int gbdw_gauge_destroy(gbdw_gauge* g);
 
-/* Spinor field with nrhs right-hand sides (stored rhs-innermost so one gauge load serves
+/* Spinor field with nrhs right-hand sides (stored side by side in every row, so one gauge load serves
  * Ls*nrhs slices). */
 int gbdw_field_create(gbdw_field** f, const gbdw_lattice* lat, int prec, int nrhs);
 int gbdw_field_destroy(gbdw_field* f);
@@ -354,10 +354,9 @@ int gbdw_tune_load(const char* path);
 int gbdw_tune_save(const char* path);
 /* Writes the chosen shape for a field into cfg[4]: threads per CTA, slices per thread,
  * form (0 direct loads, 1 TMA-staged neighbour blocks with one ring per CTA, 2 the same with
- * one ring per warp, 3 the direct form specialised for FP32/FP16 with Ls*nrhs = 16, 4 form 3 over 2x2x2x2
- * site blocks on periodic lattices with even extents, 5 the t-sweep over 2x2x2 columns that FP32
- * fields on periodic lattices with even x, y and z may get from gbdw_tune_dhop or a cache file)
- * and stages of the staged forms. */
+ * one ring per warp, 3 the direct form specialised for FP32/FP16 with Ls*nrhs = 16, 4 site blocks on
+ * periodic lattices: for FP32 2x2x2 columns swept along t (Ls*nrhs a multiple of 8 or 12, even x, y
+ * and z), for FP16 form 3 over 2x2x2x2 blocks (even extents)) and stages of the staged forms. */
 int gbdw_tune_query(const gbdw_gauge* g, const gbdw_field* in, int cfg[4]);
 /* Pins the shape for fields like `in` (threads a multiple of 32 up to 256; slices per thread
  * 1, 2 or 4 dividing Ls*nrhs, at most 2 for F64; form 0..4; stages 2/4). */
@@ -375,7 +374,8 @@ int gbdw_tune_set_split(const gbdw_gauge* g, const gbdw_field* in, int split);
  * z, y, x, t inside the brick), so neighbours along t are read close together in the sweep instead
  * of a whole 3D volume apart (what lets a site's spinor leave L2 before its next reader when a
  * site holds many slices, e.g. many right-hand sides).  The tuner chooses among 1 (natural order),
- * 2, 4, 8; gbdw_tune_brick reads the choice, gbdw_tune_set_brick pins it (Lt must be a multiple). */
+ * 2, 4, 8; gbdw_tune_brick reads the choice, gbdw_tune_set_brick pins it (Lt must be a multiple).
+ * For FP32 in form 4 the number is the slices of t one CTA walks (1: the built-in 8). */
 int gbdw_tune_brick(const gbdw_gauge* g, const gbdw_field* in, int* brick);
 int gbdw_tune_set_brick(const gbdw_gauge* g, const gbdw_field* in, int brick);
 /* The shape of the Shamir M pass (and of the CG passes built on it) for fields like `in` with one

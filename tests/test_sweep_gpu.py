@@ -31,7 +31,7 @@ def pin(gpu, tmp_path):
 
     def do(LsE, nt):
         pinned.add(LsE)
-        write(LsE, [64, 2, 5, 4, 1, nt])
+        write(LsE, [64, 2, 4, 4, 1, nt])
 
     yield do
     for LsE in pinned:
@@ -46,7 +46,7 @@ def test_sweep_dhop_m_and_mobius(gpu, pin, dims, Ls, nt):
     g = gb.Gauge(lat, c["U"], gb.F32)
     x, y, t = gb.Field(lat, gb.F32).load(c["phi"]), gb.Field(lat, gb.F32), gb.Field(lat, gb.F32)
     pin(Ls, nt)
-    assert gb.tune_query(g, x)[2] == 5
+    assert gb.tune_query(g, x)[2] == 4
     for dag in (0, 1):
         y.zero()
         gb.dhop(g, y, x, dag)
