@@ -2,10 +2,10 @@
 // right-hand sides, gauge field and storage precision FP32 or FP16) applied in ONE
 // persistent launch that is captured once in a CUDA graph and replayed.
 //
-// Work decomposition.  A thread owns `spt` consecutive innermost slices (e = s*nrhs + rhs)
+// Work decomposition.  A thread owns `spt` consecutive innermost slices (e = rhs*Ls + s)
 // of one site; the slices of a site are cut into `split` contiguous tiles of TE = LsE/split
-// slices, so a tile holds TE/nrhs values of s with all right-hand sides (an Ls tile) or, when
-// TE < nrhs, TE of the right-hand sides at one s (an RHS tile).  Threads are ordered (tile,
+// slices, so a tile holds whole right-hand sides (an RHS tile) or part of one's slices (an Ls tile)
+// where the cuts allow it.  Threads are ordered (tile,
 // site, slice group), and an instance's threads are cut into work items of one warp each.  The
 // link of a (site, leg) is loaded once per thread group and reused over its tile's slices;
 // more tiles put more sites in a CTA.

@@ -1,6 +1,7 @@
 // Lattices, gauge fields and spinor fields on the device, and the conversions between the
 // reference layout (dslash_simple.h:3-5, Nsimd lanes per bench.cc:105-139) and the GB300
 // layout of common.cuh.
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -149,7 +150,7 @@ __global__ void k_spinor_import(const SRC* src, int64_t nsite, int Ls, int nsimd
   const int64_t o = site / nsimd;
   const int lane = int(site - o * nsimd);
   const int LsE = Ls * nrhs;
-  const int e = s * nrhs + rhs;
+  const int e = rhs * Ls + s;
   double v[24];
   for (int k = 0; k < 12; ++k) {
     const int64_t j = ((o * Ls + s) * 12 + k) * nsimd + lane;
@@ -191,7 +192,7 @@ __global__ void k_spinor_export(const void* srcd, const float* norm, int64_t nsi
   const int64_t o = site / nsimd;
   const int lane = int(site - o * nsimd);
   const int LsE = Ls * nrhs;
-  const int e = s * nrhs + rhs;
+  const int e = rhs * Ls + s;
   for (int k = 0; k < 12; ++k) {
     double re, im;
     read_entry<P>(srcd, norm, site * 12 + k, e, LsP, site * LsE + e, re, im);
@@ -201,56 +202,135 @@ __global__ void k_spinor_export(const void* srcd, const float* norm, int64_t nsi
   }
 }
 
-// Site-block conversions for the common case Nsimd = 1, one right-hand side: a site's spinor
-// is one contiguous run of 12*Ls entries in both layouts, so one warp per site moves it with
-// coalesced 16-byte accesses through shared memory and permutes it there.
-template <class SRC, int P>
-__global__ void k_import_blocks(const SRC* __restrict__ src, int64_t nsite, int Ls, void* dst, float* norm, int LsP) {
+// Site-block conversions (Nsimd = 1): a site's spinor is one contiguous run in both layouts, so one
+// warp per site moves it with whole 16-byte accesses and permutes it in shared memory.  Lanes run over
+// (row, slice pair) on the field's side; SINGLE: over (row, slice), where a right-hand side's slices
+// straddle the stored pairs (several right-hand sides of an odd Ls).  e0 is the right-hand side's
+// first slice.  A slice's 24 reals take kTile reals of shared memory: the lanes of one row write 28
+// floats apart, two to a bank where 24 put four, and keep 16-byte alignment.  Bound by DRAM.
+// One of 12 right-hand sides of 24^4 x 12 FP32 (113 us of bytes): 147 us; with the right-hand
+// sides interleaved slice by slice, and one thread per 5D site, it took 771 (684 with these kernels:
+// reading every twelfth slice fetches all of the field).
+template <class R>
+constexpr int kTile = sizeof(R) == 4 ? 28 : 26;
+
+template <class SRC, int P, bool SINGLE>
+__global__ void k_import_sites(const SRC* __restrict__ src, int64_t nsite, int Ls, int LsE, int e0, void* dst,
+                               float* norm, int LsP) {
   extern __shared__ __align__(16) unsigned char sm[];
+  constexpr int TS = kTile<SRC>, V = 16 / sizeof(SRC);  // V reals per 16-byte vector
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t site = int64_t(blockIdx.x) * (blockDim.x >> 5) + warp;
   if (site >= nsite) return;
-  const int nreal = 24 * Ls;  // reals of the site block
-  SRC* buf = reinterpret_cast<SRC*>(sm) + size_t(warp) * nreal;
-  const SRC* s = src + site * nreal;
-  constexpr int V = 16 / sizeof(SRC);  // reals per 16-byte vector
-  for (int i = lane; i < nreal / V; i += 32) reinterpret_cast<uint4*>(buf)[i] = __ldg(reinterpret_cast<const uint4*>(s) + i);
+  SRC* buf = reinterpret_cast<SRC*>(sm) + size_t(warp) * TS * Ls;
+  float* scale = reinterpret_cast<float*>(reinterpret_cast<SRC*>(sm) + size_t(blockDim.x >> 5) * TS * Ls) + warp * Ls;
+  const uint4* s = reinterpret_cast<const uint4*>(src + site * 24 * Ls);
+  constexpr int VE = 24 / V;  // vectors of one slice
+  for (int i = lane; i < VE * Ls; i += 32) {
+    const int e = i / VE;
+    *reinterpret_cast<uint4*>(buf + e * TS + (i - e * VE) * V) = __ldg(s + i);
+  }
   __syncwarp();
-  for (int e = lane; e < Ls; e += 32) {
-    const SRC* v = buf + e * 24;
-    if (P == GBDW_F16) {
+  if constexpr (P == GBDW_F16) {
+    for (int e = lane; e < Ls; e += 32) {
+      const SRC* v = buf + e * TS;
       float m = 0.f;
       for (int k = 0; k < 24; ++k) m = fmaxf(m, fabsf(float(v[k])));
-      const float sc = m > 0.f ? 1.f / m : 0.f;
-      norm[site * Ls + e] = m;
-      for (int k = 0; k < 12; ++k) Elem<GBDW_F16>::st(dst, site * 12 + k, e, LsP, float(v[2 * k]) * sc, float(v[2 * k + 1]) * sc);
-    } else {
-      for (int k = 0; k < 12; ++k) Elem<P>::st(dst, site * 12 + k, e, LsP, v[2 * k], v[2 * k + 1]);
+      scale[e] = m > 0.f ? 1.f / m : 0.f;
+      norm[site * LsE + e0 + e] = m;
+    }
+    __syncwarp();
+  }
+  if constexpr (P == GBDW_F64 || SINGLE) {
+    for (int i = lane; i < 12 * Ls; i += 32) {
+      const int row = i / Ls, e = i - row * Ls;
+      const SRC* v = buf + e * TS + 2 * row;
+      if constexpr (P == GBDW_F16) Elem<P>::st(dst, site * 12 + row, e0 + e, LsP, float(v[0]) * scale[e], float(v[1]) * scale[e]);
+      else Elem<P>::st(dst, site * 12 + row, e0 + e, LsP, v[0], v[1]);
+    }
+  } else {
+    const int Q = (Ls + 1) / 2;
+    for (int i = lane; i < 12 * Q; i += 32) {
+      const int row = i / Q, e = 2 * (i - row * Q);
+      const SRC* v = buf + e * TS + 2 * row;
+      float a[4] = {float(v[0]), 0.f, float(v[1]), 0.f};
+      if (e + 1 < Ls) {  // an odd Ls leaves the last pair's second slot zero
+        a[1] = float(v[TS]);
+        a[3] = float(v[TS + 1]);
+      }
+      const int64_t g = ((site * 12 + row) * LsP + e0 + e) >> 1;
+      if constexpr (P == GBDW_F16) {
+        const float s0 = scale[e], s1 = e + 1 < Ls ? scale[e + 1] : 0.f;
+        reinterpret_cast<uint2*>(dst)[g] = make_uint2(f2h(a[0] * s0, a[1] * s1), f2h(a[2] * s0, a[3] * s1));
+      } else {
+        reinterpret_cast<float4*>(dst)[g] = make_float4(a[0], a[1], a[2], a[3]);
+      }
     }
   }
 }
 
-template <class DST, int P>
-__global__ void k_export_blocks(const void* __restrict__ srcd, const float* __restrict__ norm, int64_t nsite, int Ls,
-                                DST* __restrict__ dst, int LsP) {
+template <class DST, int P, bool SINGLE>
+__global__ void k_export_sites(const void* __restrict__ srcd, const float* __restrict__ norm, int64_t nsite, int Ls,
+                               int LsE, int e0, DST* __restrict__ dst, int LsP) {
   extern __shared__ __align__(16) unsigned char sm[];
+  constexpr int TS = kTile<DST>, V = 16 / sizeof(DST);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t site = int64_t(blockIdx.x) * (blockDim.x >> 5) + warp;
   if (site >= nsite) return;
-  const int nreal = 24 * Ls;
-  DST* buf = reinterpret_cast<DST*>(sm) + size_t(warp) * nreal;
-  for (int e = lane; e < Ls; e += 32) {
-    const float n = (P == GBDW_F16) ? __ldg(norm + site * Ls + e) : 1.f;
-    for (int k = 0; k < 12; ++k) {
-      const auto a = Elem<P>::ld(srcd, site * 12 + k, e, LsP);
-      buf[e * 24 + 2 * k] = (P == GBDW_F16) ? DST(float(a.r) * n) : DST(a.r);
-      buf[e * 24 + 2 * k + 1] = (P == GBDW_F16) ? DST(float(a.i) * n) : DST(a.i);
+  DST* buf = reinterpret_cast<DST*>(sm) + size_t(warp) * TS * Ls;
+  auto put = [&](int row, int s, float re, float im) {
+    if constexpr (P == GBDW_F16) {
+      const float n = __ldg(norm + site * LsE + e0 + s);
+      re *= n;
+      im *= n;
+    }
+    DST* b = buf + s * TS + 2 * row;
+    b[0] = DST(re);
+    b[1] = DST(im);
+  };
+  if constexpr (P == GBDW_F64) {
+    const double2* d = reinterpret_cast<const double2*>(srcd) + site * 12 * LsP;
+    for (int i = lane; i < 12 * Ls; i += 32) {
+      const int row = i / Ls, s = i - row * Ls;
+      const double2 a = __ldg(d + row * LsP + e0 + s);
+      DST* b = buf + s * TS + 2 * row;
+      b[0] = DST(a.x);
+      b[1] = DST(a.y);
+    }
+  } else {
+    auto group = [&](int row, int e) -> float4 {  // (Re, Re, Im, Im) of the stored pair of slice e
+      const int64_t g = ((site * 12 + row) * LsP + e) >> 1;
+      if constexpr (P == GBDW_F16) {
+        const uint2 h = __ldg(reinterpret_cast<const uint2*>(srcd) + g);
+        const float2 r = h2f(h.x), m = h2f(h.y);
+        return make_float4(r.x, r.y, m.x, m.y);
+      } else {
+        return __ldg(reinterpret_cast<const float4*>(srcd) + g);
+      }
+    };
+    if constexpr (SINGLE) {
+      for (int i = lane; i < 12 * Ls; i += 32) {
+        const int row = i / Ls, s = i - row * Ls, e = e0 + s;
+        const float4 a = group(row, e);
+        put(row, s, e & 1 ? a.y : a.x, e & 1 ? a.w : a.z);
+      }
+    } else {
+      const int Q = (Ls + 1) / 2;
+      for (int i = lane; i < 12 * Q; i += 32) {
+        const int row = i / Q, q = i - row * Q;
+        const float4 a = group(row, e0 + 2 * q);
+        put(row, 2 * q, a.x, a.z);
+        if (2 * q + 1 < Ls) put(row, 2 * q + 1, a.y, a.w);
+      }
     }
   }
   __syncwarp();
-  constexpr int V = 16 / sizeof(DST);
-  uint4* d = reinterpret_cast<uint4*>(dst + site * nreal);
-  for (int i = lane; i < nreal / V; i += 32) d[i] = reinterpret_cast<const uint4*>(buf)[i];
+  uint4* d = reinterpret_cast<uint4*>(dst + site * 24 * Ls);
+  constexpr int VE = 24 / V;
+  for (int i = lane; i < VE * Ls; i += 32) {
+    const int e = i / VE;
+    d[i] = *reinterpret_cast<const uint4*>(buf + e * TS + (i - e * VE) * V);
+  }
 }
 
 // Field-to-field precision conversion, one thread per 5D entry (site, e).
@@ -563,17 +643,20 @@ int gbdw_field_import(gbdw_field* f, int rhs, const void* src, int src_prec) {
   const int64_t n5 = L->nsite * L->Ls;
   const size_t bytes = size_t(n5) * 12 * (src_prec == GBDW_F64 ? 16 : 8);
   const int t = 256;
-  // site blocks: 4 warps per CTA, 24*Ls reals of shared memory per warp
-  const size_t blk_smem = 4 * size_t(24) * L->Ls * (src_prec == GBDW_F64 ? 8 : 4);
-  const bool blocks = L->nsimd == 1 && f->nrhs == 1 && blk_smem <= 48 * 1024;
+  // site blocks: up to 4 warps per CTA, the tile and the F16 scales of one site per warp
+  const size_t warp_smem = size_t(L->Ls) * ((src_prec == GBDW_F64 ? kTile<double> * 8 : kTile<float> * 4) + 4);
+  const int warps = int(std::min<size_t>(4, 48 * 1024 / warp_smem));
+  const bool blocks = L->nsimd == 1 && warps > 0;
+  const bool single = f->nrhs > 1 && L->Ls % 2;
   // host memory goes through a copy engine into the stream's staging buffer: the copy needs
   // no SMs, so copies of work queued on other streams overlap with it
   const void* dsrc = nullptr;
   if (int st = stage_in(src, bytes, 5, &dsrc)) return st;
   if (blocks && (uintptr_t(dsrc) & 15) == 0) {
-    const unsigned nb = unsigned((L->nsite + 3) / 4);
-#define GBDW_IB(SRC, P) \
-  k_import_blocks<SRC, P><<<nb, 128, blk_smem, stream()>>>((const SRC*)dsrc, L->nsite, L->Ls, f->d, f->norm, f->LsP)
+    const unsigned nb = unsigned((L->nsite + warps - 1) / warps);
+#define GBDW_IB(SRC, P)                                                                                       \
+  (single ? k_import_sites<SRC, P, true> : k_import_sites<SRC, P, false>)<<<nb, 32 * warps, warps * warp_smem, stream()>>>( \
+      (const SRC*)dsrc, L->nsite, L->Ls, f->LsE, rhs * L->Ls, f->d, f->norm, f->LsP)
     if (src_prec == GBDW_F64) {
       if (f->prec == GBDW_F64) GBDW_IB(double, GBDW_F64);
       else if (f->prec == GBDW_F32) GBDW_IB(double, GBDW_F32);
@@ -613,8 +696,10 @@ static int field_export(const gbdw_field* f, int rhs, void* dst, int dst_prec, b
   const int64_t n5 = L->nsite * L->Ls;
   const size_t bytes = size_t(n5) * 12 * (dst_prec == GBDW_F64 ? 16 : 8);
   const int t = 256;
-  const size_t blk_smem = 4 * size_t(24) * L->Ls * (dst_prec == GBDW_F64 ? 8 : 4);
-  const bool blocks = L->nsimd == 1 && f->nrhs == 1 && blk_smem <= 48 * 1024;
+  const size_t warp_smem = size_t(L->Ls) * (dst_prec == GBDW_F64 ? kTile<double> * 8 : kTile<float> * 4);
+  const int warps = int(std::min<size_t>(4, 48 * 1024 / warp_smem));
+  const bool blocks = L->nsimd == 1 && warps > 0;
+  const bool single = f->nrhs > 1 && L->Ls % 2;
   const bool dev = is_device_ptr(dst);
   void* ddst = dst;
   if (!dev) {
@@ -629,9 +714,10 @@ static int field_export(const gbdw_field* f, int rhs, void* dst, int dst_prec, b
     }
   }
   if (blocks && (uintptr_t(ddst) & 15) == 0) {
-    const unsigned nb = unsigned((L->nsite + 3) / 4);
-#define GBDW_EB(DST, P) \
-  k_export_blocks<DST, P><<<nb, 128, blk_smem, stream()>>>(f->d, f->norm, L->nsite, L->Ls, (DST*)ddst, f->LsP)
+    const unsigned nb = unsigned((L->nsite + warps - 1) / warps);
+#define GBDW_EB(DST, P)                                                                                       \
+  (single ? k_export_sites<DST, P, true> : k_export_sites<DST, P, false>)<<<nb, 32 * warps, warps * warp_smem, stream()>>>( \
+      f->d, f->norm, L->nsite, L->Ls, f->LsE, rhs * L->Ls, (DST*)ddst, f->LsP)
     if (dst_prec == GBDW_F64) {
       if (f->prec == GBDW_F64) GBDW_EB(double, GBDW_F64);
       else if (f->prec == GBDW_F32) GBDW_EB(double, GBDW_F32);

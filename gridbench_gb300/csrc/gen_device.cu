@@ -33,7 +33,7 @@ __global__ void k_field_gaussian(void* d, float* norm, int prec, int64_t nsite, 
   const int64_t site = i / Ls;
   const int s = int(i - site * Ls);
   const int LsE = Ls * nrhs;
-  const int e = s * nrhs + rhs;
+  const int e = rhs * Ls + s;
   uint64_t st = seed ^ (uint64_t(i) * 0xD1B54A32D192ED03ull);
   sm_next(st);
   double2 v[12];

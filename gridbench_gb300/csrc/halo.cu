@@ -16,7 +16,9 @@
 // lowest dimension fastest) x row k (h0 colours 0..2, then h1 colours 0..2) x the field's LsE
 // slices in its own storage format (F64: double2 per slice; F32/F16: slice pairs stored as
 // (Re s, Re s+1, Im s, Im s+1) over LsP slots); for F16 a block of nface * LsE FP32 norms (the
-// largest |component| of each slice's packed half spinor) follows the values.
+// largest |component| of each slice's packed half spinor) follows the values.  Slot e of the buffer
+// is slice s = e / nrhs of right-hand side e % nrhs; the field keeps its right-hand sides one after the
+// other, so fields with several are read slice by slice (FROM).
 // One thread per (face site, slice pair) over all requested faces in one launch: every face
 // spinor is read once, 6 of its 12 complex components are written -- HBM bound, 1.5 spinors of
 // traffic per packed 5D site.
@@ -58,12 +60,14 @@ struct HaloParams {
   int dims[4];
   int LsE;
   int LsP;
+  int Ls;
+  int nrhs;
   int nfaces;
   int64_t total;  // threads over all faces
   HaloFace face[8];
 };
 
-template <int P, int LT, int N>
+template <int P, int LT, int N, bool FROM>
 __device__ __forceinline__ void pack_face(const HaloParams& p, const HaloFace& F, int64_t f, int e0) {
   using T = typename Arith<P>::T;
   using S = LegSpin<LT>;
@@ -80,14 +84,23 @@ __device__ __forceinline__ void pack_face(const HaloParams& p, const HaloFace& F
   }
   const int64_t site = c[0] + int64_t(p.dims[0]) * (c[1] + int64_t(p.dims[1]) * (c[2] + int64_t(p.dims[2]) * c[3]));
   const int64_t row0 = site * 12;
+  auto from = [&](int e) { return FROM ? (e % p.nrhs) * p.Ls + e / p.nrhs : e; };  // the field's slot
+  auto load = [&](int64_t row, cpx<T>(&v)[N]) {
+    if constexpr (FROM) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) v[j] = Elem<P>::ld(p.in, row, from(e0 + j), p.LsP);
+    } else {
+      Vec<P, N>::load(p.in, row, e0, p.LsP, v);
+    }
+  };
   cpx<T> h[6][N];
 #pragma unroll
   for (int col = 0; col < 3; ++col) {
     cpx<T> x[N], y[N], z[N], w[N];
-    Vec<P, N>::load(p.in, row0 + 0 * 3 + col, e0, p.LsP, x);
-    Vec<P, N>::load(p.in, row0 + S::A * 3 + col, e0, p.LsP, y);
-    Vec<P, N>::load(p.in, row0 + 1 * 3 + col, e0, p.LsP, z);
-    Vec<P, N>::load(p.in, row0 + S::B * 3 + col, e0, p.LsP, w);
+    load(row0 + 0 * 3 + col, x);
+    load(row0 + S::A * 3 + col, y);
+    load(row0 + 1 * 3 + col, z);
+    load(row0 + S::B * 3 + col, w);
 #pragma unroll
     for (int j = 0; j < N; ++j) {
       const cpx<T> ya = unit_times<T, S::C0>(y[j]), wb = unit_times<T, S::C1>(w[j]);
@@ -99,7 +112,12 @@ __device__ __forceinline__ void pack_face(const HaloParams& p, const HaloFace& F
   if constexpr (P == GBDW_F16) {
     // dequantise with the source slices' norms, renormalise each slice's half spinor
     float n[N], m[N], sc[N];
-    load_norms<N>(p.in_norm, site * p.LsE + e0, n);
+    if constexpr (FROM) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) n[j] = __ldg(p.in_norm + site * p.LsE + from(e0 + j));
+    } else {
+      load_norms<N>(p.in_norm, site * p.LsE + e0, n);
+    }
 #pragma unroll
     for (int j = 0; j < N; ++j) {
       m[j] = 0.f;
@@ -130,7 +148,7 @@ __device__ __forceinline__ void pack_face(const HaloParams& p, const HaloFace& F
   }
 }
 
-template <int P, int N>
+template <int P, int N, bool FROM>
 __global__ void __launch_bounds__(256) k_halo_pack(const __grid_constant__ HaloParams p) {
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= p.total) return;
@@ -142,14 +160,14 @@ __global__ void __launch_bounds__(256) k_halo_pack(const __grid_constant__ HaloP
   const int64_t f = t / G;
   const int e0 = int(t - f * G) * N;
   switch (F.leg) {
-    case 0: pack_face<P, 0, N>(p, F, f, e0); break;
-    case 1: pack_face<P, 1, N>(p, F, f, e0); break;
-    case 2: pack_face<P, 2, N>(p, F, f, e0); break;
-    case 3: pack_face<P, 3, N>(p, F, f, e0); break;
-    case 4: pack_face<P, 4, N>(p, F, f, e0); break;
-    case 5: pack_face<P, 5, N>(p, F, f, e0); break;
-    case 6: pack_face<P, 6, N>(p, F, f, e0); break;
-    default: pack_face<P, 7, N>(p, F, f, e0); break;
+    case 0: pack_face<P, 0, N, FROM>(p, F, f, e0); break;
+    case 1: pack_face<P, 1, N, FROM>(p, F, f, e0); break;
+    case 2: pack_face<P, 2, N, FROM>(p, F, f, e0); break;
+    case 3: pack_face<P, 3, N, FROM>(p, F, f, e0); break;
+    case 4: pack_face<P, 4, N, FROM>(p, F, f, e0); break;
+    case 5: pack_face<P, 5, N, FROM>(p, F, f, e0); break;
+    case 6: pack_face<P, 6, N, FROM>(p, F, f, e0); break;
+    default: pack_face<P, 7, N, FROM>(p, F, f, e0); break;
   }
 }
 
@@ -186,8 +204,13 @@ int check_halo(const gbdw_field* f, int mu) {
 template <int P>
 void launch_pack(const HaloParams& p, int N) {
   const unsigned g = unsigned((p.total + 255) / 256);
-  if (N == 2) k_halo_pack<P, 2><<<g, 256, 0, stream()>>>(p);
-  else k_halo_pack<P, 1><<<g, 256, 0, stream()>>>(p);
+  if (p.nrhs > 1) {
+    if (N == 2) k_halo_pack<P, 2, true><<<g, 256, 0, stream()>>>(p);
+    else k_halo_pack<P, 1, true><<<g, 256, 0, stream()>>>(p);
+  } else {
+    if (N == 2) k_halo_pack<P, 2, false><<<g, 256, 0, stream()>>>(p);
+    else k_halo_pack<P, 1, false><<<g, 256, 0, stream()>>>(p);
+  }
 }
 
 // Packs the faces (mu[k], face[k]) into device buffers dst[k] in one launch.
@@ -198,6 +221,8 @@ int pack_faces(const gbdw_field* f, int n, const int* mu, const int* face, int d
   for (int k = 0; k < 4; ++k) p.dims[k] = f->lat->dims[k];
   p.LsE = f->LsE;
   p.LsP = f->LsP;
+  p.Ls = f->lat->Ls;
+  p.nrhs = f->nrhs;
   p.nfaces = n;
   const int N = (f->prec != GBDW_F64 && f->LsE % 2 == 0) ? 2 : 1;
   int64_t first = 0;
