@@ -94,42 +94,64 @@ struct M5InvParams {
 // The recursion form of D5^-1 on one chirality, per spin-colour row (x, y of length Ls):
 //   shift s-1 -> s:  y(0) = g [x(0) - mf sum_{t>=1} a5^-(Ls-t) x(t)],  y(s) = (x(s) + y(s-1)) / a5
 //   shift s+1 -> s:  y(Ls-1) = g [x(Ls-1) - mf sum_{t<=Ls-2} a5^-(t+1) x(t)],  y(s) = (x(s) + y(s+1)) / a5
-// which is the dense form above row by row (the wrap coefficient folds into g).  Phase 1:
-// one thread per (site, row) runs both sweeps into a shared-memory tile; phase 2: one thread
-// per (site, N slices) writes the tile in the field's storage format (norms for F16).
-// Both sweeps of one row over values v[0..Ls) (registers when LSC > 0), results into y.
-template <class T, bool DOWN, class V>
+// which is the dense form above row by row (the wrap coefficient folds into g).  Both sweeps of one
+// row over values v(0..Ls), results into y (which may be the row v reads: every v(t) is read before
+// y[t] is written).  The sums run as u(t) = v(t) + u(t-1)/a5, one FMA a step.
+template <class T, bool DOWN, int LSC, class V>
 __device__ __forceinline__ void m5_sweeps(const V& v, int Ls, T ia5, T g, T mf, cpx<T>* y) {
+  const int s0 = DOWN ? 0 : Ls - 1, ds = DOWN ? 1 : -1;
   cpx<T> w = {T(0), T(0)};
-  if constexpr (DOWN) {
-    for (int t = 1; t < Ls; ++t) w = {(w.r + v(t).r) * ia5, (w.i + v(t).i) * ia5};
-    cpx<T> prev = {g * (v(0).r - mf * w.r), g * (v(0).i - mf * w.i)};
-    y[0] = prev;
-    for (int t = 1; t < Ls; ++t) {
-      prev = {(v(t).r + prev.r) * ia5, (v(t).i + prev.i) * ia5};
-      y[t] = prev;
-    }
-  } else {
-    for (int t = Ls - 2; t >= 0; --t) w = {(w.r + v(t).r) * ia5, (w.i + v(t).i) * ia5};
-    cpx<T> prev = {g * (v(Ls - 1).r - mf * w.r), g * (v(Ls - 1).i - mf * w.i)};
-    y[Ls - 1] = prev;
-    for (int t = Ls - 2; t >= 0; --t) {
-      prev = {(v(t).r + prev.r) * ia5, (v(t).i + prev.i) * ia5};
-      y[t] = prev;
-    }
+#pragma unroll(LSC > 0 ? LSC : 4)
+  for (int k = 1; k < Ls; ++k) {
+    const cpx<T> x = v(s0 + k * ds);
+    w = {::fma(w.r, ia5, x.r), ::fma(w.i, ia5, x.i)};
+  }
+  const T c = -mf * ia5;
+  const cpx<T> x0 = v(s0);
+  cpx<T> prev = {g * ::fma(c, w.r, x0.r), g * ::fma(c, w.i, x0.i)};
+  y[s0] = prev;
+#pragma unroll(LSC > 0 ? LSC : 4)
+  for (int k = 1; k < Ls; ++k) {
+    const cpx<T> x = v(s0 + k * ds);
+    prev = {(x.r + prev.r) * ia5, (x.i + prev.i) * ia5};
+    y[s0 + k * ds] = prev;
   }
 }
 
+// Phase 1: one thread per (site, row) runs both sweeps into a shared-memory tile; phase 2: one
+// thread per (site, N slices) writes the tile in the field's storage format (norms for F16).
 // LSC > 0: the launch guarantees Ls == LSC (even), and a row is loaded into registers with
-// slice-pair vector loads before the sweeps; LSC == 0 reads the row slice by slice.
+// slice-pair vector loads before the sweeps.  LSC == 0: the CTA first loads its sites into the tile,
+// lanes along (row, N slices) so that whole lines are read, and the sweeps run in place; reading the
+// rows slice by slice from global memory took 66 us for 786432 5D sites of FP32 (Ls = 12), 22 us
+// being the time of its bytes.
 template <int P, int DAG, int N, int LSC>
 __global__ void __launch_bounds__(192) k_m5inv(const M5InvParams p) {
   using T = typename Arith<P>::T;
   extern __shared__ __align__(16) unsigned char m5_smem[];
-  cpx<T>* tile = reinterpret_cast<cpx<T>*>(m5_smem);  // [nsb][12][Ls + 1] (padded rows)
-  const int Ls = LSC > 0 ? LSC : p.Ls, LsT = Ls + 1;
+  cpx<T>* tile = reinterpret_cast<cpx<T>*>(m5_smem);  // [nsb][12][Ls | 1] (rows of an odd stride)
+  const int Ls = LSC > 0 ? LSC : p.Ls, LsT = Ls | 1;
   const int64_t site0 = int64_t(blockIdx.x) * p.nsb;
   const T ia5 = T(p.ia5), g = T(p.g), mf = T(p.mf);
+  const int G = Ls / N;
+  if constexpr (LSC == 0) {
+    const int per_site = 12 * G;
+    const int items = int(min(int64_t(p.nsb), p.nsite - site0)) * per_site;
+    for (int it = threadIdx.x; it < items; it += blockDim.x) {
+      const int row = it / G, s = (it - row * G) * N;  // row counts through the CTA's sites
+      cpx<T> v[N];
+      Vec<P, N>::load(p.in, site0 * 12 + row, s, p.LsP, v);
+      if constexpr (P == GBDW_F16) {
+        float nr[N];
+        load_norms<N>(p.in_norm, (site0 + row / 12) * Ls + s, nr);
+#pragma unroll
+        for (int j = 0; j < N; ++j) v[j] = {v[j].r * nr[j], v[j].i * nr[j]};
+      }
+#pragma unroll
+      for (int j = 0; j < N; ++j) tile[row * LsT + s + j] = v[j];
+    }
+    __syncthreads();
+  }
   if (threadIdx.x < 12 * p.nsb) {
     const int ls = threadIdx.x / 12, row = threadIdx.x - 12 * (threadIdx.x / 12);
     const int64_t site = site0 + ls;
@@ -153,24 +175,16 @@ __global__ void __launch_bounds__(192) k_m5inv(const M5InvParams p) {
           for (int t = 0; t < LSC; ++t) xv[t] = {xv[t].r * nr[t], xv[t].i * nr[t]};
         }
         auto v = [&](int t) -> const cpx<T>& { return xv[t]; };
-        if (down) m5_sweeps<T, true>(v, LSC, ia5, g, mf, y);
-        else m5_sweeps<T, false>(v, LSC, ia5, g, mf, y);
+        if (down) m5_sweeps<T, true, LSC>(v, LSC, ia5, g, mf, y);
+        else m5_sweeps<T, false, LSC>(v, LSC, ia5, g, mf, y);
       } else {
-        auto v = [&](int t) -> cpx<T> {
-          cpx<T> e = Elem<P>::ld(p.in, r, t, p.LsP);
-          if constexpr (P == GBDW_F16) {
-            const float n = __ldg(p.in_norm + site * Ls + t);
-            e = {e.r * n, e.i * n};
-          }
-          return e;
-        };
-        if (down) m5_sweeps<T, true>(v, Ls, ia5, g, mf, y);
-        else m5_sweeps<T, false>(v, Ls, ia5, g, mf, y);
+        auto v = [&](int t) -> cpx<T> { return y[t]; };
+        if (down) m5_sweeps<T, true, 0>(v, Ls, ia5, g, mf, y);
+        else m5_sweeps<T, false, 0>(v, Ls, ia5, g, mf, y);
       }
     }
   }
   __syncthreads();
-  const int G = Ls / N;
   for (int it = threadIdx.x; it < p.nsb * G; it += blockDim.x) {
     const int ls = it / G;
     const int64_t site = site0 + ls;
@@ -217,7 +231,7 @@ int m5inv(gbdw_field* out, const gbdw_field* in, double M5, double mf, int dag) 
   }
   p.g = 1.0 / den;
   if (int st = ensure_device()) return st;
-  const size_t per_site = 12 * size_t(Ls + 1) * (in->prec == GBDW_F64 ? 16 : 8);
+  const size_t per_site = 12 * size_t(Ls | 1) * (in->prec == GBDW_F64 ? 16 : 8);
   p.nsb = int(std::min<size_t>(16, 49152 / per_site));
   const size_t smem = size_t(p.nsb) * per_site;
   const unsigned g = nb(p.nsite, p.nsb);
