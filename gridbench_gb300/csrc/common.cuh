@@ -2,7 +2,7 @@
 //
 // Device layout ("GB300 layout"), chosen so that consecutive threads read consecutive
 // addresses and one 4D link serves every fifth-dimension slice of its site:
-//   spinor  [site][sc = spin*3+colour][e = s*nrhs + rhs]   complex (F64 16 B, F32 8 B, F16 4 B);
+//   spinor  [site][sc = spin*3+colour][e = rhs*Ls + s]    complex (F64 16 B, F32 8 B, F16 4 B);
 //           F32/F16 store slice pairs as (Re, Re, Im, Im) -- layout.cuh has the addressing --
 //           and F16 adds norm[site][e] (FP32, max |re|,|im| over the 24 reals of that 5D site)
 //   gauge   [site][mu][row][col] complex, 9 entries (F64/F32) or rows 0-1 only (F16/BF16)
@@ -152,12 +152,22 @@ __device__ __forceinline__ void block_sum_to_thread0(double (&v)[W], double (&sh
     if (lane == 0) sh[warp][w] = x;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
+  const int nw = (blockDim.x + 31) >> 5;
+  if (nw <= 4) {
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        double x = 0.0;
+        for (int k = 0; k < nw; ++k) x += sh[k][w];
+        v[w] = x;
+      }
+    }
+  } else if (warp == 0) {  // up to 32 dependent FP64 adds by one thread take longer than five exchanges
 #pragma unroll
     for (int w = 0; w < W; ++w) {
-      double x = 0.0;
-      for (int k = 0; k < nw; ++k) x += sh[k][w];
+      double x = lane < nw ? sh[lane][w] : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
       v[w] = x;
     }
   }
