@@ -321,20 +321,20 @@ __device__ __forceinline__ float4 axpby_v(float a, float4 x, float b, float4 y) 
   return make_float4(fmaf(a, x.x, b * y.x), fmaf(a, x.y, b * y.y), fmaf(a, x.z, b * y.z), fmaf(a, x.w, b * y.w));
 }
 __device__ __forceinline__ double2 axpby_v(double a, double2 x, double b, double2 y) {
-  return make_double2(::fma(a, x.x, b * y.x), ::fma(a, x.y, b * y.y));
+  return make_double2(fma(a, x.x, b * y.x), fma(a, x.y, b * y.y));
 }
 __device__ __forceinline__ void norm_v(float4 x, float& s) {
   s = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, s))));
 }
-__device__ __forceinline__ void norm_v(double2 x, double& s) { s = ::fma(x.x, x.x, ::fma(x.y, x.y, s)); }
+__device__ __forceinline__ void norm_v(double2 x, double& s) { s = fma(x.x, x.x, fma(x.y, x.y, s)); }
 // conj(x) y: an FP32 vector holds (Re, Re, Im, Im) of two slices
 __device__ __forceinline__ void dot_v(float4 x, float4 y, float& re, float& im) {
   re = fmaf(x.x, y.x, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.w, y.w, re))));
   im = fmaf(x.x, y.z, fmaf(-x.z, y.x, fmaf(x.y, y.w, fmaf(-x.w, y.y, im))));
 }
 __device__ __forceinline__ void dot_v(double2 x, double2 y, double& re, double& im) {
-  re = ::fma(x.x, y.x, ::fma(x.y, y.y, re));
-  im = ::fma(x.x, y.y, ::fma(-x.y, y.x, im));
+  re = fma(x.x, y.x, fma(x.y, y.y, re));
+  im = fma(x.x, y.y, fma(-x.y, y.x, im));
 }
 
 // f(i, k) for the vectors i of this thread, loads of kVec of them (load(i, k)) before the first f;
@@ -417,10 +417,10 @@ __global__ void k_cg_xp_f64_pairs(double alpha, double beta, double2* __restrict
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < npair; i += int64_t(gridDim.x) * blockDim.x) {
     const double2 p0 = p[2 * i], p1 = p[2 * i + 1], x0 = x[2 * i], x1 = x[2 * i + 1];
     const double2 r0 = __ldg(r + 2 * i), r1 = __ldg(r + 2 * i + 1);
-    x[2 * i] = make_double2(::fma(alpha, p0.x, x0.x), ::fma(alpha, p0.y, x0.y));
-    x[2 * i + 1] = make_double2(::fma(alpha, p1.x, x1.x), ::fma(alpha, p1.y, x1.y));
-    const double2 n0 = make_double2(::fma(beta, p0.x, r0.x), ::fma(beta, p0.y, r0.y));
-    const double2 n1 = make_double2(::fma(beta, p1.x, r1.x), ::fma(beta, p1.y, r1.y));
+    x[2 * i] = make_double2(fma(alpha, p0.x, x0.x), fma(alpha, p0.y, x0.y));
+    x[2 * i + 1] = make_double2(fma(alpha, p1.x, x1.x), fma(alpha, p1.y, x1.y));
+    const double2 n0 = make_double2(fma(beta, p0.x, r0.x), fma(beta, p0.y, r0.y));
+    const double2 n1 = make_double2(fma(beta, p1.x, r1.x), fma(beta, p1.y, r1.y));
     p[2 * i] = n0;
     p[2 * i + 1] = n1;
     if (q) q[i] = make_float4(float(n0.x), float(n1.x), float(n0.y), float(n1.y));

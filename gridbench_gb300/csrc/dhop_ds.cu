@@ -4,7 +4,8 @@
 // same bytes and computes on the FP32 pipe, at ~1e-14 relative accuracy.  It serves the solvers'
 // FP64 operator (true residuals of the reliable updates, the FP64 CG) by default and any FP64
 // operator call on request (gbdw_set_fp64_arith).
-#include "dhop_launch.cuh"
+#include "dhop_kernel.cuh"
+#include "dsfloat.cuh"
 
 namespace gbdw {
 
@@ -57,12 +58,151 @@ int ds_links(const gbdw_gauge* g, const void** out) {
   return GBDW_OK;
 }
 
-// Direct form, one slice per thread, 128-thread CTAs with registers capped for four CTAs per SM
-// (16 warps): the arithmetic is the bound, and warps hide its dependency chains.  Measured at
-// 16^4 x Ls=16 (Dhop, ms): 1.075 at this cap, 1.24 at three CTAs (170 registers), 1.79 uncapped
-// (254 registers, 8 warps); two slices per thread 1.80-2.56; native FP64 1.635.
-// minb: the register cap, as CTAs per SM (4: 128 registers; 3: 170, which spills less in the M
-// epilogue); the t-brick order comes in p.brick.
+namespace {
+
+// ------------------------------------------------------------------ packed double-single arithmetic
+// A complex number as two FP32 pairs: (re, im) of the leading parts in h and of the trailing parts in
+// l, so that one FADD2 / FMUL2 / FFMA2 serves both components: half the instructions of the scalar
+// form of dsfloat.cuh, the same error-free transformations step by step.
+struct ds2 {
+  float2 h, l;
+};
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }  // exact product
+__device__ __forceinline__ float2 swap2(float2 a) { return make_float2(a.y, a.x); }
+// s + e = a + b exactly (Knuth)
+__device__ __forceinline__ float2 two_sum2(float2 a, float2 b, float2& e) {
+  const float2 s = add2(a, b), bb = sub2(s, a);
+  e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+  return s;
+}
+// the pair (s, t) renormalised (Dekker)
+__device__ __forceinline__ ds2 join2(float2 s, float2 t) {
+  const float2 h = add2(s, t);
+  return {h, sub2(t, sub2(h, s))};
+}
+// SloppyDWPlusDW
+__device__ __forceinline__ ds2 operator+(ds2 a, ds2 b) {
+  float2 e;
+  const float2 s = two_sum2(a.h, b.h, e);
+  return join2(s, add2(e, add2(a.l, b.l)));
+}
+// c y for a unit c (codes of LegSpin)
+template <int C>
+__device__ __forceinline__ ds2 unit2(ds2 y) {
+  if constexpr (C == 0) return y;
+  else if constexpr (C == 1) return {make_float2(-y.h.x, -y.h.y), make_float2(-y.l.x, -y.l.y)};
+  else if constexpr (C == 2) return {make_float2(-y.h.y, y.h.x), make_float2(-y.l.y, y.l.x)};
+  else return {make_float2(y.h.y, -y.h.x), make_float2(y.l.y, -y.l.x)};
+}
+// One step of a compensated dot product: s + e += a b with s the running sum of the leading products
+// (every rounding error of which goes into e) and e plain FP32; a is the same real for both components
+// up to sign.
+__device__ __forceinline__ void dot2(float2 ah, float2 al, ds2 b, float2& s, float2& e) {
+  const float2 p = __fmul2_rn(ah, b.h);
+  const float2 pe = __ffma2_rn(ah, b.h, make_float2(-p.x, -p.y));  // exact
+  e = __ffma2_rn(ah, b.l, e);
+  e = __ffma2_rn(al, b.h, e);
+  float2 f;
+  s = two_sum2(s, p, f);
+  e = add2(e, add2(pe, f));
+}
+// An FP64 complex number as pairs, with the bits of ds_split: h the leading 24 mantissa bits moved over
+// by integer operations, l the other 29 rounded to 24 and scaled by 2^-52 of h's exponent.
+__device__ __forceinline__ void split1(double d, float& h, float& l) {
+  const unsigned hi = unsigned(__double2hiint(d)), lo = unsigned(__double2loint(d));
+  const unsigned t = __funnelshift_l(lo, hi, 3);
+  const unsigned hb = ((t & 0x7fffffffu) ^ 0x40000000u) | (hi & 0x80000000u);
+  const unsigned ah = hi & 0x7fffffffu;
+  const float scale = __uint_as_float(hb & 0xff800000u) * 2.220446049250313e-16f;
+  h = __uint_as_float(hb);
+  l = __uint2float_rn(lo & 0x1fffffffu) * scale;
+  if (ah - 0x38100000u >= 0x0fe00000u) {  // below 2^-126 (zero) or beyond FP32 (infinity)
+    h = __uint_as_float((hi & 0x80000000u) | (ah < 0x38100000u ? 0u : 0x7f800000u));
+    l = 0.f;
+  }
+}
+__device__ __forceinline__ ds2 split2(double2 a) {
+  float2 h, l;
+  split1(a.x, h.x, l.x);
+  split1(a.y, h.y, l.y);
+  return join2(h, l);
+}
+
+template <int DAG, int L>
+__device__ __forceinline__ void ds_leg(const float4* __restrict__ u, const double2* __restrict__ in, int64_t row0,
+                                       int LsE, ds2 (&acc)[12]) {
+  using S = LegSpin<DAG ? (L ^ 4) : L>;
+  ds2 h0[3], h1[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    h0[c] = split2(__ldg(in + (row0 + c) * LsE)) + unit2<S::C0>(split2(__ldg(in + (row0 + S::A * 3 + c) * LsE)));
+    h1[c] = split2(__ldg(in + (row0 + 3 + c) * LsE)) + unit2<S::C1>(split2(__ldg(in + (row0 + S::B * 3 + c) * LsE)));
+  }
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    float2 s0 = make_float2(0.f, 0.f), e0 = s0, s1 = s0, e1 = s0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float4 a = __ldg(u + r * 3 + c);  // re h, re l, im h, im l
+      const float2 rh = make_float2(a.x, a.x), rl = make_float2(a.y, a.y);
+      const float2 ih = make_float2(-a.z, a.z), il = make_float2(-a.w, a.w);
+      dot2(rh, rl, h0[c], s0, e0);
+      dot2(rh, rl, h1[c], s1, e1);
+      dot2(ih, il, {swap2(h0[c].h), swap2(h0[c].l)}, s0, e0);
+      dot2(ih, il, {swap2(h1[c].h), swap2(h1[c].l)}, s1, e1);
+    }
+    const ds2 u0 = join2(s0, e0), u1 = join2(s1, e1);
+    acc[r] = acc[r] + u0;
+    acc[3 + r] = acc[3 + r] + u1;
+    acc[S::A * 3 + r] = acc[S::A * 3 + r] + unit2<conj_unit<S::C0>::v>(u0);
+    acc[S::B * 3 + r] = acc[S::B * 3 + r] + unit2<conj_unit<S::C1>::v>(u1);
+  }
+}
+
+// One slice per thread, 128-thread CTAs with registers capped for MINB CTAs per SM.  What bounds the
+// kernel is its instructions on the FP32 pipe; the epilogue (M's diagonal part and |.|^2) is FP64, on a
+// pipe that is otherwise idle.  Measured (ms; Dhop, M; scalar pairs with a pair epilogue -> this):
+//   16^4 x 16  1.061, 1.45 -> 0.619, 0.717 (native FP64 1.637)   32^4 x 16  20.2, 22.9 -> 11.1, 11.5
+//   half of 16^4 x 16  0.612, 0.975 -> 0.332, 0.466
+// and 2.8e-15 from FP64 (4.0e-15 before).  Tried and slower: running some of the CTAs in native FP64
+// beside the others to use both pipes (2 of 16: 1.07 ms, 4 of 16: 1.20; they stay resident far longer
+// than their share of the work).
+template <int DAG, int EPI, int MINB>
+__global__ void __launch_bounds__(DS_THREADS, MINB) k_dhop_ds(const DhopParams p) {
+  const unsigned bid = DAG ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  const unsigned tid = bid * DS_THREADS + threadIdx.x;
+  const unsigned LsE = unsigned(p.LsE);
+  float part = 0.f;
+  double dpart = 0.0;
+  if (tid < unsigned(p.nsite) * LsE) {
+    unsigned site = tid / LsE;
+    const int s0 = int(tid - site * LsE);
+    if (p.brick > 1) site = brick_site(p, site);
+    ds2 acc[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) acc[k] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    const uint32_t* nb = p.nbr4 + size_t(site) * 8;
+    const float4* u = (const float4*)p.U + size_t(site) * 72;
+    const double2* in = (const double2*)p.in + s0;
+#define GBDW_LEG(L) ds_leg<DAG, L>(u + 9 * L, in, int64_t(__ldg(nb + L)) * 12, p.LsE, acc);
+    GBDW_LEG(0) GBDW_LEG(4) GBDW_LEG(1) GBDW_LEG(5) GBDW_LEG(2) GBDW_LEG(6) GBDW_LEG(3) GBDW_LEG(7)
+#undef GBDW_LEG
+    cpx<double> v[1][12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k)
+      v[0][k] = {double(acc[k].h.x) + double(acc[k].l.x), double(acc[k].h.y) + double(acc[k].l.y)};
+    finish_site<GBDW_F64, GBDW_F64, DAG, 1, EPI>(p, site, s0, p.LsE, p.LsP, v, part, dpart);
+  }
+  if (p.partials) {
+    double v[1] = {dpart};
+    block_partial<1>(v, p.partials);
+  }
+}
+
+}  // namespace
+
+// minb: the register cap, as CTAs per SM (4: 128 registers, 3: 168); the t-brick order comes in p.brick
 int launch_dhop_ds(const DhopParams& p, int dag, int epi, int minb) {
   if (epi > 1 || (minb != 3 && minb != 4)) {
     set_error("double-single operator: Dhop and M, three or four CTAs per SM");
@@ -70,7 +210,7 @@ int launch_dhop_ds(const DhopParams& p, int dag, int epi, int minb) {
   }
   const int64_t nthreads = p.nsite * p.LsE;
   const unsigned blocks = unsigned((nthreads + DS_THREADS - 1) / DS_THREADS);
-#define GBDW_DSK(D, E, MB) k_dhop<GBDW_DS, GBDW_DS, GBDW_DS, D, 1, E, MB, 0, DS_THREADS><<<blocks, DS_THREADS, 0, stream()>>>(p)
+#define GBDW_DSK(D, E, MB) k_dhop_ds<D, E, MB><<<blocks, DS_THREADS, 0, stream()>>>(p)
   if (minb == 4) {
     if (dag) epi ? GBDW_DSK(1, 1, 4) : GBDW_DSK(1, 0, 4);
     else epi ? GBDW_DSK(0, 1, 4) : GBDW_DSK(0, 0, 4);

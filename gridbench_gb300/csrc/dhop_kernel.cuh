@@ -32,10 +32,6 @@ template <>
 struct Arith<GBDW_F64> {
   using T = double;
 };
-template <>
-struct Arith<GBDW_DS> {
-  using T = dsf;
-};
 
 template <int N>
 __device__ __forceinline__ void load_norms(const float* nrm, int64_t e, float (&v)[N]) {
@@ -121,20 +117,6 @@ struct LinkIO<GBDW_F64> {
     for (int k = 0; k < 9; ++k) {
       const double2 a = ldv<SMEM>(p + k);
       u[k / 3][k % 3] = {a.x, a.y};
-    }
-  }
-};
-// the F64 gauge field's split copy: one float4 (re h, re l, im h, im l) per entry
-template <>
-struct LinkIO<GBDW_DS> {
-  static constexpr unsigned bytes = 144;
-  template <bool SMEM = false>
-  static __device__ __forceinline__ void load(const void* U, size_t link, cpx<dsf> (&u)[3][3]) {
-    const float4* p = (const float4*)U + link * 9;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      const float4 a = ldv<SMEM>(p + k);
-      u[k / 3][k % 3] = {dsf(a.x, a.y), dsf(a.z, a.w)};
     }
   }
 };
@@ -562,16 +544,6 @@ template <int N>
 __device__ __forceinline__ double sumsq(const cpx<float> (&)[N][12]) {
   return 0.0;
 }
-template <int N>
-__device__ __forceinline__ double sumsq(const cpx<dsf> (&v)[N][12]) {
-  dsf s(0.f, 0.f);
-#pragma unroll
-  for (int j = 0; j < N; ++j)
-#pragma unroll
-    for (int k = 0; k < 12; ++k) s = fma(v[j][k].i, v[j][k].i, fma(v[j][k].r, v[j][k].r, s));
-  return double(s);
-}
-
 // ------------------------------------------------------------------ Shamir 5D terms
 // out(s) = a5 psi(s) - k D(s) - [P- psi(s+1) + P+ psi(s-1)]       (dag = 0)
 // out(s) = a5 psi(s) - k D(s) - [P+ psi(s+1) + P- psi(s-1)]       (dag = 1)
@@ -690,7 +662,7 @@ template <int PIN, int POUT, int DAG, int N, int EPI, bool SMEM = false, class T
 __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, int s0, int LsE, int LsP,
                                             cpx<T> (&v)[N][12], float& part, double& dpart,
                                             const void* rows = nullptr) {
-  if constexpr (EPI == 1 && DAG == 1 && N == 2 && PIN != GBDW_DS) {
+  if constexpr (EPI == 1 && DAG == 1 && N == 2) {
     if (p.mob) mobius_adj_hop(p, s0, v);
   }
   if constexpr (EPI >= 1) dwf_epilogue<PIN, DAG, N, SMEM>(p, site, s0, v, rows);
@@ -731,7 +703,7 @@ __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, i
     dpart = s;
   } else {
     part = store_spinor<POUT, N>(p.out, p.out_norm, site, s0, LsE, LsP, v);
-    if constexpr (POUT == GBDW_F64 || POUT == GBDW_DS) dpart = sumsq<N>(v);
+    if constexpr (POUT == GBDW_F64) dpart = sumsq<N>(v);
   }
 }
 
@@ -759,6 +731,23 @@ __device__ __forceinline__ void dhop_thread(const DhopParams& p, unsigned site, 
   GBDW_LEG(0) GBDW_LEG(4) GBDW_LEG(1) GBDW_LEG(5) GBDW_LEG(2) GBDW_LEG(6) GBDW_LEG(3) GBDW_LEG(7)
 #undef GBDW_LEG
   acc.unpack(out);
+}
+
+// t-bricks: the sweep visits sites (t brick, z, y, x, t inside the brick), so a site's neighbours
+// along t are read within a few sites of each other instead of a whole 3D volume apart (periodic
+// lattice, Lt a multiple of the brick)
+__device__ __forceinline__ unsigned brick_site(const DhopParams& p, unsigned j) {
+  const unsigned B = unsigned(p.brick);
+  const unsigned tin = j % B;
+  j /= B;
+  const unsigned Lx = unsigned(p.dims[0]), Ly = unsigned(p.dims[1]), Lz = unsigned(p.dims[2]);
+  const unsigned x = j % Lx;
+  j /= Lx;
+  const unsigned y = j % Ly;
+  j /= Ly;
+  const unsigned z = j % Lz;
+  const unsigned tb = j / Lz;
+  return x + Lx * (y + Ly * (z + Lz * (tb * B + tin)));
 }
 
 // EPI 0: out = Dhop(in) ; EPI 1: out = M(in) (Shamir).  |out|^2 fused when p.partials != 0.
@@ -797,21 +786,7 @@ __global__ void __launch_bounds__(MINB > 0 ? MAXT : 256, MINB > 0 ? MINB : 1) k_
         s0 = int(tile) * p.TE + int(r - site * GT) * N;
       }
       if (p.brick > 1) {
-        // t-bricks: the sweep visits sites (t brick, z, y, x, t inside the brick), so a site's
-        // neighbours along t are read within a few sites of each other instead of a whole 3D
-        // volume apart (periodic lattice, Lt a multiple of the brick)
-        unsigned j = site;
-        const unsigned B = unsigned(p.brick);
-        const unsigned tin = j % B;
-        j /= B;
-        const unsigned Lx = unsigned(p.dims[0]), Ly = unsigned(p.dims[1]), Lz = unsigned(p.dims[2]);
-        const unsigned x = j % Lx;
-        j /= Lx;
-        const unsigned y = j % Ly;
-        j /= Ly;
-        const unsigned z = j % Lz;
-        const unsigned tb = j / Lz;
-        site = x + Lx * (y + Ly * (z + Lz * (tb * B + tin)));
+        site = brick_site(p, site);
       }
     }
     if constexpr (BLK) {
@@ -833,7 +808,7 @@ __global__ void __launch_bounds__(MINB > 0 ? MAXT : 256, MINB > 0 ? MINB : 1) k_
     finish_site<PIN, POUT, DAG, N, EPI>(p, site, s0, p.LsE, p.LsP, acc, part, dpart);
   }
   if (p.partials) {
-    double v[1] = {(POUT == GBDW_F64 || POUT == GBDW_DS || (EPI >= 2 && EPI <= 4)) ? dpart : double(part)};
+    double v[1] = {(POUT == GBDW_F64 || (EPI >= 2 && EPI <= 4)) ? dpart : double(part)};
     block_partial<1>(v, p.partials);
   }
 }

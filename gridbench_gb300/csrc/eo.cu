@@ -104,11 +104,11 @@ __device__ __forceinline__ void m5_sweeps(const V& v, int Ls, T ia5, T g, T mf, 
 #pragma unroll(LSC > 0 ? LSC : 4)
   for (int k = 1; k < Ls; ++k) {
     const cpx<T> x = v(s0 + k * ds);
-    w = {::fma(w.r, ia5, x.r), ::fma(w.i, ia5, x.i)};
+    w = {fma(w.r, ia5, x.r), fma(w.i, ia5, x.i)};
   }
   const T c = -mf * ia5;
   const cpx<T> x0 = v(s0);
-  cpx<T> prev = {g * ::fma(c, w.r, x0.r), g * ::fma(c, w.i, x0.i)};
+  cpx<T> prev = {g * fma(c, w.r, x0.r), g * fma(c, w.i, x0.i)};
   y[s0] = prev;
 #pragma unroll(LSC > 0 ? LSC : 4)
   for (int k = 1; k < Ls; ++k) {

@@ -13,13 +13,8 @@
 // per-slice FP32 norm held in norm[site*LsE + e].
 #pragma once
 #include "common.cuh"
-#include "dsfloat.cuh"
 
 namespace gbdw {
-
-// Internal precision tag of the double-single operator: FP64 storage (the F64 layout), arithmetic
-// on FP32 pairs (dsfloat.cuh), links from the gauge field's split copy.
-constexpr int GBDW_DS = 7;
 
 __host__ __device__ inline int padded_slices(int prec, int LsE) {
   return prec == GBDW_F64 ? LsE : LsE + (LsE & 1);
@@ -75,18 +70,6 @@ struct Elem<GBDW_F32> {
     f[2] = im;
   }
 };
-// DS: FP64 storage, split into pairs on load and joined on store.
-template <>
-struct Elem<GBDW_DS> {
-  template <bool SMEM = false>
-  __device__ static cpx<dsf> ld(const void* b, int64_t row, int e, int LsP) {
-    const double2 a = ldv<SMEM>((const double2*)b + row * LsP + e);
-    return {ds_split(a.x), ds_split(a.y)};
-  }
-  __device__ static void st(void* b, int64_t row, int e, int LsP, dsf re, dsf im) {
-    ((double2*)b)[row * LsP + e] = make_double2(double(re), double(im));
-  }
-};
 // F16: returns / takes the stored (norm-scaled) values.
 template <>
 struct Elem<GBDW_F16> {
@@ -107,10 +90,10 @@ struct Elem<GBDW_F16> {
 // e0 % N == 0; for N >= 2 the slices come in whole pairs (e0 even).
 template <int P, int N, bool SMEM = false>
 struct Vec {
-  using T = typename std::conditional<P == GBDW_F64, double, typename std::conditional<P == GBDW_DS, dsf, float>::type>::type;
+  using T = typename std::conditional<P == GBDW_F64, double, float>::type;
 
   __device__ static void load(const void* b, int64_t row, int e0, int LsP, cpx<T> (&v)[N]) {
-    if constexpr (P == GBDW_F64 || P == GBDW_DS || N == 1) {
+    if constexpr (P == GBDW_F64 || N == 1) {
 #pragma unroll
       for (int j = 0; j < N; ++j) v[j] = Elem<P>::template ld<SMEM>(b, row, e0 + j, LsP);
     } else {
@@ -127,7 +110,7 @@ struct Vec {
   // From shared memory the pair is loaded whole, one access instead of two; from global memory, where
   // the line is in L1, the wider access costs more (M at 16^4 x 16 in form 3: 64.3 -> 66.6 us).
   __device__ static cpx<T> one(const void* b, int64_t row, int e, int second, int LsP) {
-    if constexpr (P == GBDW_F64 || P == GBDW_DS || N == 1 || !SMEM) {
+    if constexpr (P == GBDW_F64 || N == 1 || !SMEM) {
       return Elem<P>::template ld<SMEM>(b, row, e, LsP);
     } else {
       cp2 q[1];
@@ -161,7 +144,7 @@ struct Vec {
   }
   // F64 / F32 stores
   __device__ static void store(void* b, int64_t row, int e0, int LsP, const cpx<T> (&v)[N]) {
-    if constexpr (P == GBDW_F64 || P == GBDW_DS || N == 1) {
+    if constexpr (P == GBDW_F64 || N == 1) {
 #pragma unroll
       for (int j = 0; j < N; ++j) Elem<P>::st(b, row, e0 + j, LsP, v[j].r, v[j].i);
     } else {
