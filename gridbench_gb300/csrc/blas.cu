@@ -172,13 +172,26 @@ __global__ void k_cg_r(double alpha, FieldOut r, FieldRef ap, int64_t nsite, int
   grid_sum<1>(acc, red.partials, red.counter, red.result);
 }
 
+// alpha and beta of the vector update, from the host or from the fused step's device scalars
+struct CgStep {
+  double alpha, beta;
+  const double* dev;
+  __device__ __forceinline__ bool go() {
+    if (!dev) return true;
+    alpha = __ldg(dev + CG_ALPHA);
+    beta = __ldg(dev + CG_BETA);
+    return __ldg(dev + CG_GO) != 0.0;
+  }
+};
+
 // x += alpha p ; p = r + beta p (both with the old p) ; optionally q = p
 template <int PX, int PP, int PR, int PQ>
-__global__ void k_cg_xp(double alpha, double beta, FieldOut x, FieldOut p, FieldRef r, FieldOut q, int64_t nsite,
+__global__ void k_cg_xp(CgStep cg, FieldOut x, FieldOut p, FieldRef r, FieldOut q, int64_t nsite,
                         int LsE) {
   using T = typename Calc<(PX == GBDW_F64 || PR == GBDW_F64) ? GBDW_F64 : GBDW_F32>::T;
   const int64_t n = nsite * LsE;
-  const T al = T(alpha), be = T(beta);
+  if (!cg.go()) return;
+  const T al = T(cg.alpha), be = T(cg.beta);
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     const int64_t site = i / LsE;
     const int e = int(i - site * LsE);
@@ -253,10 +266,11 @@ __device__ __forceinline__ void ld_pair(const void* d, const float* nrm, int64_t
 }
 
 template <int PX, int PP, int PR>
-__global__ void k_cg_xp_pairs(double alpha, double beta, FieldOut x, FieldOut p, FieldRef r, int64_t nsite, int LsE) {
+__global__ void k_cg_xp_pairs(CgStep cg, FieldOut x, FieldOut p, FieldRef r, int64_t nsite, int LsE) {
   const int G = LsE / 2;
   const int64_t n = nsite * G;
-  const float al = float(alpha), be = float(beta);
+  if (!cg.go()) return;
+  const float al = float(cg.alpha), be = float(cg.beta);
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     const int64_t site = i / G;
     const int e0 = int(i - site * G) * 2;
@@ -412,8 +426,10 @@ __global__ void k_xmy_norm_flat(const double2* __restrict__ b, const double2* __
 
 // x += alpha p ; p = r + beta p, all FP64, and q = p in the FP32 pair layout: one thread per slice
 // pair of a row, which is two FP64 vectors side by side and one FP32 vector
-__global__ void k_cg_xp_f64_pairs(double alpha, double beta, double2* __restrict__ x, double2* __restrict__ p,
+__global__ void k_cg_xp_f64_pairs(CgStep cg, double2* __restrict__ x, double2* __restrict__ p,
                                   const double2* __restrict__ r, float4* __restrict__ q, int64_t npair) {
+  if (!cg.go()) return;
+  const double alpha = cg.alpha, beta = cg.beta;
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < npair; i += int64_t(gridDim.x) * blockDim.x) {
     const double2 p0 = p[2 * i], p1 = p[2 * i + 1], x0 = x[2 * i], x1 = x[2 * i + 1];
     const double2 r0 = __ldg(r + 2 * i), r1 = __ldg(r + 2 * i + 1);
@@ -543,17 +559,19 @@ int blas_cg_r(double alpha, gbdw_field* r, const gbdw_field* ap, double* rr) {
   return reduce_fetch(red, 1, rr);
 }
 
-int blas_cg_xp(double alpha, double beta, gbdw_field* x, gbdw_field* p, const gbdw_field* r, gbdw_field* q) {
+int blas_cg_xp(double alpha, double beta, gbdw_field* x, gbdw_field* p, const gbdw_field* r, gbdw_field* q,
+               const double* dev) {
   const int64_t ns = r->lat->nsite;
   const int L = r->LsE;
+  const CgStep cg{alpha, beta, dev};
   if (!q && pairs_ok(x) && pairs_ok(p) && pairs_ok(r) && x->prec == GBDW_F32) {
     const unsigned g = unsigned(grid_pairs(r));
     if (p->prec == GBDW_F16 && r->prec == GBDW_F16)
-      k_cg_xp_pairs<GBDW_F32, GBDW_F16, GBDW_F16><<<g, kThreads, 0, stream()>>>(alpha, beta, out(x), out(p), ref(r), ns, L);
+      k_cg_xp_pairs<GBDW_F32, GBDW_F16, GBDW_F16><<<g, kThreads, 0, stream()>>>(cg, out(x), out(p), ref(r), ns, L);
     else if (p->prec == GBDW_F16 && r->prec == GBDW_F32)
-      k_cg_xp_pairs<GBDW_F32, GBDW_F16, GBDW_F32><<<g, kThreads, 0, stream()>>>(alpha, beta, out(x), out(p), ref(r), ns, L);
+      k_cg_xp_pairs<GBDW_F32, GBDW_F16, GBDW_F32><<<g, kThreads, 0, stream()>>>(cg, out(x), out(p), ref(r), ns, L);
     else if (p->prec == GBDW_F32 && r->prec == GBDW_F32)
-      k_cg_xp_pairs<GBDW_F32, GBDW_F32, GBDW_F32><<<g, kThreads, 0, stream()>>>(alpha, beta, out(x), out(p), ref(r), ns, L);
+      k_cg_xp_pairs<GBDW_F32, GBDW_F32, GBDW_F32><<<g, kThreads, 0, stream()>>>(cg, out(x), out(p), ref(r), ns, L);
     else {
       set_error("blas_cg_xp: unsupported precision combination");
       return GBDW_ERR_INVALID;
@@ -565,7 +583,7 @@ int blas_cg_xp(double alpha, double beta, gbdw_field* x, gbdw_field* p, const gb
       (!q || q->prec == GBDW_F32)) {
     const int64_t npair = ns * 12 * int64_t(L / 2);
     k_cg_xp_f64_pairs<<<unsigned(grid_flat(npair)), kThreads, 0, stream()>>>(
-        alpha, beta, (double2*)x->d, (double2*)p->d, (const double2*)r->d, q ? (float4*)q->d : nullptr, npair);
+        cg, (double2*)x->d, (double2*)p->d, (const double2*)r->d, q ? (float4*)q->d : nullptr, npair);
     GBDW_LAUNCHED();
     return GBDW_OK;
   }
@@ -575,7 +593,7 @@ int blas_cg_xp(double alpha, double beta, gbdw_field* x, gbdw_field* p, const gb
   const int key = ((x->prec * 4 + p->prec) * 4 + r->prec) * 8 + (qp + 1);
 #define GBDW_XP(PX, PP, PR, PQ)                                                                              \
   case ((PX * 4 + PP) * 4 + PR) * 8 + (PQ + 1):                                                              \
-    k_cg_xp<PX, PP, PR, PQ><<<unsigned(g), kThreads, 0, stream()>>>(alpha, beta, out(x), out(p), ref(r), qo, ns, L); \
+    k_cg_xp<PX, PP, PR, PQ><<<unsigned(g), kThreads, 0, stream()>>>(cg, out(x), out(p), ref(r), qo, ns, L); \
     break;
   switch (key) {
     GBDW_XP(GBDW_F64, GBDW_F64, GBDW_F64, -1)

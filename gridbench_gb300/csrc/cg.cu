@@ -38,10 +38,10 @@ struct Fields {
 
 // out = A in, and |M in|^2 (= <in, A in>) into pap when non-null.
 using Op = std::function<int(gbdw_field* out, const gbdw_field* in, double* pap)>;
-// One CG step's operator with the residual update fused into its last pass:
-//   r -= alpha A p with alpha = rr / <p, A p>; out = {<p, A p>, alpha, |r|^2}.  sink: a field of
-//   p's lattice and precision the passes may name as their output.
-using FusedOp = std::function<int(const gbdw_field* p, gbdw_field* sink, gbdw_field* r, double rr, double out[3])>;
+// One CG step's operator with the residual update fused into its last pass, queued:
+//   r -= alpha A p with alpha = rr / <p, A p>, the step's scalars in cg_scalars().  sink: a field of
+// p's lattice and precision the passes may name as their output.
+using FusedOp = std::function<int(const gbdw_field* p, gbdw_field* sink, gbdw_field* r, const CgRule& rule)>;
 
 struct Problem {
   const gbdw_lattice* lat;  // lattice of x and b
@@ -129,13 +129,22 @@ int cg_core(const Problem& P, int mode, gbdw_field* x, const gbdw_field* b, cons
   const bool fused = P.fused && mode != GBDW_CG_DOUBLE;
   while (!converged && it < prm->max_iter) {
     double pap = 0.0, alpha = 0.0, rr_new = 0.0;
+    bool updated = false;  // x and p have been updated already
     if (fused) {
-      // A p, alpha = rr / <p, A p> on the device, and r -= alpha A p in the last pass
-      double s[3];
-      TRY(P.fused(pq ? pq : p, ap, rs, rr, s));
-      pap = s[0];
-      alpha = s[1];
-      rr_new = s[2];
+      // A p, alpha = rr / <p, A p> on the device, r -= alpha A p in the last pass, and the common
+      // vector update, which the device skips when its scalars call for the host.  The host reads them
+      // while that update runs and queues the next step behind it: waiting for them first left the GPU
+      // idle for 28 us a step at 12^4 x 8 (of 163) and 45 us through the Schur complement at 16^4 x 16
+      double s[CG_SCALARS];
+      double* dev = cg_scalars();
+      TRY(P.fused(pq ? pq : p, ap, rs, CgRule{rr, delta * delta * maxrr, stop}));
+      TRY(fetch_queue(dev, CG_SCALARS));
+      TRY(blas_cg_xp(0.0, 0.0, xs, p, rs, pq, dev));
+      TRY(fetch_wait(CG_SCALARS, s));
+      pap = s[CG_PAP];
+      alpha = s[CG_ALPHA];
+      rr_new = s[CG_RR];
+      updated = s[CG_GO] != 0.0;
     } else {
       TRY(P.sloppy(ap, pq ? pq : p, &pap));
     }
@@ -157,8 +166,7 @@ int cg_core(const Problem& P, int mode, gbdw_field* x, const gbdw_field* b, cons
     }
     if (!(rr_new < delta * delta * maxrr || rr_new <= stop)) {
       // the common iteration: x and p updated in one pass over the vectors
-      const double beta = rr_new / rr;
-      TRY(blas_cg_xp(alpha, beta, xs, p, rs, pq));
+      if (!updated) TRY(blas_cg_xp(alpha, rr_new / rr, xs, p, rs, pq));
       rr = rr_new;
       if (rr > maxrr) maxrr = rr;
       continue;
@@ -272,8 +280,8 @@ extern "C" int gbdw_cg_solve(const gbdw_gauge* g64, const gbdw_gauge* g32, const
     return gbdw_dwf_mdagm(gop, out, tmps ? tmps : tmp64, in, M5, mf, pap);
   };
   if (tmps)
-    P.fused = [&](const gbdw_field* in, gbdw_field*, gbdw_field* r, double rr, double out[3]) {
-      return mdagm_residual(gop, tmps, r, in, M5, mf, rr, out);
+    P.fused = [&](const gbdw_field* in, gbdw_field*, gbdw_field* r, const CgRule& rule) {
+      return mdagm_residual(gop, tmps, r, in, M5, mf, rule);
     };
   return cg_core(P, mode, x, b, prm, stats, who);
 }
@@ -495,8 +503,8 @@ extern "C" int gbdw_cg_solve_eo(const gbdw_gauge* const g64[2], const gbdw_gauge
     return mpcdagmpc(gpo, gqe, out, tps, tq1s, tq2s, in, M5, mf, pap);
   };
   if (op_prec != GBDW_F64)
-    P.fused = [&](const gbdw_field* in, gbdw_field* sink, gbdw_field* r, double rr, double out[3]) {
-      return mpcdagmpc_residual(gpo, gqe, sink, tps, tq1s, tq2s, r, in, M5, mf, rr, out);
+    P.fused = [&](const gbdw_field* in, gbdw_field* sink, gbdw_field* r, const CgRule& rule) {
+      return mpcdagmpc_residual(gpo, gqe, sink, tps, tq1s, tq2s, r, in, M5, mf, rule);
     };
   gbdw_cg_stats S{};
   const int cst = cg_core(P, mode, xo, co, prm, &S, who);

@@ -271,13 +271,25 @@ struct Reduce {
   double* result;
 };
 int reduce_scratch(int64_t nblocks, int width, Reduce* r);
-// result[0] = sum of partials[0..n) in a fixed order (one CTA, on the library stream); with
-// alpha_out, also alpha_out[0] = num / result[0] (the CG step length, computed on the device)
-int sum_partials(const double* partials, int64_t n, double* result, double num = 0.0, double* alpha_out = nullptr);
-// three device doubles for one fused CG step: <p, A p>, alpha, |r|^2 after the update
+// One fused CG step's device scalars (cg_scalars): <p, A p>, alpha, |r|^2 after the update, beta, and
+// whether the step goes on with the common vector update (1) or the host takes over (0).
+enum { CG_PAP = 0, CG_ALPHA = 1, CG_RR = 2, CG_BETA = 3, CG_GO = 4, CG_SCALARS = 5 };
 double* cg_scalars();
+// The rule of that last scalar: the step's residual is finite, <p, A p> positive, and |r|^2 neither
+// below `update` (a reliable update is due) nor at most `stop`; rr: |r|^2 before the step.
+struct CgRule {
+  double rr, update, stop;
+};
+// result[0] = sum of partials[0..n) in a fixed order (on the library stream); with alpha_out, also
+// alpha_out[0] = num / result[0] (the CG step length, computed on the device); with rule, result is
+// cg_scalars() + CG_RR and the scalars after it are set
+int sum_partials(const double* partials, int64_t n, double* result, double num = 0.0, double* alpha_out = nullptr,
+                 const CgRule* rule = nullptr);
 // copies n <= 8 device doubles to the host (synchronising the library stream)
 int fetch_doubles(const double* dev, int n, double* host);
+// the same in two halves: work queued between them runs while the host waits for the values
+int fetch_queue(const double* dev, int n);
+int fetch_wait(int n, double* host);
 int reduce_fetch(const Reduce& r, int width, double* host);
 
 }  // namespace gbdw

@@ -37,7 +37,8 @@ struct SlotTable {
 SlotTable g_scratch_own;
 std::map<cudaStream_t, SlotTable> g_scratch_user;
 SlotTable& slot_table() { return g_have_user_stream ? g_scratch_user[g_user_stream] : g_scratch_own; }
-double* g_pinned = nullptr;
+double* g_pinned = nullptr;         // 64 doubles: fetches use [0, 32), queued fetches the rest
+cudaEvent_t g_fetched = nullptr;    // the last queued fetch
 }  // namespace
 
 void set_error(const std::string& msg) { g_error = msg; }
@@ -159,7 +160,7 @@ namespace {
 constexpr int kSumShare = 4096;
 __global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict__ partials, int64_t n, double* sums,
                                                        unsigned* counter, double* result, double num,
-                                                       double* alpha_out) {
+                                                       double* alpha_out, CgRule rule) {
   __shared__ double sh[32][1];
   __shared__ bool last;
   const int64_t first = n * blockIdx.x / gridDim.x, end = n * (blockIdx.x + 1) / gridDim.x;
@@ -187,11 +188,17 @@ __global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict_
   if (threadIdx.x == 0) {
     result[0] = v[0];
     if (alpha_out) alpha_out[0] = num / v[0];
+    if (rule.rr > 0.0) {
+      double* s = result - CG_RR;
+      s[CG_BETA] = v[0] / rule.rr;
+      const bool go = s[CG_PAP] > 0.0 && isfinite(s[CG_PAP]) && isfinite(v[0]) && !(v[0] < rule.update) && !(v[0] <= rule.stop);
+      s[CG_GO] = go ? 1.0 : 0.0;
+    }
   }
 }
 }  // namespace
 
-int sum_partials(const double* partials, int64_t n, double* result, double num, double* alpha_out) {
+int sum_partials(const double* partials, int64_t n, double* result, double num, double* alpha_out, const CgRule* rule) {
   int64_t ctas = (n + kSumShare - 1) / kSumShare;
   if (ctas > 64) ctas = 64;
   char* s = (char*)scratch(4096, 1);  // CTA sums at +1024, their counter (zero between launches) at +1536
@@ -201,7 +208,7 @@ int sum_partials(const double* partials, int64_t n, double* result, double num, 
   }
   const int threads = n >= 4096 ? 1024 : 256;
   k_sum_partials<<<unsigned(ctas), threads, 0, stream()>>>(partials, n, (double*)(s + 1024), (unsigned*)(s + 1536),
-                                                           result, num, alpha_out);
+                                                           result, num, alpha_out, rule ? *rule : CgRule{0.0, 0.0, 0.0});
   GBDW_LAUNCHED();
   return GBDW_OK;
 }
@@ -212,6 +219,19 @@ int fetch_doubles(const double* dev, int n, double* host) {
   GBDW_CUDA(cudaMemcpyAsync(g_pinned, dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, stream()));
   GBDW_CUDA(cudaStreamSynchronize(stream()));
   for (int k = 0; k < n; ++k) host[k] = g_pinned[k];
+  return GBDW_OK;
+}
+
+int fetch_queue(const double* dev, int n) {
+  if (!g_fetched) GBDW_CUDA(cudaEventCreateWithFlags(&g_fetched, cudaEventDisableTiming));
+  GBDW_CUDA(cudaMemcpyAsync(g_pinned + 32, dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, stream()));
+  GBDW_CUDA(cudaEventRecord(g_fetched, stream()));
+  return GBDW_OK;
+}
+
+int fetch_wait(int n, double* host) {
+  GBDW_CUDA(cudaEventSynchronize(g_fetched));
+  for (int k = 0; k < n; ++k) host[k] = g_pinned[32 + k];
   return GBDW_OK;
 }
 

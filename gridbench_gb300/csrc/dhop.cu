@@ -230,7 +230,7 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
     if (st) return st;
     if (reduce) {
       double* to = (ex && ex->sum_to) ? ex->sum_to : red.result;
-      if (int s2 = sum_partials(red.partials, blocks_ds, to, ex ? ex->num : 0.0, ex ? ex->alpha_to : nullptr)) return s2;
+      if (int s2 = sum_partials(red.partials, blocks_ds, to, ex ? ex->num : 0.0, ex ? ex->alpha_to : nullptr, ex ? ex->rule : nullptr)) return s2;
       if (norm2 && fetch) return ex && ex->sum_to ? fetch_doubles(to, 1, norm2) : reduce_fetch(red, 1, norm2);
     }
     return GBDW_OK;
@@ -244,7 +244,7 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
   if (reduce) {
     // the kernel leaves one partial per CTA; one CTA sums them in a fixed order
     double* to = (ex && ex->sum_to) ? ex->sum_to : red.result;
-    if (int s2 = sum_partials(red.partials, blocks, to, ex ? ex->num : 0.0, ex ? ex->alpha_to : nullptr)) return s2;
+    if (int s2 = sum_partials(red.partials, blocks, to, ex ? ex->num : 0.0, ex ? ex->alpha_to : nullptr, ex ? ex->rule : nullptr)) return s2;
     if (norm2 && fetch) return ex && ex->sum_to ? fetch_doubles(to, 1, norm2) : reduce_fetch(red, 1, norm2);
   }
   return GBDW_OK;
@@ -283,7 +283,7 @@ bool tma_shape(int prec, int LsE, DhopLaunch L, int* NS, int* threads, size_t* s
 }
 
 int mdagm_residual(const gbdw_gauge* g, gbdw_field* t, gbdw_field* r, const gbdw_field* p, double M5, double mf,
-                   double rr, double out[3]) {
+                   const CgRule& rule) {
   if (int st = check_operands(g, t, p, true)) return st;
   double* s = cg_scalars();
   if (!s) {
@@ -291,18 +291,18 @@ int mdagm_residual(const gbdw_gauge* g, gbdw_field* t, gbdw_field* r, const gbdw
     return GBDW_ERR_ALLOC;
   }
   DhopExtra e1;
-  e1.sum_to = s;
-  e1.num = rr;
-  e1.alpha_to = s + 1;
+  e1.sum_to = s + CG_PAP;
+  e1.num = rule.rr;
+  e1.alpha_to = s + CG_ALPHA;
   e1.tune_key = cg_step_key(r->prec);
   if (int st = run_dhop(g, t, p, 0, 1, 5.0 - M5, mf, nullptr, false, nullptr, 0.5, &e1)) return st;
   DhopExtra e2;
   e2.r = r;
-  e2.alpha = s + 1;
-  e2.sum_to = s + 2;
+  e2.alpha = s + CG_ALPHA;
+  e2.sum_to = s + CG_RR;
+  e2.rule = &rule;
   e2.tune_key = e1.tune_key;
-  if (int st = run_dhop(g, t, t, 1, 1, 5.0 - M5, mf, nullptr, false, nullptr, 0.5, &e2)) return st;
-  return fetch_doubles(s, 3, out);
+  return run_dhop(g, t, t, 1, 1, 5.0 - M5, mf, nullptr, false, nullptr, 0.5, &e2);
 }
 
 }  // namespace gbdw

@@ -319,8 +319,8 @@ int mpcdagmpc(const gbdw_gauge* gp, const gbdw_gauge* gq, gbdw_field* out, gbdw_
 }
 
 int mpcdagmpc_residual(const gbdw_gauge* gp, const gbdw_gauge* gq, gbdw_field* sink, gbdw_field* tp, gbdw_field* tq1,
-                       gbdw_field* tq2, gbdw_field* r, const gbdw_field* in, double M5, double mf, double rr,
-                       double out[3]) {
+                       gbdw_field* tq2, gbdw_field* r, const gbdw_field* in, double M5, double mf,
+                       const CgRule& rule) {
   if (!gp || !gq || gq->lat != gp->lat->partner || !tp || !tq1 || !tq2 || !sink || tp == in || sink == tp ||
       sink == in) {
     set_error("fused Schur step: partner gauge halves, distinct temporaries");
@@ -332,20 +332,20 @@ int mpcdagmpc_residual(const gbdw_gauge* gp, const gbdw_gauge* gq, gbdw_field* s
     return GBDW_ERR_ALLOC;
   }
   DhopExtra e1;
-  e1.sum_to = s;
-  e1.num = rr;
-  e1.alpha_to = s + 1;
+  e1.sum_to = s + CG_PAP;
+  e1.num = rule.rr;
+  e1.alpha_to = s + CG_ALPHA;
   if (int st = hop_eo(gq, tq1, in, 0, nullptr, M5, mf, 0.5, nullptr, true)) return st;
   if (int st = m5inv(tq2, tq1, M5, mf, 0)) return st;
   if (int st = hop_eo(gp, tp, tq2, 0, in, M5, mf, 0.25, nullptr, false, &e1)) return st;
   DhopExtra e2;
   e2.r = r;
-  e2.alpha = s + 1;
-  e2.sum_to = s + 2;
+  e2.alpha = s + CG_ALPHA;
+  e2.sum_to = s + CG_RR;
+  e2.rule = &rule;
   if (int st = hop_eo(gq, tq1, tp, 1, nullptr, M5, mf, 0.5, nullptr, true)) return st;
   if (int st = m5inv(tq2, tq1, M5, mf, 1)) return st;
-  if (int st = hop_eo(gp, sink, tq2, 1, tp, M5, mf, 0.25, nullptr, false, &e2)) return st;
-  return fetch_doubles(s, 3, out);
+  return hop_eo(gp, sink, tq2, 1, tp, M5, mf, 0.25, nullptr, false, &e2);
 }
 
 int field_pick(gbdw_field* half, const gbdw_field* full) {

@@ -17,12 +17,12 @@ int mpc(const gbdw_gauge* gp, const gbdw_gauge* gq, gbdw_field* out, gbdw_field*
 // out = Mpc^dag Mpc in, pap = |Mpc in|^2
 int mpcdagmpc(const gbdw_gauge* gp, const gbdw_gauge* gq, gbdw_field* out, gbdw_field* tp, gbdw_field* tq1,
               gbdw_field* tq2, const gbdw_field* in, double M5, double mf, double* pap);
-// Mpc^dag Mpc with the CG update of its last pass fused in (see mdagm_residual): tp = Mpc in,
-// s[0] = |tp|^2, s[1] = alpha = rr / s[0], r -= alpha Mpc^dag tp, s[2] = |r|^2 -> out[3].
+// Mpc^dag Mpc with the CG update of its last pass fused in, queued (see mdagm_residual): tp = Mpc in,
+// r -= alpha Mpc^dag tp, the step's scalars in cg_scalars().
 // sink: any field of in's lattice and precision (written by nothing, named as the output).
 int mpcdagmpc_residual(const gbdw_gauge* gp, const gbdw_gauge* gq, gbdw_field* sink, gbdw_field* tp, gbdw_field* tq1,
-                       gbdw_field* tq2, gbdw_field* r, const gbdw_field* in, double M5, double mf, double rr,
-                       double out[3]);
+                       gbdw_field* tq2, gbdw_field* r, const gbdw_field* in, double M5, double mf,
+                       const CgRule& rule);
 // Mobius M^dag M on a full lattice (mobius.cu); t, tmp temporaries like in; pap = |M in|^2
 int mobius_mdagm(const gbdw_gauge* g, gbdw_field* out, gbdw_field* t, gbdw_field* tmp, const gbdw_field* in,
                  double b, double c, double M5, double mf, double* pap);

@@ -278,12 +278,11 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
       float best_cg_ms = 1e30f;
       for (const DhopLaunch& L : shortlist) {
         set_tuned_launch(g->prec, in->prec, in->LsE, key, L);
-        double o3[3];
-        for (int w = 0; w < 2 && !status; ++w) status = mdagm_residual(g, out, r, in, 1.8, 0.01, 1.0, o3);
+        for (int w = 0; w < 2 && !status; ++w) status = mdagm_residual(g, out, r, in, 1.8, 0.01, CgRule{1.0, 0.0, 0.0});
         if (status) break;
         const int reps = 6;
         cudaEventRecord(a, stream());
-        for (int k = 0; k < reps && !status; ++k) status = mdagm_residual(g, out, r, in, 1.8, 0.01, 1.0, o3);
+        for (int k = 0; k < reps && !status; ++k) status = mdagm_residual(g, out, r, in, 1.8, 0.01, CgRule{1.0, 0.0, 0.0});
         cudaEventRecord(b, stream());
         cudaEventSynchronize(b);
         if (status) break;

@@ -14,6 +14,7 @@ struct DhopExtra {
   double* sum_to = nullptr;         // device: where the fused |.|^2 goes (default: the reduce result)
   double num = 0.0;                 // with alpha_to: alpha_to = num / sum
   double* alpha_to = nullptr;       // device
+  const CgRule* rule = nullptr;     // with sum_to = cg_scalars() + CG_RR
   double c5 = 1.0;                  // the epilogue's 5th-dimension hopping coefficient
   // Mobius operator in one pass: A(mb, mc) on the loaded neighbours (dag 0, FP32) or A(mb, mc)^dag
   // on DhopDag in before the epilogue (dag 1); epi 1, one right-hand side, Ls a power of two <= 64
@@ -33,11 +34,11 @@ bool find_tuned_launch(int gprec, int sprec, int LsE, int epi, DhopLaunch* L);
 int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag, int epi, double a5, double mf,
              double* norm2, bool fetch = true, const gbdw_field* cen = nullptr, double khop = 0.5,
              const DhopExtra* ex = nullptr);
-// The two passes of M^dag M with the CG update of the second fused in:
-//   t = M p, s[0] = |t|^2, s[1] = alpha = rr / s[0], r -= alpha M^dag t, s[2] = |r|^2
-// (s = cg_scalars(), fetched into out[3] with one synchronisation).
+// The two passes of M^dag M with the CG update of the second fused in, queued:
+//   t = M p, <p, A p> = |t|^2, alpha = rule.rr / <p, A p>, r -= alpha M^dag t, |r|^2, and the rule's
+// scalars, all in cg_scalars().
 int mdagm_residual(const gbdw_gauge* g, gbdw_field* t, gbdw_field* r, const gbdw_field* p, double M5, double mf,
-                   double rr, double out[3]);
+                   const CgRule& rule);
 int check_operands(const gbdw_gauge* g, const gbdw_field* out, const gbdw_field* in, bool need_single_rhs);
 DhopParams make_params(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in);
 // form 3 (specialised direct) applies: slice pairs, Ls*nrhs = 16 (FP32/FP16) or 12 / 144 (FP32
