@@ -170,8 +170,7 @@ __device__ __forceinline__ void ds_leg(const float4* __restrict__ u, const doubl
 // than their share of the work).
 template <int DAG, int EPI, int MINB>
 __global__ void __launch_bounds__(DS_THREADS, MINB) k_dhop_ds(const DhopParams p) {
-  const unsigned bid = DAG ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
-  const unsigned tid = bid * DS_THREADS + threadIdx.x;
+  const unsigned tid = sweep_block(DAG) * DS_THREADS + threadIdx.x;
   const unsigned LsE = unsigned(p.LsE);
   float part = 0.f;
   double dpart = 0.0;

@@ -733,6 +733,12 @@ __device__ __forceinline__ void dhop_thread(const DhopParams& p, unsigned site, 
   acc.unpack(out);
 }
 
+// The CTA's place in the sweep over sites.  An adjoint pass runs it backwards: what it reads first is
+// what the forward pass before it (M then M^dag, Dhop then DhopDag) wrote last and still holds in L2.
+// A chain of them, us per pass, forwards only -> alternating (TMA warp rings): 16^4 x 16 59.3 -> 57.2,
+// 24^4 x 16 303 -> 289, 32^4 x 16 1016 -> 1014.
+__device__ __forceinline__ unsigned sweep_block(int dag) { return dag ? gridDim.x - 1 - blockIdx.x : blockIdx.x; }
+
 // t-bricks: the sweep visits sites (t brick, z, y, x, t inside the brick), so a site's neighbours
 // along t are read within a few sites of each other instead of a whole 3D volume apart (periodic
 // lattice, Lt a multiple of the brick)
@@ -767,7 +773,8 @@ __global__ void __launch_bounds__(MINB > 0 ? MAXT : 256, MINB > 0 ? MINB : 1) k_
     p.LsP = LSPC;
   }
   const unsigned G = unsigned(p.LsE) / N;
-  const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned bid = sweep_block(DAG);
+  const unsigned tid = bid * blockDim.x + threadIdx.x;
   const bool active = tid < unsigned(p.nsite) * G;
   float part = 0.f;
   double dpart = 0.0;
@@ -792,7 +799,7 @@ __global__ void __launch_bounds__(MINB > 0 ? MAXT : 256, MINB > 0 ? MINB : 1) k_
     if constexpr (BLK) {
       const unsigned l = threadIdx.x / G;  // 0..15 inside the block
       const unsigned hx = unsigned(p.dims[0]) >> 1, hy = unsigned(p.dims[1]) >> 1, hz = unsigned(p.dims[2]) >> 1;
-      unsigned b = blockIdx.x;
+      unsigned b = bid;
       const unsigned bx = b % hx;
       b /= hx;
       const unsigned by = b % hy;

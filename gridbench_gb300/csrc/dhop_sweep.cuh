@@ -130,9 +130,7 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
   const int vol3 = Lx * Ly * Lz;
   const uint32_t row_bytes = uint32_t(p.LsP) * 8;
   const int64_t site_bytes = int64_t(12) * row_bytes, plane_bytes = site_bytes * vol3;
-  // an adjoint pass walks the columns in the opposite order: it usually reads what the forward pass
-  // wrote last, which is still in L2
-  unsigned b = DAG ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  unsigned b = sweep_block(DAG);
   const int tile = int(b % q.ntile);
   b /= q.ntile;
   const int x = int(b % q.nbx) * 2 + xl;

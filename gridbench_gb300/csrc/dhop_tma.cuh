@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) k_dhop_tma(const DhopParams p, int NS) {
   unsigned char* links = smem + STAGES * stage;
   uint64_t* bars = reinterpret_cast<uint64_t*>(links + NS * LB);
   const int tid = threadIdx.x;
-  const int64_t site0 = int64_t(blockIdx.x) * NS;
+  const int64_t site0 = int64_t(sweep_block(DAG)) * NS;
   const int nvalid = int(min(int64_t(NS), p.nsite - site0));
   const int sl = tid / Tps;
   const int s0 = (tid - sl * Tps) * N;
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(256) k_dhop_tmaw(const DhopParams p_) {
   unsigned char* wbase = smem + warp * tmaw_warp_bytes<PIN, GP>(NSW, LsE, LsP, STAGES);
   unsigned char* links = wbase + STAGES * stage;
   uint64_t* bars = reinterpret_cast<uint64_t*>(links + NSW * LB);
-  const int64_t site0 = (int64_t(blockIdx.x) * (blockDim.x >> 5) + warp) * NSW;
+  const int64_t site0 = (int64_t(sweep_block(DAG)) * (blockDim.x >> 5) + warp) * NSW;
   const int nvalid = int(max(int64_t(0), min(int64_t(NSW), p.nsite - site0)));
   const int sl = lane / Tps;
   const int s0 = (lane - sl * Tps) * N;
