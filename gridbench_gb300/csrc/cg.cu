@@ -138,9 +138,9 @@ int cg_core(const Problem& P, int mode, gbdw_field* x, const gbdw_field* b, cons
       double s[CG_SCALARS];
       double* dev = cg_scalars();
       TRY(P.fused(pq ? pq : p, ap, rs, CgRule{rr, delta * delta * maxrr, stop}));
-      TRY(fetch_queue(dev, CG_SCALARS));
+      TRY(cg_scalars_mark());
       TRY(blas_cg_xp(0.0, 0.0, xs, p, rs, pq, dev));
-      TRY(fetch_wait(CG_SCALARS, s));
+      TRY(cg_scalars_wait(s));
       pap = s[CG_PAP];
       alpha = s[CG_ALPHA];
       rr_new = s[CG_RR];

@@ -264,7 +264,8 @@ __device__ __forceinline__ void grid_sum(double (&v)[W], double* partials, unsig
   }
 }
 
-// Scratch slots used for reductions: partial sums and a counter/result block.
+// Scratch slots used for reductions: partial sums and a counter; result is page-locked host memory,
+// valid once the stream has been waited for (reduce_fetch).
 struct Reduce {
   double* partials;
   unsigned* counter;
@@ -282,14 +283,15 @@ struct CgRule {
 };
 // result[0] = sum of partials[0..n) in a fixed order (on the library stream); with alpha_out, also
 // alpha_out[0] = num / result[0] (the CG step length, computed on the device); with rule, result is
-// cg_scalars() + CG_RR and the scalars after it are set
+// cg_scalars() + CG_RR, the scalars after it are set and all of them copied to the host
 int sum_partials(const double* partials, int64_t n, double* result, double num = 0.0, double* alpha_out = nullptr,
                  const CgRule* rule = nullptr);
 // copies n <= 8 device doubles to the host (synchronising the library stream)
 int fetch_doubles(const double* dev, int n, double* host);
-// the same in two halves: work queued between them runs while the host waits for the values
-int fetch_queue(const double* dev, int n);
-int fetch_wait(int n, double* host);
+// the host's copy of a step's scalars in two halves, the first behind the step: work queued between
+// them runs while the host waits
+int cg_scalars_mark();
+int cg_scalars_wait(double* host);
 int reduce_fetch(const Reduce& r, int width, double* host);
 
 }  // namespace gbdw

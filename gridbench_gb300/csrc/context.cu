@@ -37,8 +37,8 @@ struct SlotTable {
 SlotTable g_scratch_own;
 std::map<cudaStream_t, SlotTable> g_scratch_user;
 SlotTable& slot_table() { return g_have_user_stream ? g_scratch_user[g_user_stream] : g_scratch_own; }
-double* g_pinned = nullptr;         // 64 doubles: fetches use [0, 32), queued fetches the rest
-cudaEvent_t g_fetched = nullptr;    // the last queued fetch
+double* g_pinned = nullptr;         // 64 doubles the GPU writes too: sums in [0, 32), CG scalars from 32
+cudaEvent_t g_scalars = nullptr;    // behind the kernel that wrote the last CG scalars
 }  // namespace
 
 void set_error(const std::string& msg) { g_error = msg; }
@@ -139,7 +139,7 @@ void* scratch(size_t bytes, int slot) {
 
 int reduce_scratch(int64_t nblocks, int width, Reduce* r) {
   void* part = scratch(size_t(nblocks) * size_t(width) * sizeof(double), 0);
-  // slot 1: result doubles at +64 (sum_partials at +1024, the device error word at +2048)
+  // slot 1: sum_partials at +1024, the device error word at +2048
   void* ctl = scratch(4096, 1);
   // slot 8: the two-level reduction's counters, 1 + one per group of kReduceGroup blocks
   void* cnt = scratch((size_t(1) + size_t((nblocks + kReduceGroup - 1) / kReduceGroup)) * sizeof(unsigned), 8);
@@ -149,7 +149,8 @@ int reduce_scratch(int64_t nblocks, int width, Reduce* r) {
   }
   r->partials = (double*)part;
   r->counter = (unsigned*)cnt;
-  r->result = (double*)((char*)ctl + 64);
+  // sums go straight to page-locked host memory: a device result and its copy cost 4 us more per call
+  r->result = g_pinned;
   return GBDW_OK;
 }
 
@@ -160,7 +161,7 @@ namespace {
 constexpr int kSumShare = 4096;
 __global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict__ partials, int64_t n, double* sums,
                                                        unsigned* counter, double* result, double num,
-                                                       double* alpha_out, CgRule rule) {
+                                                       double* alpha_out, CgRule rule, double* host) {
   __shared__ double sh[32][1];
   __shared__ bool last;
   const int64_t first = n * blockIdx.x / gridDim.x, end = n * (blockIdx.x + 1) / gridDim.x;
@@ -193,6 +194,7 @@ __global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict_
       s[CG_BETA] = v[0] / rule.rr;
       const bool go = s[CG_PAP] > 0.0 && isfinite(s[CG_PAP]) && isfinite(v[0]) && !(v[0] < rule.update) && !(v[0] <= rule.stop);
       s[CG_GO] = go ? 1.0 : 0.0;
+      for (int k = 0; k < CG_SCALARS; ++k) host[k] = s[k];
     }
   }
 }
@@ -208,7 +210,8 @@ int sum_partials(const double* partials, int64_t n, double* result, double num, 
   }
   const int threads = n >= 4096 ? 1024 : 256;
   k_sum_partials<<<unsigned(ctas), threads, 0, stream()>>>(partials, n, (double*)(s + 1024), (unsigned*)(s + 1536),
-                                                           result, num, alpha_out, rule ? *rule : CgRule{0.0, 0.0, 0.0});
+                                                           result, num, alpha_out, rule ? *rule : CgRule{0.0, 0.0, 0.0},
+                                                           g_pinned + 32);
   GBDW_LAUNCHED();
   return GBDW_OK;
 }
@@ -222,16 +225,15 @@ int fetch_doubles(const double* dev, int n, double* host) {
   return GBDW_OK;
 }
 
-int fetch_queue(const double* dev, int n) {
-  if (!g_fetched) GBDW_CUDA(cudaEventCreateWithFlags(&g_fetched, cudaEventDisableTiming));
-  GBDW_CUDA(cudaMemcpyAsync(g_pinned + 32, dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, stream()));
-  GBDW_CUDA(cudaEventRecord(g_fetched, stream()));
+int cg_scalars_mark() {
+  if (!g_scalars) GBDW_CUDA(cudaEventCreateWithFlags(&g_scalars, cudaEventDisableTiming));
+  GBDW_CUDA(cudaEventRecord(g_scalars, stream()));
   return GBDW_OK;
 }
 
-int fetch_wait(int n, double* host) {
-  GBDW_CUDA(cudaEventSynchronize(g_fetched));
-  for (int k = 0; k < n; ++k) host[k] = g_pinned[32 + k];
+int cg_scalars_wait(double* host) {
+  GBDW_CUDA(cudaEventSynchronize(g_scalars));
+  for (int k = 0; k < CG_SCALARS; ++k) host[k] = g_pinned[32 + k];
   return GBDW_OK;
 }
 
@@ -241,9 +243,8 @@ unsigned* device_error_word() {
 }
 
 int reduce_fetch(const Reduce& r, int width, double* host) {
-  GBDW_CUDA(cudaMemcpyAsync(g_pinned, r.result, size_t(width) * sizeof(double), cudaMemcpyDeviceToHost, stream()));
   GBDW_CUDA(cudaStreamSynchronize(stream()));
-  for (int w = 0; w < width; ++w) host[w] = g_pinned[w];
+  for (int w = 0; w < width; ++w) host[w] = r.result[w];
   return GBDW_OK;
 }
 
