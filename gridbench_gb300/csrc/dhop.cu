@@ -40,10 +40,14 @@ int check_operands(const gbdw_gauge* g, const gbdw_field* out, const gbdw_field*
   return GBDW_OK;
 }
 
+bool slices_ok(const gbdw_field* in, int epi, int spt, int form) {
+  if (in->LsE % spt == 0) return true;
+  return in->prec == GBDW_F32 && spt == 2 && epi <= 1 && (form == 0 || form == 3);
+}
+
 bool form3_ok(const gbdw_field* in, int epi, int spt) {
-  if (in->prec == GBDW_F64 || spt != 2 || in->LsE != in->LsP) return false;
-  if (in->LsE == 16) return true;
-  return in->prec == GBDW_F32 && epi <= 1 && (in->LsE == 12 || in->LsE == 144);
+  if (in->prec == GBDW_F64 || spt != 2) return false;
+  return in->prec == GBDW_F32 ? slices_ok(in, epi, spt, 3) : in->LsE == 16 && in->LsP == 16;
 }
 
 bool blocked_ok(const gbdw_lattice* lat, const gbdw_field* in) {
@@ -81,9 +85,13 @@ int brick_extent(const gbdw_lattice* lat, const DhopLaunch& L) {
 bool mobius_fusable(const gbdw_gauge* g, const gbdw_field* in, int dag) {
   const int Ls = g->lat->Ls;
   // the adjoint (A^dag in the epilogue) in every precision; the forward operator (A on the loaded
-  // neighbours) on FP32 slice pairs
-  return g->lat->fast && (dag || in->prec == GBDW_F32) && in->nrhs == 1 && in->LsE == in->LsP && Ls >= 2 &&
-         Ls <= 64 && (Ls & (Ls - 1)) == 0;
+  // neighbours) on FP32 slice pairs.  Other even Ls: the FP32 adjoint on the warp rings, where a warp
+  // holds whole sites.
+  if (!g->lat->fast || in->nrhs != 1 || in->LsE != in->LsP || Ls < 2 || Ls > 64 || Ls % 2) return false;
+  if ((Ls & (Ls - 1)) == 0) return dag || in->prec == GBDW_F32;
+  int ns, threads;
+  size_t smem;
+  return dag && in->prec == GBDW_F32 && tma_shape(in->prec, in->LsE, DhopLaunch{64, 2, 2, 2}, &ns, &threads, &smem);
 }
 
 DhopParams make_params(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in) {
@@ -164,16 +172,15 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
   // the forward Mobius M (A(b, c) on the loaded neighbours) has the hopping term's access pattern
   // and no Shamir epilogue: it runs on the hopping term's shape
   const int key_epi = (p.mob && epi == 6) ? 0 : tune_epi;
-  DhopLaunch L = tuned_launch(g->prec, in->prec, in->LsE, key_epi);
-  if (g->lat->parity >= 0) find_tuned_launch(g->prec, in->prec, in->LsE, key_epi + EO_KEY, &L);
-  if (ex && ex->tune_key >= 0) find_tuned_launch(g->prec, in->prec, in->LsE, ex->tune_key, &L);
-  if (in->LsE % L.spt != 0) L.spt = 1;
+  DhopLaunch L;
+  bool tuned = find_tuned_launch(g->prec, in->prec, in->LsE, key_epi, &L);
+  if (!tuned) L = untuned_launch(g, in, epi);
+  if (g->lat->parity >= 0) tuned |= find_tuned_launch(g->prec, in->prec, in->LsE, key_epi + EO_KEY, &L);
+  if (ex && ex->tune_key >= 0) tuned |= find_tuned_launch(g->prec, in->prec, in->LsE, ex->tune_key, &L);
   if (p.mob) L.spt = 2;  // the fused adjoint works on slice pairs, one site's pairs in consecutive lanes
-  int NS = 0, tthreads = 0;
-  size_t smem = 0;
-  const bool staged = L.mode == 1 || L.mode == 2;
-  if (staged && !tma_shape(in->prec, in->LsE, L, &NS, &tthreads, &smem)) L.mode = 0;
-  // fall back before fixing the CTA size: the block count below must match the launch
+  if (p.mob && (in->lat->Ls & (in->lat->Ls - 1))) L = DhopLaunch{64, 2, 2, 2};  // whole sites in a warp
+  // untuned hopping terms of a CTA per SM or fewer (dhop_small.cu)
+  const bool small = !tuned && epi == 0 && in->prec == GBDW_F32 && small_blocks(p) <= num_sms();
   // form 4: the t-sweep for FP32, the 2x2x2x2 blocks for FP16
   int sweep = L.mode == 4 && in->prec == GBDW_F32 ? sweep_extent(g, in, epi, L.spt) : 0;
   if (p.mob && (sweep == 12 || (epi == 6 && g->lat->parity >= 0))) sweep = 0;
@@ -181,12 +188,18 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
     L.mode = 3;
     L.brick = 1;  // a sweep's brick is its slices of t
   }
+  if (!slices_ok(in, epi, L.spt, L.mode)) L.spt = 1;
+  int NS = 0, tthreads = 0;
+  size_t smem = 0;
+  const bool staged = L.mode == 1 || L.mode == 2;
+  if (staged && !tma_shape(in->prec, in->LsE, L, &NS, &tthreads, &smem)) L.mode = 0;
+  // fall back before fixing the CTA size: the block count below must match the launch
   if (L.mode == 3 && !form3_ok(in, epi, L.spt)) L.mode = 0;
   if (L.mode == 3) L.threads = 64;
   if (L.mode == 4) L.threads = 128;
   p.TE = tile_extent(in->LsE, L, p.mob != 0);
   p.brick = brick_extent(g->lat, L);
-  const int64_t nthreads = p.nsite * (p.LsE / L.spt);
+  const int64_t nthreads = p.nsite * ((p.LsE + L.spt - 1) / L.spt);
   int64_t blocks = staged ? (p.nsite + NS - 1) / NS : (nthreads + L.threads - 1) / L.threads;
   SweepParams sw;
   if (sweep) {
@@ -236,6 +249,7 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
     return GBDW_OK;
   }
   if (in->prec == GBDW_F64) st = launch_dhop_f64(p, dag, epi, L);
+  else if (small) st = launch_dhop_small(p, dag);
   else if (sweep)
     st = (sweep == 16 ? launch_dhop_sweep16 : sweep == 12 ? launch_dhop_sweep12 : launch_dhop_sweep8)(p, sw, unsigned(blocks), dag, epi);
   else if (in->prec == GBDW_F32) st = launch_dhop_f32(p, dag, epi, L);

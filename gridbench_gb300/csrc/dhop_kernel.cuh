@@ -568,9 +568,11 @@ __device__ __forceinline__ void dwf_epilogue(const DhopParams& p, int64_t site, 
     for (int j = 0; j < N; ++j) cen[j][k] = x[j];
   }
   const int slo = (s0 == 0) ? Ls - 1 : s0 - 1;
-  const int shi = (s0 + N == Ls) ? 0 : s0 + N;
+  const int shi = (s0 + N >= Ls) ? 0 : s0 + N;
   const T flo = (s0 == 0) ? T(-p.mf) : T(1);
-  const T fhi = (s0 + N == Ls) ? T(-p.mf) : T(1);
+  const T fhi = (s0 + N >= Ls) ? T(-p.mf) : T(1);
+  // an odd Ls in pairs: the last pair's second slot is padding, kept zero
+  const bool half = PIN == GBDW_F32 && N == 2 && !SMEM && s0 + N > Ls;
   constexpr int LO0 = DAG ? 2 : 0;  // first spin fed by psi(s-1)
   constexpr int HI0 = DAG ? 0 : 2;  // first spin fed by psi(s+1)
   cpx<T> lo[6], hi[6];
@@ -606,10 +608,14 @@ __device__ __forceinline__ void dwf_epilogue(const DhopParams& p, int64_t site, 
       const cpx<T> m = (j == 0) ? cpx<T>{lo[k].r * nlo, lo[k].i * nlo} : cen[j - 1 < 0 ? 0 : j - 1][LO0 * 3 + k];
       acc[j][LO0 * 3 + k].r -= c5 * m.r;
       acc[j][LO0 * 3 + k].i -= c5 * m.i;
-      const cpx<T> q = (j == N - 1) ? cpx<T>{hi[k].r * nhi, hi[k].i * nhi} : cen[j + 1 >= N ? N - 1 : j + 1][HI0 * 3 + k];
+      const cpx<T> q = (j == N - 1 || half) ? cpx<T>{hi[k].r * nhi, hi[k].i * nhi} : cen[j + 1 >= N ? N - 1 : j + 1][HI0 * 3 + k];
       acc[j][HI0 * 3 + k].r -= c5 * q.r;
       acc[j][HI0 * 3 + k].i -= c5 * q.i;
     }
+  }
+  if (half) {
+#pragma unroll
+    for (int k = 0; k < 12; ++k) acc[N - 1][k] = {T(0), T(0)};
   }
 }
 
@@ -620,19 +626,18 @@ __device__ __forceinline__ void dwf_epilogue(const DhopParams& p, int64_t site, 
 // consecutive lanes (pairs in order), so P- v(s0-1) is the second slice of the lane below and
 // P+ v(s0+2) the first slice of the lane above, both taken with shuffles inside the site's
 // group of lanes (which wraps around the 5th dimension).  Every site's lanes are active or
-// inactive together.
+// inactive together, and in one warp: any form for a power of two, the warp rings for other Ls.
 template <class T>
 __device__ __forceinline__ void mobius_adj_hop(const DhopParams& p, int s0, cpx<T> (&v)[2][12]) {
-  const int G = p.Ls >> 1;  // lanes per site: a power of two <= 32
+  const int G = p.Ls >> 1, lg = s0 >> 1;  // lanes per site, this one's place among them
   const unsigned mask = __activemask();
-  const int lg = int(threadIdx.x) & (G - 1);
-  const int from_lo = (lg + G - 1) & (G - 1);
-  const int from_hi = (lg + 1) & (G - 1);
+  const int base = int(threadIdx.x & 31) - lg;
+  const int from_lo = base + (lg == 0 ? G - 1 : lg - 1), from_hi = base + (lg == G - 1 ? 0 : lg + 1);
   cpx<T> vm[6], vp[6];
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
-    vm[k] = {__shfl_sync(mask, v[1][6 + k].r, from_lo, G), __shfl_sync(mask, v[1][6 + k].i, from_lo, G)};
-    vp[k] = {__shfl_sync(mask, v[0][k].r, from_hi, G), __shfl_sync(mask, v[0][k].i, from_hi, G)};
+    vm[k] = {__shfl_sync(mask, v[1][6 + k].r, from_lo), __shfl_sync(mask, v[1][6 + k].i, from_lo)};
+    vp[k] = {__shfl_sync(mask, v[0][k].r, from_hi), __shfl_sync(mask, v[0][k].i, from_hi)};
   }
   const T b = T(p.mb), c = T(p.mc);
   const T clo = s0 == 0 ? T(-p.mf) * c : c;           // slice s0: its s-1 wraps at the wall
@@ -772,7 +777,8 @@ __global__ void __launch_bounds__(MINB > 0 ? MAXT : 256, MINB > 0 ? MINB : 1) k_
     p.LsE = LSPC;
     p.LsP = LSPC;
   }
-  const unsigned G = unsigned(p.LsE) / N;
+  // FP32 rows of an odd extent are walked in pairs too (N = 2), the last one half padding
+  const unsigned G = (unsigned(p.LsE) + N - 1) / N;
   const unsigned bid = sweep_block(DAG);
   const unsigned tid = bid * blockDim.x + threadIdx.x;
   const bool active = tid < unsigned(p.nsite) * G;
@@ -879,6 +885,9 @@ int launch_dhop_bf16(const DhopParams& p, int dag, int epi, DhopLaunch L);
 int launch_dhop_sweep8(const DhopParams& p, const SweepParams& q, unsigned blocks, int dag, int epi);
 int launch_dhop_sweep12(const DhopParams& p, const SweepParams& q, unsigned blocks, int dag, int epi);
 int launch_dhop_sweep16(const DhopParams& p, const SweepParams& q, unsigned blocks, int dag, int epi);
+// the hopping term with its legs over four warps, for small lattices (dhop_small.cu): FP32 slice pairs
+int launch_dhop_small(const DhopParams& p, int dag);
+int64_t small_blocks(const DhopParams& p);
 int launch_dhop_general(const DhopParams& p, int prec, int dag);
 // The double-single form of the FP64 operator (dhop_ds.cu): direct loads, one slice per thread in
 // CTAs of DS_THREADS with registers capped for minb (3 or 4) CTAs per SM, Dhop and M; p.U must be

@@ -8,7 +8,7 @@ namespace gbdw {
 
 template <int PIN, int POUT, int GP, int DAG, int N, int EPI>
 int go_direct(const DhopParams& p, DhopLaunch L) {
-  const int64_t nthreads = p.nsite * (p.LsE / N);
+  const int64_t nthreads = p.nsite * ((p.LsE + N - 1) / N);
   const unsigned blocks = unsigned((nthreads + L.threads - 1) / L.threads);
   if constexpr (PIN == GBDW_F32 && N == 2) {
     // compile-time row strides for the extents of the benchmarked shapes: Ls = 16, and Ls = 12
@@ -95,12 +95,15 @@ int by_shape(const DhopParams& p, DhopLaunch L) {
         return GBDW_OK;
       }
     }
-    // FP32 Dhop / M at Ls*nrhs = 12 (one rhs at Ls = 12) and 144 (12 rhs at Ls = 12)
-    if constexpr (PIN == GBDW_F32 && EPI <= 1) {
-      if (L.spt == 2 && p.LsE == p.LsP && (p.LsE == 12 || p.LsE == 144)) {
-        const unsigned blocks = unsigned((p.nsite * (p.LsE / 2) + 63) / 64);
-        if (p.LsE == 12) k_dhop<PIN, POUT, GP, DAG, 2, EPI, 6, 12, 64><<<blocks, 64, 0, stream()>>>(p);
-        else k_dhop<PIN, POUT, GP, DAG, 2, EPI, 6, 144, 64><<<blocks, 64, 0, stream()>>>(p);
+    // other FP32 extents: Ls*nrhs = 12 (one rhs at Ls = 12) and 144 (12 rhs at Ls = 12) at compile time
+    // for Dhop and M, the rest with runtime strides
+    if constexpr (PIN == GBDW_F32) {
+      if (L.spt == 2) {
+        const unsigned blocks = unsigned((p.nsite * ((p.LsE + 1) / 2) + 63) / 64);
+        constexpr bool fixed = EPI <= 1;
+        if (fixed && p.LsE == 12) k_dhop<PIN, POUT, GP, DAG, 2, EPI, 6, fixed ? 12 : 0, 64><<<blocks, 64, 0, stream()>>>(p);
+        else if (fixed && p.LsE == 144) k_dhop<PIN, POUT, GP, DAG, 2, EPI, 6, fixed ? 144 : 0, 64><<<blocks, 64, 0, stream()>>>(p);
+        else k_dhop<PIN, POUT, GP, DAG, 2, EPI, 6, 0, 64><<<blocks, 64, 0, stream()>>>(p);
         GBDW_LAUNCHED();
         return GBDW_OK;
       }

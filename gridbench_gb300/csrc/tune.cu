@@ -29,20 +29,36 @@ std::string key_of(int gprec, int sprec, int LsE, int epi) {
 }
 }  // namespace
 
-DhopLaunch default_launch(int gprec, int sprec, int LsE, int epi) {
-  (void)gprec;
-  (void)epi;
-  DhopLaunch L{128, 1};
-  if (sprec == GBDW_F32) L.spt = (LsE % 2 == 0) ? 2 : 1;
-  else if (sprec == GBDW_F16) L.spt = (LsE % 4 == 0) ? 4 : (LsE % 2 == 0) ? 2 : 1;
-  return L;
-}
-
-DhopLaunch tuned_launch(int gprec, int sprec, int LsE, int epi) {
-  std::lock_guard<std::mutex> lk(g_tune_mu);
-  auto it = g_tuned.find(key_of(gprec, sprec, LsE, epi));
-  if (it != g_tuned.end()) return it->second;
-  return default_launch(gprec, sprec, LsE, epi);
+// Which form runs a shape nobody tuned.  Measured on lattices from 4^4 to 32^4 (us, hopping term / M):
+//   FP32, t-sweep against form 3:  16^4 x 8 37/40 - 49/53, 12^4 x 8 17/19 - 18/20, 10^4 x 8 12/13 - 10/12,
+//     16^4 x 12 58/65 - 64/74, 12^4 x 12 26/28 - 25/29, 24^4 x 16 268/293 - 318/332, 20^4 x 16 134/147 -
+//     135/146: rows of 8 or 12 slices from 400 thousand 5D sites, of 16 from 4 million (their two-thirds
+//     larger planes leave fewer CTAs to even out the last wave)
+//   FP32, the warp rings against form 3:  24^4 x 20 423/461 - 480/537, 16^3 x 32 x 10 114/123 - 115/132:
+//     from a million 5D sites where whole sites fill 30 lanes, and not at 16 (59/66 - 60/64) or 8
+//     (52/58 - 49/53)
+//   FP32, form 3 against form 0:  16^4 x 16 60/64 - 72/68, 16^4 x 10 62/70 - 67/73, 24^4 x 8 215/234 -
+//     223/244, 15x9x21x14 x 7 31/35 - 33/37: always
+//   FP16, form 3 against form 0:  16^4 x 16 51 - 61
+//   FP64: the pipe's time is the CTAs of the fullest SM; CTAs of one warp even small lattices out
+//     (8^4 x 8: 64.6 us with CTAs of 128 threads, the pipe alone 47)
+DhopLaunch untuned_launch(const gbdw_gauge* g, const gbdw_field* in, int epi) {
+  const int64_t sites5 = in->lat->nsite * in->LsE;
+  const int LsE = in->LsE;
+  if (in->prec == GBDW_F64) return DhopLaunch{sites5 / 128 < 8 * num_sms() ? 32 : 128, 1};
+  if (in->prec == GBDW_F16) {
+    if (form3_ok(in, epi, 2)) return DhopLaunch{64, 2, 3};
+    return DhopLaunch{128, LsE % 4 == 0 ? 4 : LsE % 2 == 0 ? 2 : 1};
+  }
+  if (const int te = sweep_extent(g, in, epi, 2))
+    if (sites5 >= (te == 16 ? 4000000 : 400000)) return DhopLaunch{64, 2, 4, 4, 1, 4};
+  DhopLaunch rings{64, 2, 2, 2};
+  int ns, threads;
+  size_t smem;
+  if (sites5 >= 1000000 && LsE % 2 == 0 && LsE >= 10 && LsE != 16 && 32 / (LsE / 2) * (LsE / 2) >= 30 &&
+      tma_shape(in->prec, LsE, rings, &ns, &threads, &smem))
+    return rings;
+  return DhopLaunch{64, 2, 3};
 }
 
 bool find_tuned_launch(int gprec, int sprec, int LsE, int epi, DhopLaunch* L) {
@@ -69,7 +85,8 @@ std::vector<int> cg_residual_precs(int gprec, int sprec) {
 // the shape run_dhop takes for epilogue key epi with this gauge field (half lattices: their own
 // entry if one exists)
 DhopLaunch lookup(const gbdw_gauge* g, const gbdw_field* in, int epi) {
-  DhopLaunch L = tuned_launch(g->prec, in->prec, in->LsE, epi);
+  DhopLaunch L;
+  if (!find_tuned_launch(g->prec, in->prec, in->LsE, epi, &L)) L = untuned_launch(g, in, epi);
   if (g->lat->parity >= 0) find_tuned_launch(g->prec, in->prec, in->LsE, epi + EO_KEY, &L);
   return L;
 }
@@ -111,7 +128,7 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
   const int s1 = in->prec == GBDW_F16 ? 2 : 1, s2 = in->prec == GBDW_F16 ? 4 : 2;
   for (int th : threads_c) {
     for (int spt : {1, 2, 4}) {
-      if (in->LsE % spt != 0 || (in->prec == GBDW_F64 && spt > 2)) continue;
+      if (!slices_ok(in, 0, spt, 0) || (in->prec == GBDW_F64 && spt > 2)) continue;
       // Ls / RHS tiles of the direct form where they cut whole groups: with many right-hand sides
       // a site's slices are many KB and the reuse distance of its spinor (one 3D volume of sites
       // along t) can exceed L2; a tile sweep over all sites shortens it by the split factor
@@ -169,7 +186,7 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
       return st;
     }
   }
-  DhopLaunch saved = tuned_launch(g->prec, in->prec, in->LsE, 0);
+  DhopLaunch saved = lookup(g, in, 0);
   if (eo) find_tuned_launch(g->prec, in->prec, in->LsE, ko, &saved);
   DhopLaunch best = saved, best_m = saved;
   float best_ms = 1e30f, best_m_ms = 1e30f;
@@ -195,7 +212,7 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
   };
   // M (one right-hand side) is timed over the same shapes on its own: its epilogue reads the
   // centre site and its 5th-dimension neighbours besides the hopping term's gather.
-  DhopLaunch saved_m = tuned_launch(g->prec, in->prec, in->LsE, 1);
+  DhopLaunch saved_m = lookup(g, in, 1);
   if (eo) find_tuned_launch(g->prec, in->prec, in->LsE, 1 + ko, &saved_m);
   std::vector<std::pair<float, DhopLaunch>> m_times;
   for (const DhopLaunch& L : cands) {
@@ -356,7 +373,7 @@ int gbdw_tune_set_ds(const gbdw_gauge* g, const gbdw_field* in, int epi, int min
 
 int gbdw_tune_set(const gbdw_gauge* g, const gbdw_field* in, int threads, int spt, int form, int stages) {
   if (!g || !in || threads < 32 || threads > 256 || threads % 32 != 0 || !(spt == 1 || spt == 2 || spt == 4) ||
-      in->LsE % spt != 0 || (in->prec == GBDW_F64 && spt > 2) || form < 0 || form > 4 ||
+      !slices_ok(in, 0, spt, form) || (in->prec == GBDW_F64 && spt > 2) || form < 0 || form > 4 ||
       (stages != 2 && stages != 4)) {
     set_error("gbdw_tune_set: threads 32..256 in steps of 32, spt 1/2/4 dividing Ls*nrhs (<= 2 for F64), "
               "form 0..4, stages 2/4");
@@ -364,8 +381,7 @@ int gbdw_tune_set(const gbdw_gauge* g, const gbdw_field* in, int threads, int sp
   }
   const DhopLaunch L{threads, spt, form, stages};
   if (form == 3 && !form3_ok(in, 0, spt)) {
-    set_error("gbdw_tune_set: form 3 is the kernel with 2 slices per thread for Ls*nrhs = 16 (FP32/FP16) or "
-              "12 / 144 (FP32)");
+    set_error("gbdw_tune_set: form 3 is the kernel with 2 slices per thread for FP32, or FP16 with Ls*nrhs = 16");
     return GBDW_ERR_INVALID;
   }
   if (form == 4 && !(in->prec == GBDW_F32 ? sweep_extent(g, in, 0, spt) > 0 : spt == 2 && blocked_ok(g->lat, in))) {

@@ -3,9 +3,8 @@
 #include "dhop_kernel.cuh"
 
 namespace gbdw {
-// Tuned entry if present, otherwise the built-in default for this precision and extent.
-DhopLaunch tuned_launch(int gprec, int sprec, int LsE, int epi);
-DhopLaunch default_launch(int gprec, int sprec, int LsE, int epi);
+// The shape for these operands when no entry exists (the rules' reasons are with the code).
+DhopLaunch untuned_launch(const gbdw_gauge* g, const gbdw_field* in, int epi);
 void set_tuned_launch(int gprec, int sprec, int LsE, int epi, DhopLaunch L);
 // Optional parts of a hopping launch used by the fused CG step.
 struct DhopExtra {
@@ -41,8 +40,11 @@ int mdagm_residual(const gbdw_gauge* g, gbdw_field* t, gbdw_field* r, const gbdw
                    const CgRule& rule);
 int check_operands(const gbdw_gauge* g, const gbdw_field* out, const gbdw_field* in, bool need_single_rhs);
 DhopParams make_params(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in);
-// form 3 (specialised direct) applies: slice pairs, Ls*nrhs = 16 (FP32/FP16) or 12 / 144 (FP32
-// Dhop and M)
+// spt slices per thread cut a row: whole groups, or pairs of an odd FP32 extent whose last one is half
+// padding (direct forms, Dhop and M)
+bool slices_ok(const gbdw_field* in, int epi, int spt, int form);
+// form 3 (direct, registers capped for six or eight CTAs per SM) applies: slice pairs, FP32 or FP16
+// with Ls*nrhs = 16
 bool form3_ok(const gbdw_field* in, int epi, int spt);
 // form 4 for FP16 (blocked site order) applies: Ls*nrhs = 16, periodic lattice, even extents
 bool blocked_ok(const gbdw_lattice* lat, const gbdw_field* in);
