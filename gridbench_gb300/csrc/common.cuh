@@ -33,6 +33,24 @@ int num_sms();
 int library_device();
 // cudaMalloc through the library's one allocation point (honours gbdw_debug_fail_allocs).
 cudaError_t dev_alloc(void** p, size_t bytes);
+// The memory of lattices, links and fields.  While an ArenaScope lives on this thread it comes from a
+// buffer of the current stream's scratch (kept, at most kArenaMax bytes; cudaMalloc serves what does not
+// fit) and object_free leaves it alone: for objects that live inside one call.
+cudaError_t object_alloc(void** p, size_t bytes);
+void object_free(void* p);
+constexpr size_t kArenaMax = size_t(256) << 20;
+struct ArenaScope {
+  explicit ArenaScope(size_t bytes);
+  ~ArenaScope();
+  bool held;
+};
+// While alive on this thread, imports let the kernels read host memory in place where the GPU can (for
+// a call that waits for the stream before it returns).
+struct HostInPlace {
+  HostInPlace();
+  ~HostInPlace();
+};
+bool host_in_place(const void* p);  // p is 16-byte aligned and such a scope is open
 unsigned* device_error_word();  // set by kernels whose bounded waits expired
 size_t max_dynamic_smem();      // opt-in dynamic shared memory per CTA, minus room for static
 

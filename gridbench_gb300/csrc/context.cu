@@ -25,6 +25,14 @@ int g_num_sms = 0;
 std::atomic<long> g_alloc_skip{0};
 std::atomic<long> g_alloc_fail{0};
 
+struct Arena {
+  char* base = nullptr;
+  size_t size = 0, used = 0;
+};
+thread_local Arena g_arena;
+std::atomic<bool> g_arena_taken{false};  // by one call at a time: a second thread's call allocates
+thread_local bool g_in_place = false;
+
 struct ScratchSlot {
   void* p = nullptr;
   size_t bytes = 0;
@@ -91,6 +99,44 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
   }
   return cudaMalloc(p, bytes);
 }
+
+cudaError_t object_alloc(void** p, size_t bytes) {
+  const size_t take = (bytes + 255) & ~size_t(255);
+  if (!g_arena.base || g_arena.used + take > g_arena.size) return dev_alloc(p, bytes);
+  *p = g_arena.base + g_arena.used;
+  g_arena.used += take;
+  return cudaSuccess;
+}
+
+void object_free(void* p) {
+  if (g_arena.base && (char*)p >= g_arena.base && (char*)p < g_arena.base + g_arena.size) return;
+  cudaFree(p);
+}
+
+ArenaScope::ArenaScope(size_t bytes) {
+  held = bytes <= kArenaMax && !g_arena_taken.exchange(true);
+  if (!held) return;
+  if (char* b = (char*)scratch(bytes, 10)) g_arena = Arena{b, bytes, 0};
+}
+ArenaScope::~ArenaScope() {
+  if (!held) return;
+  g_arena = Arena{};
+  g_arena_taken = false;
+}
+
+HostInPlace::HostInPlace() {
+  static const bool can = [] {
+    int dev = 0, access = 0, tables = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, dev);
+    cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev);
+    cudaGetLastError();
+    return access && tables;
+  }();
+  g_in_place = can;
+}
+HostInPlace::~HostInPlace() { g_in_place = false; }
+bool host_in_place(const void* p) { return g_in_place && (uintptr_t(p) & 15) == 0; }
 
 size_t max_dynamic_smem() {
   static size_t v = 0;

@@ -43,12 +43,12 @@ int ds_links(const gbdw_gauge* g, const void** out) {
   if (!g->d_ds) {
     const int64_t n = g->lat->nsite * 8 * 9;
     void* d = nullptr;
-    cudaError_t e = dev_alloc(&d, size_t(n) * sizeof(float4));
+    cudaError_t e = object_alloc(&d, size_t(n) * sizeof(float4));
     if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(double-single links)");
     const int t = 256;
     k_split_links<<<unsigned((n + t - 1) / t), t, 0, stream()>>>((const double2*)g->d, (float4*)d, n);
     if ((e = cudaGetLastError()) != cudaSuccess) {
-      cudaFree(d);
+      object_free(d);
       return cuda_fail(e, "k_split_links");
     }
     count_launch();

@@ -32,7 +32,7 @@ bool is_pinned_host(const void* p) {
 // Makes `bytes` of src available on the device: returns src itself for device memory,
 // otherwise a copy in scratch slot `slot` (a staging buffer of the current stream).
 int stage_in(const void* src, size_t bytes, int slot, const void** dev) {
-  if (is_device_ptr(src)) {
+  if (is_device_ptr(src) || host_in_place(src)) {
     *dev = src;
     return GBDW_OK;
   }
@@ -137,6 +137,20 @@ __global__ void k_gauge_import(const SRC* src, int64_t nsite, int nsimd, void* d
       ((__nv_bfloat162*)dst)[i * 6 + k] = __floats2bfloat162_rn(float(re), float(im));
     }
   }
+}
+
+// The same for one lane, where both sides keep the order of the entries: one thread per entry.
+template <class SRC, int P>
+__global__ void k_gauge_flat(const SRC* __restrict__ src, int64_t n, void* dst) {
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;  // stored entry
+  if (i >= n) return;
+  constexpr int per = (P == GBDW_F16 || P == GBDW_BF16) ? 6 : 9;
+  using V = typename std::conditional<sizeof(SRC) == 8, double2, float2>::type;
+  const V v = __ldg(reinterpret_cast<const V*>(src) + (per == 9 ? i : i / per * 9 + i % per));
+  if (P == GBDW_F64) ((double2*)dst)[i] = make_double2(v.x, v.y);
+  else if (P == GBDW_F32) ((float2*)dst)[i] = make_float2(float(v.x), float(v.y));
+  else if (P == GBDW_F16) ((__half2*)dst)[i] = __floats2half2_rn(float(v.x), float(v.y));
+  else ((__nv_bfloat162*)dst)[i] = __floats2bfloat162_rn(float(v.x), float(v.y));
 }
 
 // Reference spinor (complex SRC, nsimd lanes, Ls slices) -> right-hand side `rhs` of a field.
@@ -420,12 +434,12 @@ int lattice_from_table_impl(gbdw_lattice** out, uint64_t nouter, int Ls, int nsi
     return GBDW_ERR_ALLOC;
   }
   auto fail = [&](int st) {
-    if (L->nbr4) cudaFree(L->nbr4);
-    if (L->nbr5) cudaFree(L->nbr5);
+    if (L->nbr4) object_free(L->nbr4);
+    if (L->nbr5) object_free(L->nbr5);
     delete L;
     return st;
   };
-  cudaError_t e = dev_alloc((void**)&L->nbr4, size_t(L->nsite) * 8 * sizeof(uint32_t));
+  cudaError_t e = object_alloc((void**)&L->nbr4, size_t(L->nsite) * 8 * sizeof(uint32_t));
   if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc(nbr4)"));
   if ((e = cudaMemsetAsync(dflags, 0, sizeof(unsigned), stream())) != cudaSuccess) return fail(cuda_fail(e, "memset"));
   k_table_check<<<nblk(nent, 256), 256, 0, stream()>>>((const uint64_t*)dnbr, (const uint8_t*)dprm, int64_t(nouter), Ls,
@@ -442,7 +456,7 @@ int lattice_from_table_impl(gbdw_lattice** out, uint64_t nouter, int Ls, int nsi
   }
   L->fast = !(flags & 2u) && !force_general;
   if (!L->fast) {
-    e = dev_alloc((void**)&L->nbr5, size_t(L->nsite) * Ls * 8 * sizeof(uint32_t));
+    e = object_alloc((void**)&L->nbr5, size_t(L->nsite) * Ls * 8 * sizeof(uint32_t));
     if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc(nbr5)"));
     k_table_general<<<nblk(nent, 256), 256, 0, stream()>>>((const uint64_t*)dnbr, (const uint8_t*)dprm, int64_t(nouter),
                                                             Ls, nsimd, L->nbr5);
@@ -490,14 +504,14 @@ int gbdw_lattice_create(gbdw_lattice** lat, const int dims[4], int Ls) {
   L->fast = true;
   L->nbr5 = nullptr;
   for (int d = 0; d < 4; ++d) L->dims[d] = dims[d];
-  cudaError_t e = dev_alloc((void**)&L->nbr4, size_t(V) * 8 * sizeof(uint32_t));
+  cudaError_t e = object_alloc((void**)&L->nbr4, size_t(V) * 8 * sizeof(uint32_t));
   if (e != cudaSuccess) {
     delete L;
     return cuda_fail(e, "cudaMalloc(nbr4)");
   }
   k_table_periodic<<<nblk(V, 256), 256, 0, stream()>>>(make_int4(dims[0], dims[1], dims[2], dims[3]), L->nbr4);
   if ((e = cudaGetLastError()) != cudaSuccess) {
-    cudaFree(L->nbr4);
+    object_free(L->nbr4);
     delete L;
     return cuda_fail(e, "k_table_periodic");
   }
@@ -509,9 +523,9 @@ int gbdw_lattice_create(gbdw_lattice** lat, const int dims[4], int Ls) {
 int gbdw_lattice_destroy(gbdw_lattice* lat) {
   if (!lat) return GBDW_OK;
   cudaStreamSynchronize(stream());
-  if (lat->nbr4) cudaFree(lat->nbr4);
-  if (lat->nbr5) cudaFree(lat->nbr5);
-  if (lat->cbsite) cudaFree(lat->cbsite);
+  if (lat->nbr4) object_free(lat->nbr4);
+  if (lat->nbr5) object_free(lat->nbr5);
+  if (lat->cbsite) object_free(lat->cbsite);
   delete lat;
   return GBDW_OK;
 }
@@ -539,7 +553,7 @@ int gbdw_gauge_create(gbdw_gauge** g, const gbdw_lattice* lat, int prec, const v
   G->lat = lat;
   G->prec = prec;
   G->bytes = size_t(nlink) * link_bytes(prec);
-  cudaError_t e = dev_alloc((void**)&G->d, G->bytes);
+  cudaError_t e = object_alloc((void**)&G->d, G->bytes);
   if (e != cudaSuccess) {
     delete G;
     return cuda_fail(e, "cudaMalloc(gauge)");
@@ -547,7 +561,11 @@ int gbdw_gauge_create(gbdw_gauge** g, const gbdw_lattice* lat, int prec, const v
   const int t = 256;
   const int64_t nsite = lat->nsite;
   const int ns = lat->nsimd;
-#define GBDW_GI(SRC, P) k_gauge_import<SRC, P><<<nblk(nlink, t), t, 0, stream()>>>((const SRC*)dsrc, nsite, ns, G->d)
+  const bool flat = ns == 1 && (uintptr_t(dsrc) & 15) == 0;
+  const int64_t entries = nlink * (prec == GBDW_F16 || prec == GBDW_BF16 ? 6 : 9);
+#define GBDW_GI(SRC, P)                                                                            \
+  if (flat) k_gauge_flat<SRC, P><<<nblk(entries, t), t, 0, stream()>>>((const SRC*)dsrc, entries, G->d); \
+  else k_gauge_import<SRC, P><<<nblk(nlink, t), t, 0, stream()>>>((const SRC*)dsrc, nsite, ns, G->d)
   if (src_prec == GBDW_F64) {
     switch (prec) {
       case GBDW_F64: GBDW_GI(double, GBDW_F64); break;
@@ -565,7 +583,7 @@ int gbdw_gauge_create(gbdw_gauge** g, const gbdw_lattice* lat, int prec, const v
   }
 #undef GBDW_GI
   if ((e = cudaGetLastError()) != cudaSuccess) {
-    cudaFree(G->d);
+    object_free(G->d);
     delete G;
     return cuda_fail(e, "k_gauge_import");
   }
@@ -577,8 +595,8 @@ int gbdw_gauge_create(gbdw_gauge** g, const gbdw_lattice* lat, int prec, const v
 int gbdw_gauge_destroy(gbdw_gauge* g) {
   if (!g) return GBDW_OK;
   cudaStreamSynchronize(stream());
-  cudaFree(g->d);
-  if (g->d_ds) cudaFree(g->d_ds);
+  object_free(g->d);
+  if (g->d_ds) object_free(g->d_ds);
   delete g;
   return GBDW_OK;
 }
@@ -601,15 +619,15 @@ int gbdw_field_create(gbdw_field** f, const gbdw_lattice* lat, int prec, int nrh
   F->LsP = padded_slices(prec, F->LsE);
   F->norm = nullptr;
   F->bytes = size_t(F->elems()) * spinor_elem_bytes(prec);
-  cudaError_t e = dev_alloc((void**)&F->d, F->bytes);
+  cudaError_t e = object_alloc((void**)&F->d, F->bytes);
   if (e != cudaSuccess) {
     delete F;
     return cuda_fail(e, "cudaMalloc(field)");
   }
   if (prec == GBDW_F16) {
-    e = dev_alloc((void**)&F->norm, size_t(lat->nsite) * F->LsE * sizeof(float));
+    e = object_alloc((void**)&F->norm, size_t(lat->nsite) * F->LsE * sizeof(float));
     if (e != cudaSuccess) {
-      cudaFree(F->d);
+      object_free(F->d);
       delete F;
       return cuda_fail(e, "cudaMalloc(norm)");
     }
@@ -621,8 +639,8 @@ int gbdw_field_create(gbdw_field** f, const gbdw_lattice* lat, int prec, int nrh
 int gbdw_field_destroy(gbdw_field* f) {
   if (!f) return GBDW_OK;
   cudaStreamSynchronize(stream());
-  cudaFree(f->d);
-  if (f->norm) cudaFree(f->norm);
+  object_free(f->d);
+  if (f->norm) object_free(f->norm);
   delete f;
   return GBDW_OK;
 }
