@@ -10,6 +10,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "common.cuh"
@@ -19,12 +20,16 @@
 namespace gbdw {
 
 namespace {
-std::map<std::string, DhopLaunch> g_tuned;
+// (gauge precision, spinor precision, Ls*nrhs, epilogue key); looked up on every launch, so the text form
+// is made for the cache file only
+using TuneKey = std::tuple<int, int, int, int>;
+std::map<TuneKey, DhopLaunch> g_tuned;
 std::mutex g_tune_mu;
 
-std::string key_of(int gprec, int sprec, int LsE, int epi) {
+TuneKey key_of(int gprec, int sprec, int LsE, int epi) { return TuneKey{gprec, sprec, LsE, epi}; }
+std::string key_text(const TuneKey& k) {
   char buf[96];
-  snprintf(buf, sizeof buf, "g%d_s%d_L%d_e%d", gprec, sprec, LsE, epi);
+  snprintf(buf, sizeof buf, "g%d_s%d_L%d_e%d", std::get<0>(k), std::get<1>(k), std::get<2>(k), std::get<3>(k));
   return buf;
 }
 }  // namespace
@@ -450,7 +455,9 @@ int gbdw_tune_save(const char* path) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   fprintf(f, "{");
   bool first = true;
-  for (auto& kv : g_tuned) {
+  std::map<std::string, DhopLaunch> text;  // in the order of the keys' text
+  for (auto& kv : g_tuned) text[key_text(kv.first)] = kv.second;
+  for (auto& kv : text) {
     fprintf(f, "%s\n  \"%s\": [%d, %d, %d, %d, %d, %d]", first ? "" : ",", kv.first.c_str(), kv.second.threads,
             kv.second.spt, kv.second.mode, kv.second.stages, kv.second.split, kv.second.brick);
     first = false;
