@@ -267,6 +267,7 @@ __device__ __forceinline__ void ld_pair(const void* d, const float* nrm, int64_t
 
 template <int PX, int PP, int PR>
 __global__ void k_cg_xp_pairs(CgStep cg, FieldOut x, FieldOut p, FieldRef r, int64_t nsite, int LsE) {
+  dep_wait();
   const int G = LsE / 2;
   const int64_t n = nsite * G;
   if (!cg.go()) return;
@@ -369,6 +370,7 @@ __device__ __forceinline__ void flat_loop(int64_t n, LOAD load, F f, DONE done) 
 
 template <int P>
 __global__ void k_axpby_flat(typename Arith<P>::T a, const void* x_, typename Arith<P>::T b, void* y_, int64_t n) {
+  dep_wait();
   using V = typename Flat<P>::V;
   const V* x = (const V*)x_;
   V* y = (V*)y_;
@@ -379,6 +381,7 @@ __global__ void k_axpby_flat(typename Arith<P>::T a, const void* x_, typename Ar
 
 template <int P>
 __global__ void k_norm2_flat(const void* x_, int64_t n, Reduce red) {
+  dep_wait();
   using V = typename Flat<P>::V;
   const V* x = (const V*)x_;
   double acc[1] = {0.0};
@@ -389,11 +392,13 @@ __global__ void k_norm2_flat(const void* x_, int64_t n, Reduce red) {
               acc[0] += double(s);
               s = 0;
             });
+  dep_release();
   grid_sum<1>(acc, red.partials, red.counter, red.result);
 }
 
 template <int P>
 __global__ void k_dot_flat(const void* x_, const void* y_, int64_t n, Reduce red) {
+  dep_wait();
   using V = typename Flat<P>::V;
   const V *x = (const V*)x_, *y = (const V*)y_;
   double acc[2] = {0.0, 0.0};
@@ -406,12 +411,14 @@ __global__ void k_dot_flat(const void* x_, const void* y_, int64_t n, Reduce red
               acc[1] += double(im);
               re = im = 0;
             });
+  dep_release();
   grid_sum<2>(acc, red.partials, red.counter, red.result);
 }
 
 // r = b - t, |r|^2, all FP64
 __global__ void k_xmy_norm_flat(const double2* __restrict__ b, const double2* __restrict__ t, double2* __restrict__ r,
                                 int64_t n, Reduce red) {
+  dep_wait();
   double acc[1] = {0.0};
   double2 u[kVec], v[kVec];
   flat_loop(n, [&](int64_t i, int k) { u[k] = __ldg(b + i); v[k] = __ldg(t + i); },
@@ -421,6 +428,7 @@ __global__ void k_xmy_norm_flat(const double2* __restrict__ b, const double2* __
               norm_v(d, acc[0]);
             },
             [] {});
+  dep_release();
   grid_sum<1>(acc, red.partials, red.counter, red.result);
 }
 
@@ -428,6 +436,7 @@ __global__ void k_xmy_norm_flat(const double2* __restrict__ b, const double2* __
 // pair of a row, which is two FP64 vectors side by side and one FP32 vector
 __global__ void k_cg_xp_f64_pairs(CgStep cg, double2* __restrict__ x, double2* __restrict__ p,
                                   const double2* __restrict__ r, float4* __restrict__ q, int64_t npair) {
+  dep_wait();
   if (!cg.go()) return;
   const double alpha = cg.alpha, beta = cg.beta;
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < npair; i += int64_t(gridDim.x) * blockDim.x) {
@@ -470,8 +479,8 @@ int blas_norm2(const gbdw_field* x, double* out, bool fetch) {
     const int64_t n = vectors(x), g = grid_flat(n);
     Reduce red;
     if (int st = reduce_scratch(g, 1, &red)) return st;
-    if (x->prec == GBDW_F64) k_norm2_flat<GBDW_F64><<<unsigned(g), kThreads, 0, stream()>>>(x->d, n, red);
-    else k_norm2_flat<GBDW_F32><<<unsigned(g), kThreads, 0, stream()>>>(x->d, n, red);
+    if (x->prec == GBDW_F64) launch_after(k_norm2_flat<GBDW_F64>, unsigned(g), kThreads, 0, x->d, n, red);
+    else launch_after(k_norm2_flat<GBDW_F32>, unsigned(g), kThreads, 0, x->d, n, red);
     GBDW_LAUNCHED();
     return fetch ? reduce_fetch(red, 1, out) : GBDW_OK;
   }
@@ -498,7 +507,7 @@ int blas_xmy_norm(const gbdw_field* b, const gbdw_field* t, gbdw_field* r, doubl
     const int64_t n = vectors(r), g = grid_flat(n);
     Reduce red;
     if (int st = reduce_scratch(g, 1, &red)) return st;
-    k_xmy_norm_flat<<<unsigned(g), kThreads, 0, stream()>>>((const double2*)b->d, (const double2*)t->d, (double2*)r->d, n, red);
+    launch_after(k_xmy_norm_flat, unsigned(g), kThreads, 0, (const double2*)b->d, (const double2*)t->d, (double2*)r->d, n, red);
     GBDW_LAUNCHED();
     return reduce_fetch(red, 1, rr);
   }
@@ -567,11 +576,11 @@ int blas_cg_xp(double alpha, double beta, gbdw_field* x, gbdw_field* p, const gb
   if (!q && pairs_ok(x) && pairs_ok(p) && pairs_ok(r) && x->prec == GBDW_F32) {
     const unsigned g = unsigned(grid_pairs(r));
     if (p->prec == GBDW_F16 && r->prec == GBDW_F16)
-      k_cg_xp_pairs<GBDW_F32, GBDW_F16, GBDW_F16><<<g, kThreads, 0, stream()>>>(cg, out(x), out(p), ref(r), ns, L);
+      launch_after(k_cg_xp_pairs<GBDW_F32, GBDW_F16, GBDW_F16>, g, kThreads, 0, cg, out(x), out(p), ref(r), ns, L);
     else if (p->prec == GBDW_F16 && r->prec == GBDW_F32)
-      k_cg_xp_pairs<GBDW_F32, GBDW_F16, GBDW_F32><<<g, kThreads, 0, stream()>>>(cg, out(x), out(p), ref(r), ns, L);
+      launch_after(k_cg_xp_pairs<GBDW_F32, GBDW_F16, GBDW_F32>, g, kThreads, 0, cg, out(x), out(p), ref(r), ns, L);
     else if (p->prec == GBDW_F32 && r->prec == GBDW_F32)
-      k_cg_xp_pairs<GBDW_F32, GBDW_F32, GBDW_F32><<<g, kThreads, 0, stream()>>>(cg, out(x), out(p), ref(r), ns, L);
+      launch_after(k_cg_xp_pairs<GBDW_F32, GBDW_F32, GBDW_F32>, g, kThreads, 0, cg, out(x), out(p), ref(r), ns, L);
     else {
       set_error("blas_cg_xp: unsupported precision combination");
       return GBDW_ERR_INVALID;
@@ -582,7 +591,7 @@ int blas_cg_xp(double alpha, double beta, gbdw_field* x, gbdw_field* p, const gb
   if (x->prec == GBDW_F64 && p->prec == GBDW_F64 && r->prec == GBDW_F64 && L % 2 == 0 && x != p && x != r && p != r &&
       (!q || q->prec == GBDW_F32)) {
     const int64_t npair = ns * 12 * int64_t(L / 2);
-    k_cg_xp_f64_pairs<<<unsigned(grid_flat(npair)), kThreads, 0, stream()>>>(
+    launch_after(k_cg_xp_f64_pairs, unsigned(grid_flat(npair)), kThreads, 0,
         cg, (double2*)x->d, (double2*)p->d, (const double2*)r->d, q ? (float4*)q->d : nullptr, npair);
     GBDW_LAUNCHED();
     return GBDW_OK;
@@ -640,8 +649,8 @@ int blas_axpby(double a, const gbdw_field* x, double b, gbdw_field* y) {
   if (x->prec == y->prec && flat_ok(x)) {
     const int64_t n = vectors(y);
     const unsigned g = unsigned(grid_flat(n));
-    if (x->prec == GBDW_F64) k_axpby_flat<GBDW_F64><<<g, kThreads, 0, stream()>>>(a, x->d, b, y->d, n);
-    else k_axpby_flat<GBDW_F32><<<g, kThreads, 0, stream()>>>(float(a), x->d, float(b), y->d, n);
+    if (x->prec == GBDW_F64) launch_after(k_axpby_flat<GBDW_F64>, g, kThreads, 0, a, x->d, b, y->d, n);
+    else launch_after(k_axpby_flat<GBDW_F32>, g, kThreads, 0, float(a), x->d, float(b), y->d, n);
     GBDW_LAUNCHED();
     return GBDW_OK;
   }
@@ -674,8 +683,8 @@ int blas_dot(const gbdw_field* x, const gbdw_field* y, double* re, double* im) {
     const int64_t n = vectors(x), g = grid_flat(n);
     Reduce red;
     if (int st = reduce_scratch(g, 2, &red)) return st;
-    if (x->prec == GBDW_F64) k_dot_flat<GBDW_F64><<<unsigned(g), kThreads, 0, stream()>>>(x->d, y->d, n, red);
-    else k_dot_flat<GBDW_F32><<<unsigned(g), kThreads, 0, stream()>>>(x->d, y->d, n, red);
+    if (x->prec == GBDW_F64) launch_after(k_dot_flat<GBDW_F64>, unsigned(g), kThreads, 0, x->d, y->d, n, red);
+    else launch_after(k_dot_flat<GBDW_F32>, unsigned(g), kThreads, 0, x->d, y->d, n, red);
     GBDW_LAUNCHED();
     double v[2];
     if (int st = reduce_fetch(red, 2, v)) return st;

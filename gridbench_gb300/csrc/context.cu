@@ -208,6 +208,7 @@ constexpr int kSumShare = 4096;
 __global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict__ partials, int64_t n, double* sums,
                                                        unsigned* counter, double* result, double num,
                                                        double* alpha_out, CgRule rule, double* host) {
+  dep_wait();
   __shared__ double sh[32][1];
   __shared__ bool last;
   const int64_t first = n * blockIdx.x / gridDim.x, end = n * (blockIdx.x + 1) / gridDim.x;
@@ -218,6 +219,7 @@ __global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict_
     for (int j = 0; j < 4; ++j) x[j] = k + j * blockDim.x < end ? __ldcg(partials + k + j * blockDim.x) : 0.0;
     v[0] += (x[0] + x[1]) + (x[2] + x[3]);
   }
+  dep_release();
   block_sum_to_thread0<1>(v, sh);
   if (gridDim.x > 1) {
     if (threadIdx.x == 0) {
@@ -255,7 +257,7 @@ int sum_partials(const double* partials, int64_t n, double* result, double num, 
     return GBDW_ERR_ALLOC;
   }
   const int threads = n >= 4096 ? 1024 : 256;
-  k_sum_partials<<<unsigned(ctas), threads, 0, stream()>>>(partials, n, (double*)(s + 1024), (unsigned*)(s + 1536),
+  launch_after(k_sum_partials, unsigned(ctas), threads, 0, partials, n, (double*)(s + 1024), (unsigned*)(s + 1536),
                                                            result, num, alpha_out, rule ? *rule : CgRule{0.0, 0.0, 0.0},
                                                            g_pinned + 32);
   GBDW_LAUNCHED();

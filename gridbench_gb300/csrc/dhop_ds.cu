@@ -170,6 +170,7 @@ __device__ __forceinline__ void ds_leg(const float4* __restrict__ u, const doubl
 // than their share of the work).
 template <int DAG, int EPI, int MINB>
 __global__ void __launch_bounds__(DS_THREADS, MINB) k_dhop_ds(const DhopParams p) {
+  dep_wait();
   const unsigned tid = sweep_block(DAG) * DS_THREADS + threadIdx.x;
   const unsigned LsE = unsigned(p.LsE);
   float part = 0.f;
@@ -209,7 +210,7 @@ int launch_dhop_ds(const DhopParams& p, int dag, int epi, int minb) {
   }
   const int64_t nthreads = p.nsite * p.LsE;
   const unsigned blocks = unsigned((nthreads + DS_THREADS - 1) / DS_THREADS);
-#define GBDW_DSK(D, E, MB) k_dhop_ds<D, E, MB><<<blocks, DS_THREADS, 0, stream()>>>(p)
+#define GBDW_DSK(D, E, MB) launch_after(k_dhop_ds<D, E, MB>, blocks, DS_THREADS, 0, p)
   if (minb == 4) {
     if (dag) epi ? GBDW_DSK(1, 1, 4) : GBDW_DSK(1, 0, 4);
     else epi ? GBDW_DSK(0, 1, 4) : GBDW_DSK(0, 0, 4);

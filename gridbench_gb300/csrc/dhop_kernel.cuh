@@ -771,6 +771,7 @@ __device__ __forceinline__ unsigned brick_site(const DhopParams& p, unsigned j) 
 template <int PIN, int POUT, int GP, int DAG, int N, int EPI, int MINB = 0, int LSPC = 0, int MAXT = 128,
           int BLK = 0>
 __global__ void __launch_bounds__(MINB > 0 ? MAXT : 256, MINB > 0 ? MINB : 1) k_dhop(const DhopParams p_) {
+  dep_wait();
   using T = typename Arith<PIN>::T;
   DhopParams p = p_;
   if constexpr (LSPC > 0) {
@@ -818,6 +819,7 @@ __global__ void __launch_bounds__(MINB > 0 ? MAXT : 256, MINB > 0 ? MINB : 1) k_
     }
     cpx<T> acc[N][12];
     dhop_thread<PIN, GP, DAG, N, EPI == 6>(p, site, s0, acc);
+    if constexpr (EPI <= 1 || EPI == 6) dep_release();
     finish_site<PIN, POUT, DAG, N, EPI>(p, site, s0, p.LsE, p.LsP, acc, part, dpart);
   }
   if (p.partials) {

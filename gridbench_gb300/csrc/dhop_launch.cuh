@@ -14,14 +14,14 @@ int go_direct(const DhopParams& p, DhopLaunch L) {
     // compile-time row strides for the extents of the benchmarked shapes: Ls = 16, and Ls = 12
     // with one or 12 right-hand sides
     if (p.LsE == p.LsP && (p.LsE == 16 || p.LsE == 12 || p.LsE == 144)) {
-      if (p.LsE == 16) k_dhop<PIN, POUT, GP, DAG, N, EPI, 0, 16><<<blocks, L.threads, 0, stream()>>>(p);
-      else if (p.LsE == 12) k_dhop<PIN, POUT, GP, DAG, N, EPI, 0, 12><<<blocks, L.threads, 0, stream()>>>(p);
-      else k_dhop<PIN, POUT, GP, DAG, N, EPI, 0, 144><<<blocks, L.threads, 0, stream()>>>(p);
+      if (p.LsE == 16) launch_after(k_dhop<PIN, POUT, GP, DAG, N, EPI, 0, 16>, blocks, L.threads, 0, p);
+      else if (p.LsE == 12) launch_after(k_dhop<PIN, POUT, GP, DAG, N, EPI, 0, 12>, blocks, L.threads, 0, p);
+      else launch_after(k_dhop<PIN, POUT, GP, DAG, N, EPI, 0, 144>, blocks, L.threads, 0, p);
       GBDW_LAUNCHED();
       return GBDW_OK;
     }
   }
-  k_dhop<PIN, POUT, GP, DAG, N, EPI><<<blocks, L.threads, 0, stream()>>>(p);
+  launch_after(k_dhop<PIN, POUT, GP, DAG, N, EPI>, blocks, L.threads, 0, p);
   GBDW_LAUNCHED();
   return GBDW_OK;
 }
@@ -44,7 +44,7 @@ int go_tma(const DhopParams& p, DhopLaunch L) {
     opted_in = true;
   }
   const unsigned blocks = unsigned((p.nsite + NS - 1) / NS);
-  kern<<<blocks, threads, smem, stream()>>>(p, NS);
+  launch_after(kern, blocks, threads, smem, p, NS);
   GBDW_LAUNCHED();
   return GBDW_OK;
 }
@@ -69,7 +69,7 @@ int go_tmaw(const DhopParams& p, DhopLaunch L) {
     opted_in[opted_in[0] ? 1 : 0] = (const void*)kern;
   }
   const unsigned blocks = unsigned((p.nsite + NS - 1) / NS);
-  kern<<<blocks, threads, smem, stream()>>>(p);
+  launch_after(kern, blocks, threads, smem, p);
   GBDW_LAUNCHED();
   return GBDW_OK;
 }
@@ -90,7 +90,7 @@ int by_shape(const DhopParams& p, DhopLaunch L) {
         // fewer loads in flight per thread), so it keeps the cap of six
         constexpr int MB = PIN == GBDW_F16 ? 8 : 6;
         const unsigned blocks = unsigned((p.nsite * 8 + 63) / 64);
-        k_dhop<PIN, POUT, GP, DAG, 2, EPI, MB, 16, 64><<<blocks, 64, 0, stream()>>>(p);
+        launch_after(k_dhop<PIN, POUT, GP, DAG, 2, EPI, MB, 16, 64>, blocks, 64, 0, p);
         GBDW_LAUNCHED();
         return GBDW_OK;
       }
@@ -101,9 +101,9 @@ int by_shape(const DhopParams& p, DhopLaunch L) {
       if (L.spt == 2) {
         const unsigned blocks = unsigned((p.nsite * ((p.LsE + 1) / 2) + 63) / 64);
         constexpr bool fixed = EPI <= 1;
-        if (fixed && p.LsE == 12) k_dhop<PIN, POUT, GP, DAG, 2, EPI, 6, fixed ? 12 : 0, 64><<<blocks, 64, 0, stream()>>>(p);
-        else if (fixed && p.LsE == 144) k_dhop<PIN, POUT, GP, DAG, 2, EPI, 6, fixed ? 144 : 0, 64><<<blocks, 64, 0, stream()>>>(p);
-        else k_dhop<PIN, POUT, GP, DAG, 2, EPI, 6, 0, 64><<<blocks, 64, 0, stream()>>>(p);
+        if (fixed && p.LsE == 12) launch_after(k_dhop<PIN, POUT, GP, DAG, 2, EPI, 6, fixed ? 12 : 0, 64>, blocks, 64, 0, p);
+        else if (fixed && p.LsE == 144) launch_after(k_dhop<PIN, POUT, GP, DAG, 2, EPI, 6, fixed ? 144 : 0, 64>, blocks, 64, 0, p);
+        else launch_after(k_dhop<PIN, POUT, GP, DAG, 2, EPI, 6, 0, 64>, blocks, 64, 0, p);
         GBDW_LAUNCHED();
         return GBDW_OK;
       }
@@ -112,7 +112,7 @@ int by_shape(const DhopParams& p, DhopLaunch L) {
     // FP16 (FP32 runs the t-sweep there, dhop_sweep.cuh)
     if constexpr (PIN == GBDW_F16) {
       if (L.spt == 2 && p.LsE == 16 && p.LsP == 16 && p.nsite % 16 == 0) {
-        k_dhop<PIN, POUT, GP, DAG, 2, EPI, 3, 16, 128, 1><<<unsigned(p.nsite / 16), 128, 0, stream()>>>(p);
+        launch_after(k_dhop<PIN, POUT, GP, DAG, 2, EPI, 3, 16, 128, 1>, unsigned(p.nsite / 16), 128, 0, p);
         GBDW_LAUNCHED();
         return GBDW_OK;
       }

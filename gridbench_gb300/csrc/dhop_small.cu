@@ -33,6 +33,7 @@ __device__ __forceinline__ void small_direction(const DhopParams& p, unsigned si
 
 template <int DAG>
 __global__ void __launch_bounds__(4 * SMALL_ITEMS) k_dhop_small(const DhopParams p) {
+  dep_wait();
   __shared__ float4 parts[4][12][SMALL_ITEMS];
   const unsigned G = (unsigned(p.LsE) + 1) / 2;
   const unsigned item = sweep_block(DAG) * SMALL_ITEMS + (threadIdx.x & 31);
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(4 * SMALL_ITEMS) k_dhop_small(const DhopParams
     for (int k = 0; k < 12; ++k)
       parts[w][k][threadIdx.x & 31] = make_float4(acc[k].r.x, acc[k].r.y, acc[k].i.x, acc[k].i.y);
   }
+  dep_release();
   __syncthreads();
   if (!active) return;
 #pragma unroll
@@ -73,8 +75,8 @@ int64_t small_blocks(const DhopParams& p) { return (p.nsite * ((p.LsE + 1) / 2) 
 
 int launch_dhop_small(const DhopParams& p, int dag) {
   const unsigned blocks = unsigned(small_blocks(p));
-  if (dag) k_dhop_small<1><<<blocks, 4 * SMALL_ITEMS, 0, stream()>>>(p);
-  else k_dhop_small<0><<<blocks, 4 * SMALL_ITEMS, 0, stream()>>>(p);
+  if (dag) launch_after(k_dhop_small<1>, blocks, 4 * SMALL_ITEMS, 0, p);
+  else launch_after(k_dhop_small<0>, blocks, 4 * SMALL_ITEMS, 0, p);
   GBDW_LAUNCHED();
   return GBDW_OK;
 }

@@ -121,6 +121,7 @@ __device__ __forceinline__ void sweep_leg(const cpx<float> (&u)[3][3], RawSpinor
 template <int DAG, int EPI, int TE, int EO>
 __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) / 32 * 32))
     k_dhop_sweep(const DhopParams p, const SweepParams q) {
+  dep_wait();
   constexpr int NS = 8, G = TE / 2, SS = sweep_site_bytes(TE), ROW = TE * 8;
   extern __shared__ __align__(16) char sw_smem[];
   const int tid = threadIdx.x;
@@ -234,6 +235,7 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
       float pt = 0.f;
       double dt = 0.0;
       const int64_t site = int64_t(t) * vol3 + col;
+      if ((EPI <= 1 || EPI == 6) && !more) dep_release();
       if (!EO && EPI >= 1 && !p.cen)  // the diagonal part reads this site's plane t, in shared memory
         finish_site<GBDW_F32, GBDW_F32, DAG, 2, EPI, !EO && EPI >= 1>(p, site, e0, p.LsE, p.LsP, v, pt, dt, sc - lg * 16);
       else

@@ -12,7 +12,7 @@ int go_sweep(const DhopParams& p, const SweepParams& q, unsigned blocks) {
     GBDW_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sweep_smem(TE))));
     opted_in = true;
   }
-  kern<<<blocks, (4 * TE + 31) / 32 * 32, sweep_smem(TE), stream()>>>(p, q);
+  launch_after(kern, blocks, (4 * TE + 31) / 32 * 32, sweep_smem(TE), p, q);
   GBDW_LAUNCHED();
   return GBDW_OK;
 }

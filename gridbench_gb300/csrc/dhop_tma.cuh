@@ -73,6 +73,7 @@ struct ESz {
 // then STAGES+1 mbarriers (the last one for the links).
 template <int PIN, int POUT, int GP, int DAG, int N, int EPI, int STAGES>
 __global__ void __launch_bounds__(256) k_dhop_tma(const DhopParams p, int NS) {
+  dep_wait();
   using T = typename Arith<PIN>::T;
   extern __shared__ __align__(128) unsigned char smem[];
   const int LsE = p.LsE, LsP = p.LsP;
@@ -196,6 +197,7 @@ __host__ __device__ inline unsigned tmaw_warp_bytes(int NSW, int LsE, int LsP, i
 
 template <int PIN, int POUT, int GP, int DAG, int N, int EPI, int STAGES, int LSPC = 0>
 __global__ void __launch_bounds__(256) k_dhop_tmaw(const DhopParams p_) {
+  dep_wait();
   using T = typename Arith<PIN>::T;
   extern __shared__ __align__(128) unsigned char smem[];
   DhopParams p = p_;

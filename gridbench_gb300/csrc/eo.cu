@@ -127,6 +127,7 @@ __device__ __forceinline__ void m5_sweeps(const V& v, int Ls, T ia5, T g, T mf, 
 // being the time of its bytes.
 template <int P, int DAG, int N, int LSC>
 __global__ void __launch_bounds__(192) k_m5inv(const M5InvParams p) {
+  dep_wait();
   using T = typename Arith<P>::T;
   extern __shared__ __align__(16) unsigned char m5_smem[];
   cpx<T>* tile = reinterpret_cast<cpx<T>*>(m5_smem);  // [nsb][12][Ls | 1] (rows of an odd stride)
@@ -239,14 +240,14 @@ int m5inv(gbdw_field* out, const gbdw_field* in, double M5, double mf, int dag) 
   const bool pair = Ls % 2 == 0;
 #define GBDW_M5(P)                                                                               \
   if (Ls == 16) {                                                                                \
-    if (dag) k_m5inv<P, 1, 2, 16><<<g, threads, smem, stream()>>>(p);                            \
-    else k_m5inv<P, 0, 2, 16><<<g, threads, smem, stream()>>>(p);                                \
+    if (dag) launch_after(k_m5inv<P, 1, 2, 16>, g, threads, smem, p);                            \
+    else launch_after(k_m5inv<P, 0, 2, 16>, g, threads, smem, p);                                \
   } else if (pair) {                                                                             \
-    if (dag) k_m5inv<P, 1, 2, 0><<<g, threads, smem, stream()>>>(p);                             \
-    else k_m5inv<P, 0, 2, 0><<<g, threads, smem, stream()>>>(p);                                 \
+    if (dag) launch_after(k_m5inv<P, 1, 2, 0>, g, threads, smem, p);                             \
+    else launch_after(k_m5inv<P, 0, 2, 0>, g, threads, smem, p);                                 \
   } else {                                                                                       \
-    if (dag) k_m5inv<P, 1, 1, 0><<<g, threads, smem, stream()>>>(p);                             \
-    else k_m5inv<P, 0, 1, 0><<<g, threads, smem, stream()>>>(p);                                 \
+    if (dag) launch_after(k_m5inv<P, 1, 1, 0>, g, threads, smem, p);                             \
+    else launch_after(k_m5inv<P, 0, 1, 0>, g, threads, smem, p);                                 \
   }
   if (in->prec == GBDW_F64) {
     GBDW_M5(GBDW_F64)

@@ -286,6 +286,7 @@ __global__ void k_import_sites(const SRC* __restrict__ src, int64_t nsite, int L
 template <class DST, int P, bool SINGLE>
 __global__ void k_export_sites(const void* __restrict__ srcd, const float* __restrict__ norm, int64_t nsite, int Ls,
                                int LsE, int e0, DST* __restrict__ dst, int LsP) {
+  dep_wait();
   extern __shared__ __align__(16) unsigned char sm[];
   constexpr int TS = kTile<DST>, V = 16 / sizeof(DST);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -339,6 +340,7 @@ __global__ void k_export_sites(const void* __restrict__ srcd, const float* __res
     }
   }
   __syncwarp();
+  dep_release();
   uint4* d = reinterpret_cast<uint4*>(dst + site * 24 * Ls);
   constexpr int VE = 24 / V;
   for (int i = lane; i < VE * Ls; i += 32) {
@@ -351,6 +353,7 @@ __global__ void k_export_sites(const void* __restrict__ srcd, const float* __res
 template <int PS, int PD>
 __global__ void k_field_convert(const void* src, const float* snorm, void* dst, float* dnorm, int64_t nsite, int LsE,
                                 int LsPs, int LsPd) {
+  dep_wait();
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i >= nsite * LsE) return;
   const int64_t site = i / LsE;
@@ -377,7 +380,7 @@ int field_convert(gbdw_field* dst, const gbdw_field* src) {
   if (n == 0) return GBDW_OK;
   const int t = 256;
 #define GBDW_CONV(PS, PD) \
-  k_field_convert<PS, PD><<<nblk(n, t), t, 0, stream()>>>(src->d, src->norm, dst->d, dst->norm, src->lat->nsite, src->LsE, \
+  launch_after(k_field_convert<PS, PD>, nblk(n, t), t, 0, src->d, src->norm, dst->d, dst->norm, src->lat->nsite, src->LsE, \
                                                           src->LsP, dst->LsP)
   const int key = src->prec * 4 + dst->prec;
   switch (key) {
@@ -734,7 +737,7 @@ static int field_export(const gbdw_field* f, int rhs, void* dst, int dst_prec, b
   if (blocks && (uintptr_t(ddst) & 15) == 0) {
     const unsigned nb = unsigned((L->nsite + warps - 1) / warps);
 #define GBDW_EB(DST, P)                                                                                       \
-  (single ? k_export_sites<DST, P, true> : k_export_sites<DST, P, false>)<<<nb, 32 * warps, warps * warp_smem, stream()>>>( \
+  launch_after(single ? k_export_sites<DST, P, true> : k_export_sites<DST, P, false>, nb, 32 * warps, warps * warp_smem, \
       f->d, f->norm, L->nsite, L->Ls, f->LsE, rhs * L->Ls, (DST*)ddst, f->LsP)
     if (dst_prec == GBDW_F64) {
       if (f->prec == GBDW_F64) GBDW_EB(double, GBDW_F64);

@@ -135,6 +135,7 @@ __device__ __forceinline__ void apply5(const Coef5& c, const void* v, const floa
 
 template <int P, int DAG, int N, bool TWO>
 __global__ void __launch_bounds__(128) k_m5d(const __grid_constant__ M5DParams p) {
+  dep_wait();
   using T = typename Arith<P>::T;
   const int G = p.Ls / N;
   const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
@@ -303,11 +304,11 @@ int m5d(gbdw_field* out, const gbdw_field* x, const Coef5& a, const gbdw_field* 
   const unsigned g = nblk(n, 128);
 #define GBDW_M5D_N(P, N)                                                          \
   if (y) {                                                                        \
-    if (dag) k_m5d<P, 1, N, true><<<g, 128, 0, stream()>>>(p);                    \
-    else k_m5d<P, 0, N, true><<<g, 128, 0, stream()>>>(p);                        \
+    if (dag) launch_after(k_m5d<P, 1, N, true>, g, 128, 0, p);                    \
+    else launch_after(k_m5d<P, 0, N, true>, g, 128, 0, p);                        \
   } else {                                                                        \
-    if (dag) k_m5d<P, 1, N, false><<<g, 128, 0, stream()>>>(p);                   \
-    else k_m5d<P, 0, N, false><<<g, 128, 0, stream()>>>(p);                       \
+    if (dag) launch_after(k_m5d<P, 1, N, false>, g, 128, 0, p);                   \
+    else launch_after(k_m5d<P, 0, N, false>, g, 128, 0, p);                       \
   }
 #define GBDW_M5D(P)      \
   if (pair) {            \
