@@ -34,11 +34,35 @@ std::string key_text(const TuneKey& k) {
 }
 }  // namespace
 
+// Slices of t per CTA for an untuned sweep of `columns` 2x2x2 columns (times slice tiles): the cheapest
+// by the waves it takes.  A slice costs a CTA the first number below with its SM to itself and the last
+// with every slot of it taken (us; measured from 8^4 x 16 to 24^4 x 16), a CTA's start about one more.
+int sweep_slices(int64_t columns, int Lt, int te) {
+  static const double f8[8] = {1.95, 2.0, 2.2, 2.8, 3.4, 3.7, 4.1, 4.6}, f12[4] = {1.95, 2.3, 3.4, 4.0},
+                      f16[4] = {1.95, 2.2, 3.3, 3.7};
+  const double* f = te == 8 ? f8 : te == 12 ? f12 : f16;
+  const int64_t slots = te == 8 ? 8 : 4, sms = num_sms();
+  double best = 1e30;
+  int nt = 2;
+  for (int seg = (Lt + 15) / 16; seg <= (Lt + 1) / 2; ++seg) {  // 2 to 16 slices
+    const double mean = double(Lt) / seg;
+    const int64_t blocks = columns * seg, full = blocks / (slots * sms), rest = blocks % (slots * sms);
+    const double cost = double(full) * (mean * f[slots - 1] + 1.0) + (rest ? mean * f[(rest - 1) / sms] + 1.0 : 0.0);
+    if (cost < best) {
+      best = cost;
+      nt = (Lt + seg - 1) / seg;
+    }
+  }
+  return nt < 2 ? 2 : nt;
+}
+
 // Which form runs a shape nobody tuned.  Measured on lattices from 4^4 to 32^4 (us, hopping term / M):
-//   FP32, t-sweep against form 3:  16^4 x 8 37/40 - 49/53, 12^4 x 8 17/19 - 18/20, 10^4 x 8 12/13 - 10/12,
-//     16^4 x 12 58/65 - 64/74, 12^4 x 12 26/28 - 25/29, 24^4 x 16 268/293 - 318/332, 20^4 x 16 134/147 -
-//     135/146: rows of 8 or 12 slices from 400 thousand 5D sites, of 16 from 4 million (their two-thirds
-//     larger planes leave fewer CTAs to even out the last wave)
+//   FP32, t-sweep against form 3:  16^4 x 8 34/38 - 43/48, 12^4 x 8 12/14 - 15/18, 8^3 x 16 x 16 8.8/9.6 -
+//     8.9/10.6, 10^4 x 8 8.4/9.3 - 8.1/9.7, 16^4 x 12 55/62 - 60/71, 12^4 x 12 20/22 - 21/25, 24^4 x 16
+//     264/282 - 308/338, 16^4 x 16 56/61 - 57/64, 12^4 x 16 18/20 - 17/20, 8^4 x 16 6.2/6.6 - 5.0/6.3: from
+//     120 thousand 5D sites, for the hopping term on rows of 16 from a million.  Schur steps on half
+//     lattices: 16^4 x 8 23 - 29, 16^4 x 12 38 - 40, 24^4 x 8 101 - 120, but 16^4 x 16 38.8 - 37.6 and 24^4 x 16
+//     176 - 174: rows of 16 from 4 million
 //   FP32, the warp rings against form 3:  24^4 x 20 423/461 - 480/537, 16^3 x 32 x 10 114/123 - 115/132:
 //     from a million 5D sites where whole sites fill 30 lanes, and not at 16 (59/66 - 60/64) or 8
 //     (52/58 - 49/53)
@@ -55,8 +79,14 @@ DhopLaunch untuned_launch(const gbdw_gauge* g, const gbdw_field* in, int epi) {
     if (form3_ok(in, epi, 2)) return DhopLaunch{64, 2, 3};
     return DhopLaunch{128, LsE % 4 == 0 ? 4 : LsE % 2 == 0 ? 2 : 1};
   }
-  if (const int te = sweep_extent(g, in, epi, 2))
-    if (sites5 >= (te == 16 ? 4000000 : 400000)) return DhopLaunch{64, 2, 4, 4, 1, 4};
+  if (const int te = sweep_extent(g, in, epi, 2)) {
+    const bool half = in->lat->parity >= 0;
+    if (sites5 >= (te != 16 ? 120000 : half ? 4000000 : epi ? 120000 : 1000000)) {
+      const int* d = half ? in->lat->parent->dims : in->lat->dims;
+      const int64_t columns = in->lat->nsite / (8 * int64_t(d[3])) * (LsE / te);
+      return DhopLaunch{64, 2, 4, 4, 1, sweep_slices(columns, d[3], te)};
+    }
+  }
   DhopLaunch rings{64, 2, 2, 2};
   int ns, threads;
   size_t smem;
@@ -171,11 +201,10 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
       }
   }
   if (blocked_ok(g->lat, in)) cands.push_back(DhopLaunch{128, 2, 4, 4});
-  // the t-sweep with 4, 8 or 16 slices of t per CTA: more slices reread fewer planes, fewer fill the
-  // last wave better (measured best 4 to 8 on lattices from 16^4 to 32^4)
+  // the t-sweep by slices of t per CTA: more slices reread fewer planes, fewer fill the last wave better
   if (sweep_extent(g, in, 0, 2))
-    for (int nt : {4, 8, 16})
-      if (nt <= 4 || nt <= (g->lat->parity >= 0 ? g->lat->parent : g->lat)->dims[3]) cands.push_back(DhopLaunch{64, 2, 4, 4, 1, nt});
+    for (int nt : {2, 3, 4, 5, 6, 8, 12, 16})
+      if (nt <= 2 || nt <= (g->lat->parity >= 0 ? g->lat->parent : g->lat)->dims[3]) cands.push_back(DhopLaunch{64, 2, 4, 4, 1, nt});
   // FP64 fields whose operator calls run the double-single form (gbdw_set_fp64_arith): only that
   // form's shapes are timed
   const bool ds_only = in->prec == GBDW_F64 && g->prec == GBDW_F64 && !eo && fp64_double_single();

@@ -82,3 +82,19 @@ def test_mobius_adjoint_for_other_even_ls(gpu, dims, Ls):
         src = masked(c["phi"], dims, Ls, 1)
         full = mob.mobius_m(c["U"], src, c["nbr"], c["prm"], c["nsite"], Ls, 1.5, 0.5, M5, MF, 1)
         assert rel_err(ye.numpy(), halves(full, dims, Ls)[0]) < TOL[gb.F32]
+
+
+@pytest.mark.parametrize("dims,Ls", [((8, 8, 8, 11), 24), ((8, 8, 6, 10), 40), ((14, 12, 10, 11), 8)])
+def test_untuned_sweep_slices(gpu, dims, Ls):
+    """Above 120 thousand 5D sites the t-sweep, with slices per CTA that leave a shorter last piece."""
+    c = make_case(dims, Ls)
+    lat = gb.Lattice.periodic(dims, Ls)
+    g = gb.Gauge(lat, c["U"], gb.F32)
+    x, y = gb.Field(lat, gb.F32).load(c["phi"]), gb.Field(lat, gb.F32)
+    for dag in (0, 1):
+        gb.dhop(g, y, x, dag)
+        assert rel_err(y.numpy(), oracle.dslash(c["U"], c["phi"], c["nbr"], c["prm"], c["nsite"], Ls, dag)) < TOL[gb.F32]
+        n2 = gb.dwf_m(g, y, x, M5, MF, dag, want_norm=True)
+        out = y.numpy()
+        assert rel_err(out, oracle.dwf_m(c["U"], c["phi"], c["nbr"], c["nsite"], Ls, M5, MF, dag)) < TOL[gb.F32]
+        assert abs(n2 - float(np.sum(out ** 2))) / n2 < 1e-5
