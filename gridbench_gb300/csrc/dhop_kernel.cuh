@@ -690,7 +690,11 @@ __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, i
     constexpr int RP = EPI == 2 ? GBDW_F32 : GBDW_F64;
     using TR = typename Arith<RP>::T;
     const TR al = TR(*p.alpha);
-    double s = 0.0;
+    // The FP64 pipe takes some 90 clocks a warp instruction and scheduler, and an FP64 r costs it one FMA a
+    // component for the update and one for the sum; each component of the slices keeps a sum of its own.
+    // FP32 rows are added exactly in two floats instead, and widened once.
+    TR sr[N] = {}, si[N] = {};
+    float hi = 0.f, lo = 0.f;
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
       cpx<TR> rv[N];
@@ -700,10 +704,25 @@ __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, i
       for (int j = 0; j < N; ++j) {
         rv[j].r -= al * TR(v[j][k].r);
         rv[j].i -= al * TR(v[j][k].i);
-        ks += rv[j].r * rv[j].r + rv[j].i * rv[j].i;
+        if constexpr (RP == GBDW_F64) {
+          sr[j] += rv[j].r * rv[j].r;
+          si[j] += rv[j].i * rv[j].i;
+        } else {
+          ks += rv[j].r * rv[j].r + rv[j].i * rv[j].i;
+        }
       }
-      s += double(ks);
+      if constexpr (RP == GBDW_F32) {
+        const float t = hi + ks, part_of = t - hi;
+        lo += (hi - (t - part_of)) + (ks - part_of);
+        hi = t;
+      }
       Vec<RP, N>::store(p.r, site * 12 + k, s0, p.rLsP, rv);
+    }
+    double s = double(hi) + double(lo);
+    if constexpr (RP == GBDW_F64) {
+      s = sr[0] + si[0];
+#pragma unroll
+      for (int j = 1; j < N; ++j) s += sr[j] + si[j];
     }
     dpart = s;
   } else {
