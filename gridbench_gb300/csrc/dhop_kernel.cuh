@@ -895,6 +895,7 @@ struct SweepParams {
   int parity;        // parity of the output half lattice, -1 on a full lattice
   int nbx, nby, nbz; // column blocks per direction
   int ntile;         // slice tiles per site
+  int tile_pass;     // 1: one pass over the lattice per tile, 0: a column's tiles next to each other
   int nt;            // t-slices per CTA
 };
 

@@ -132,8 +132,10 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
   const uint32_t row_bytes = uint32_t(p.LsP) * 8;
   const int64_t site_bytes = int64_t(12) * row_bytes, plane_bytes = site_bytes * vol3;
   unsigned b = sweep_block(DAG);
-  const int tile = int(b % q.ntile);
-  b /= q.ntile;
+  // slice tiles of a column side by side, or a whole pass over the lattice per tile
+  const unsigned per = gridDim.x / unsigned(q.ntile);
+  const int tile = int(q.tile_pass ? b / per : b % unsigned(q.ntile));
+  b = q.tile_pass ? b % per : b / unsigned(q.ntile);
   const int x = int(b % q.nbx) * 2 + xl;
   b /= q.nbx;
   const int y = int(b % q.nby) * 2 + yl;
