@@ -331,11 +331,20 @@ __global__ void k_export_sites(const void* __restrict__ srcd, const float* __res
       }
     } else {
       const int Q = (Ls + 1) / 2;
-      for (int i = lane; i < 12 * Q; i += 32) {
-        const int row = i / Q, q = i - row * Q;
-        const float4 a = group(row, e0 + 2 * q);
-        put(row, 2 * q, a.x, a.z);
-        if (2 * q + 1 < Ls) put(row, 2 * q + 1, a.y, a.w);
+      for (int i0 = lane; i0 < 12 * Q; i0 += 128) {  // four loads ahead of the first use
+        float4 a[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int i = i0 + 32 * j, row = i / Q;
+          if (i < 12 * Q) a[j] = group(row, e0 + 2 * (i - row * Q));
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int i = i0 + 32 * j, row = i / Q, q = i - row * Q;
+          if (i >= 12 * Q) break;
+          put(row, 2 * q, a[j].x, a[j].z);
+          if (2 * q + 1 < Ls) put(row, 2 * q + 1, a[j].y, a[j].w);
+        }
       }
     }
   }
