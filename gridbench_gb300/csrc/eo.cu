@@ -118,8 +118,9 @@ __device__ __forceinline__ void m5_sweeps(const V& v, int Ls, T ia5, T g, T mf, 
   }
 }
 
-// Phase 1: one thread per (site, row) runs both sweeps into a shared-memory tile; phase 2: one
-// thread per (site, N slices) writes the tile in the field's storage format (norms for F16).
+// Phase 1: one thread per (site, row) runs both sweeps into a shared-memory tile; phase 2: for F16 one
+// thread per (site, N slices) writes the tile with its norms, else lanes along (row, N slices) write whole
+// lines.
 // LSC > 0: the launch guarantees Ls == LSC (even), and a row is loaded into registers with
 // slice-pair vector loads before the sweeps.  LSC == 0: the CTA first loads its sites into the tile,
 // lanes along (row, N slices) so that whole lines are read, and the sweeps run in place; reading the
@@ -138,18 +139,28 @@ __global__ void __launch_bounds__(192) k_m5inv(const M5InvParams p) {
   if constexpr (LSC == 0) {
     const int per_site = 12 * G;
     const int items = int(min(int64_t(p.nsb), p.nsite - site0)) * per_site;
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-      const int row = it / G, s = (it - row * G) * N;  // row counts through the CTA's sites
-      cpx<T> v[N];
-      Vec<P, N>::load(p.in, site0 * 12 + row, s, p.LsP, v);
-      if constexpr (P == GBDW_F16) {
-        float nr[N];
-        load_norms<N>(p.in_norm, (site0 + row / 12) * Ls + s, nr);
+    constexpr int B = P == GBDW_F16 ? 1 : 3;  // loads ahead of their stores to the tile
+    for (int it0 = threadIdx.x; it0 < items; it0 += B * blockDim.x) {
+      cpx<T> v[B][N];
 #pragma unroll
-        for (int j = 0; j < N; ++j) v[j] = {v[j].r * nr[j], v[j].i * nr[j]};
+      for (int i = 0; i < B; ++i) {
+        const int it = it0 + i * blockDim.x, row = it / G, s = (it - row * G) * N;  // row counts through the CTA's sites
+        if (it >= items) break;
+        Vec<P, N>::load(p.in, site0 * 12 + row, s, p.LsP, v[i]);
+        if constexpr (P == GBDW_F16) {
+          float nr[N];
+          load_norms<N>(p.in_norm, (site0 + row / 12) * Ls + s, nr);
+#pragma unroll
+          for (int j = 0; j < N; ++j) v[i][j] = {v[i][j].r * nr[j], v[i][j].i * nr[j]};
+        }
       }
 #pragma unroll
-      for (int j = 0; j < N; ++j) tile[row * LsT + s + j] = v[j];
+      for (int i = 0; i < B; ++i) {
+        const int it = it0 + i * blockDim.x, row = it / G, s = (it - row * G) * N;
+        if (it >= items) break;
+#pragma unroll
+        for (int j = 0; j < N; ++j) tile[row * LsT + s + j] = v[i][j];
+      }
     }
     __syncthreads();
   }
@@ -186,6 +197,17 @@ __global__ void __launch_bounds__(192) k_m5inv(const M5InvParams p) {
     }
   }
   __syncthreads();
+  if constexpr (P != GBDW_F16) {  // no norms: rows are written as they were read
+    const int items = int(min(int64_t(p.nsb), p.nsite - site0)) * 12 * G;
+    for (int it = threadIdx.x; it < items; it += blockDim.x) {
+      const int row = it / G, s = (it - row * G) * N;
+      cpx<T> v[N];
+#pragma unroll
+      for (int j = 0; j < N; ++j) v[j] = tile[row * LsT + s + j];
+      Vec<P, N>::store(p.out, site0 * 12 + row, s, p.LsP, v);
+    }
+    return;
+  }
   for (int it = threadIdx.x; it < p.nsb * G; it += blockDim.x) {
     const int ls = it / G;
     const int64_t site = site0 + ls;
