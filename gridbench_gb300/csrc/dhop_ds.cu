@@ -87,14 +87,6 @@ __device__ __forceinline__ ds2 operator+(ds2 a, ds2 b) {
   const float2 s = two_sum2(a.h, b.h, e);
   return join2(s, add2(e, add2(a.l, b.l)));
 }
-// c y for a unit c (codes of LegSpin)
-template <int C>
-__device__ __forceinline__ ds2 unit2(ds2 y) {
-  if constexpr (C == 0) return y;
-  else if constexpr (C == 1) return {make_float2(-y.h.x, -y.h.y), make_float2(-y.l.x, -y.l.y)};
-  else if constexpr (C == 2) return {make_float2(-y.h.y, y.h.x), make_float2(-y.l.y, y.l.x)};
-  else return {make_float2(y.h.y, -y.h.x), make_float2(y.l.y, -y.l.x)};
-}
 // One step of a compensated dot product: s + e += a b with s the running sum of the leading products
 // (every rounding error of which goes into e) and e plain FP32; a is the same real for both components
 // up to sign.
@@ -129,16 +121,33 @@ __device__ __forceinline__ ds2 split2(double2 a) {
   return join2(h, l);
 }
 
-template <int DAG, int L>
+// c y for a unit c known at run time: the components exchanged or not, times a pair of signs
+struct Unit2 {
+  bool swap;
+  float2 sign;
+};
+__device__ __forceinline__ Unit2 unit_of(int code) {  // codes of LegSpin
+  return {code >= 2, make_float2(code == 1 || code == 2 ? -1.f : 1.f, code == 1 || code == 3 ? -1.f : 1.f)};
+}
+__device__ __forceinline__ ds2 times(const Unit2& c, ds2 y) {
+  return {__fmul2_rn(c.swap ? swap2(y.h) : y.h, c.sign), __fmul2_rn(c.swap ? swap2(y.l) : y.l, c.sign)};
+}
+
+// One leg, its direction and side known at run time (and the same for the whole CTA): spins 0 and 1
+// take c0 and c1 times spins A and B.
 __device__ __forceinline__ void ds_leg(const float4* __restrict__ u, const double2* __restrict__ in, int64_t row0,
-                                       int LsE, ds2 (&acc)[12]) {
-  using S = LegSpin<DAG ? (L ^ 4) : L>;
+                                       int LsE, int leg, ds2 (&acc)[12]) {
+  const int d = leg & 3, back = leg >> 2;
+  const int spin_a = d < 2 ? 3 : 2, spin_b = d < 2 ? 2 : 3;
+  const int k0 = (d == 1 ? 0 : d == 3 ? 1 : 3) ^ back, k1 = (d == 0 ? 3 : d == 2 ? 2 : 1) ^ back;
+  const Unit2 c0 = unit_of(k0), c1 = unit_of(k1);
   ds2 h0[3], h1[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    h0[c] = split2(__ldg(in + (row0 + c) * LsE)) + unit2<S::C0>(split2(__ldg(in + (row0 + S::A * 3 + c) * LsE)));
-    h1[c] = split2(__ldg(in + (row0 + 3 + c) * LsE)) + unit2<S::C1>(split2(__ldg(in + (row0 + S::B * 3 + c) * LsE)));
+    h0[c] = split2(__ldg(in + (row0 + c) * LsE)) + times(c0, split2(__ldg(in + (row0 + spin_a * 3 + c) * LsE)));
+    h1[c] = split2(__ldg(in + (row0 + 3 + c) * LsE)) + times(c1, split2(__ldg(in + (row0 + spin_b * 3 + c) * LsE)));
   }
+  const Unit2 q0 = unit_of(k0 >= 2 ? k0 ^ 1 : k0), q1 = unit_of(k1 >= 2 ? k1 ^ 1 : k1);
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
     float2 s0 = make_float2(0.f, 0.f), e0 = s0, s1 = s0, e1 = s0;
@@ -155,18 +164,23 @@ __device__ __forceinline__ void ds_leg(const float4* __restrict__ u, const doubl
     const ds2 u0 = join2(s0, e0), u1 = join2(s1, e1);
     acc[r] = acc[r] + u0;
     acc[3 + r] = acc[3 + r] + u1;
-    acc[S::A * 3 + r] = acc[S::A * 3 + r] + unit2<conj_unit<S::C0>::v>(u0);
-    acc[S::B * 3 + r] = acc[S::B * 3 + r] + unit2<conj_unit<S::C1>::v>(u1);
+    const ds2 w0 = times(q0, u0), w1 = times(q1, u1);
+    acc[6 + r] = acc[6 + r] + (d < 2 ? w1 : w0);
+    acc[9 + r] = acc[9 + r] + (d < 2 ? w0 : w1);
   }
 }
 
 // One slice per thread, 128-thread CTAs with registers capped for MINB CTAs per SM.  What bounds the
 // kernel is its instructions on the FP32 pipe; the epilogue (M's diagonal part and |.|^2) is FP64, on a
-// pipe that is otherwise idle.  Measured (ms; Dhop, M; scalar pairs with a pair epilogue -> this):
-//   16^4 x 16  1.061, 1.45 -> 0.619, 0.717 (native FP64 1.637)   32^4 x 16  20.2, 22.9 -> 11.1, 11.5
-//   half of 16^4 x 16  0.612, 0.975 -> 0.332, 0.466
-// and 2.8e-15 from FP64 (4.0e-15 before).  Tried and slower: running some of the CTAs in native FP64
-// beside the others to use both pipes (2 of 16: 1.07 ms, 4 of 16: 1.20; they stay resident far longer
+// pipe that is otherwise idle.  The legs are one loop: eight copies of a leg are 180 KB of code, more than
+// the SM's instruction cache holds, and a quarter of the warps' time went into waiting for instructions;
+// the units and spins that a leg then selects at run time are 5 % more of them.  Measured (ms; Dhop, M;
+// scalar pairs -> packed pairs, legs unrolled -> this):
+//   16^4 x 16  1.061, 1.45 -> 0.619, 0.717 -> 0.496, 0.516 (native FP64 1.63)
+//   32^4 x 16  20.2, 22.9 -> 11.1, 11.5 -> 7.79, 8.07
+//   half of 16^4 x 16  0.612, 0.975 -> 0.332, 0.466 -> 0.253, 0.270
+// and 2.8e-15 from FP64 (4.0e-15 with scalar pairs).  Tried and slower: running some of the CTAs in native
+// FP64 beside the others to use both pipes (2 of 16: 1.07 ms, 4 of 16: 1.20; they stay resident far longer
 // than their share of the work).
 template <int DAG, int EPI, int MINB>
 __global__ void __launch_bounds__(DS_THREADS, MINB) k_dhop_ds(const DhopParams p) {
@@ -185,9 +199,11 @@ __global__ void __launch_bounds__(DS_THREADS, MINB) k_dhop_ds(const DhopParams p
     const uint32_t* nb = p.nbr4 + size_t(site) * 8;
     const float4* u = (const float4*)p.U + size_t(site) * 72;
     const double2* in = (const double2*)p.in + s0;
-#define GBDW_LEG(L) ds_leg<DAG, L>(u + 9 * L, in, int64_t(__ldg(nb + L)) * 12, p.LsE, acc);
-    GBDW_LEG(0) GBDW_LEG(4) GBDW_LEG(1) GBDW_LEG(5) GBDW_LEG(2) GBDW_LEG(6) GBDW_LEG(3) GBDW_LEG(7)
-#undef GBDW_LEG
+#pragma unroll 1
+    for (int k = 0; k < 8; ++k) {
+      const int leg = (k >> 1) + 4 * (k & 1);
+      ds_leg(u + 9 * leg, in, int64_t(__ldg(nb + leg)) * 12, p.LsE, DAG ? leg ^ 4 : leg, acc);
+    }
     cpx<double> v[1][12];
 #pragma unroll
     for (int k = 0; k < 12; ++k)
