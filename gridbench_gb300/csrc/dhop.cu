@@ -94,6 +94,19 @@ bool mobius_fusable(const gbdw_gauge* g, const gbdw_field* in, int dag) {
   return dag && in->prec == GBDW_F32 && tma_shape(in->prec, in->LsE, DhopLaunch{64, 2, 2, 2}, &ns, &threads, &smem);
 }
 
+// D5^-1 in the hopping term's epilogue (m5inv_lanes): on the t-sweep, or, for an Ls that is a power of two,
+// on form 3; a shape of another form gives way to form 3.
+DhopLaunch m5inv_launch(DhopLaunch L) { return L.mode == 4 ? L : DhopLaunch{64, 2, 3, 4, 1, L.brick}; }
+
+bool m5inv_fusable(const gbdw_gauge* g, const gbdw_field* in) {
+  const int Ls = in->lat->Ls;
+  if (!g->lat->fast || g->lat->parity < 0 || in->nrhs != 1 || in->LsE != in->LsP || Ls < 2 || Ls > 64 || Ls % 2) return false;
+  if (in->prec != GBDW_F32 && in->prec != GBDW_F16) return false;
+  const DhopLaunch L = lookup(g, in, 0);
+  if (L.mode == 4 && sweep_extent(g, in, 5, 2)) return true;
+  return (L.mode == 0 || L.mode == 3) && (Ls & (Ls - 1)) == 0 && form3_ok(in, 5, 2);
+}
+
 DhopParams make_params(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in) {
   DhopParams p;
   p.U = g->d;
@@ -154,6 +167,15 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
     p.mc = ex->mc;
     if (!dag) epi = 6;  // A(b, c) on the neighbours as they are loaded; the adjoint's is in the epilogue
   }
+  if (ex && ex->m5inv) {
+    if (epi || norm2 || cen || !m5inv_fusable(g, in)) {
+      set_error("fused D5^-1: the plain hopping term in a form that keeps whole sites in a warp");
+      return GBDW_ERR_INVALID;
+    }
+    epi = 5;
+    p.mb = ex->mb;
+    p.mc = ex->mc;
+  }
   if (cen) {
     p.cen = cen->d;
     p.cen_norm = cen->norm;
@@ -171,12 +193,13 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
   }
   // the forward Mobius M (A(b, c) on the loaded neighbours) has the hopping term's access pattern
   // and no Shamir epilogue: it runs on the hopping term's shape
-  const int key_epi = (p.mob && epi == 6) ? 0 : tune_epi;
+  const int key_epi = (p.mob && epi == 6) ? 0 : tune_epi;  // (tune_epi is 0 for D5^-1 after the hopping term)
   DhopLaunch L;
   bool tuned = find_tuned_launch(g->prec, in->prec, in->LsE, key_epi, &L);
   if (!tuned) L = untuned_launch(g, in, epi);
   if (g->lat->parity >= 0) tuned |= find_tuned_launch(g->prec, in->prec, in->LsE, key_epi + EO_KEY, &L);
   if (ex && ex->tune_key >= 0) tuned |= find_tuned_launch(g->prec, in->prec, in->LsE, ex->tune_key, &L);
+  if (epi == 5) L = m5inv_launch(L);
   if (p.mob) L.spt = 2;  // the fused adjoint works on slice pairs, one site's pairs in consecutive lanes
   if (p.mob && (in->lat->Ls & (in->lat->Ls - 1))) L = DhopLaunch{64, 2, 2, 2};  // whole sites in a warp
   // untuned hopping terms of a CTA per SM or fewer (dhop_small.cu)
@@ -197,7 +220,7 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
   if (L.mode == 3 && !form3_ok(in, epi, L.spt)) L.mode = 0;
   if (L.mode == 3) L.threads = 64;
   if (L.mode == 4) L.threads = 128;
-  p.TE = tile_extent(in->LsE, L, p.mob != 0);
+  p.TE = tile_extent(in->LsE, L, p.mob != 0 || epi == 5);
   p.brick = brick_extent(g->lat, L);
   const int64_t nthreads = p.nsite * ((p.LsE + L.spt - 1) / L.spt);
   int64_t blocks = staged ? (p.nsite + NS - 1) / NS : (nthreads + L.threads - 1) / L.threads;

@@ -476,7 +476,7 @@ struct DhopParams {
   // M epilogue (Mooee^dag in - khop A(b, c)^dag DhopDag in); with EPI 6 (FP32) A(mb, mc) is
   // applied to the neighbours as they are loaded (Mooee in - khop Dhop A(b, c) in)
   int mob = 0;
-  double mb = 1.0, mc = 0.0;
+  double mb = 1.0, mc = 0.0;  // EPI 5: 1 / a5 and 1 / (a5 (1 + mf a5^-Ls))
   // direct forms: slices per tile when each site's slices are cut into tiles (0: one tile)
   int TE = 0;
   // direct forms on periodic lattices: sweep in t-bricks of this many t-slices (0/1: natural order)
@@ -658,10 +658,78 @@ __device__ __forceinline__ void mobius_adj_hop(const DhopParams& p, int s0, cpx<
     for (int k = 0; k < 12; ++k) v[j][k] = h[j][k];
 }
 
+// ------------------------------------------------------------------ D5^-1 on a site's lanes
+// v <- D5^-1 v (DAG: D5^-dag v) on one thread's slice pair, the site's pairs being consecutive lanes of a
+// warp.  Per chirality y(s) = (v(s) + w y(s-1)) / a5, with w = -mf where s-1 wraps and 1 elsewhere (the
+// other chirality runs downwards), so with q = a5^-2 the pair's later slice is g times the sum of the
+// ring's pairs behind it, weighted q^d and by -mf beyond the wall.  The sum grows by doubling windows, and
+// both slices follow from the later one of the lane behind by the recursion itself, which shrinks the sum's
+// rounding by a5^-1 a step to that of the plain recursion.  8 to 10 exchanges a component, under the FP32
+// work of the other warps, in place of a pass of its own (k_m5inv).  Hopping term and D5^-1, us: FP16 on half
+// of 16^4 x 16 27.5 + 15.8 -> 30.6, FP32 on half of 16^3 x 32 x 12 58.6 + 33.2 -> 73.
+template <int DAG>
+__device__ __forceinline__ void m5inv_lanes(const DhopParams& p, int s0, cpx<float> (&v)[2][12]) {
+  const int G = p.LsE >> 1, lg = s0 >> 1, base = int(threadIdx.x & 31) - lg;
+  const unsigned mask = __activemask();
+  const float ia = float(p.mb), g = float(p.mc), wall = float(-p.mf);
+#pragma unroll
+  for (int ch = 0; ch < 2; ++ch) {
+    const bool down = (ch == 0) != (DAG != 0);  // s-1 feeds s
+    const int F = down ? 0 : 1, B = 1 - F, k0 = 6 * ch;
+    const int pos = down ? lg : G - 1 - lg;  // along the recursion
+    auto lane_behind = [&](int d) {
+      const int q = pos - d < 0 ? pos - d + G : pos - d;
+      return base + (down ? q : G - 1 - q);
+    };
+    cpx<float> w[6], r[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      w[k] = {fmaf(ia, v[F][k0 + k].r, v[B][k0 + k].r), fmaf(ia, v[F][k0 + k].i, v[B][k0 + k].i)};
+      r[k] = {0.f, 0.f};
+    }
+    // x += a^(2 d) w of the lane d behind
+    auto add_behind = [&](cpx<float>(&x)[6], int d, float qd) {
+      const int from = lane_behind(d);
+      const float f = pos - d < 0 ? wall * qd : qd;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const float br = __shfl_sync(mask, w[k].r, from), bi = __shfl_sync(mask, w[k].i, from);
+        x[k] = {fmaf(f, br, x[k].r), fmaf(f, bi, x[k].i)};
+      }
+    };
+    int have = 0;                       // lanes summed in r
+    float qb = ia * ia, qr = 1.f;       // q^b, q^have
+    for (int b = 1; b <= G; b *= 2) {   // w: windows of b lanes
+      if (G & b) {
+        if (have == 0) {
+#pragma unroll
+          for (int k = 0; k < 6; ++k) r[k] = w[k];
+        } else {
+          add_behind(r, have, qr);
+        }
+        have += b;
+        qr *= qb;
+      }
+      if (2 * b <= G) add_behind(w, b, qb);
+      qb *= qb;
+    }
+    const int from = lane_behind(1);
+    const float f = pos == 0 ? wall : 1.f;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const float yr = g * r[k].r, yi = g * r[k].i;
+      const float br = __shfl_sync(mask, yr, from), bi = __shfl_sync(mask, yi, from);
+      const cpx<float> y = {ia * fmaf(f, br, v[F][k0 + k].r), ia * fmaf(f, bi, v[F][k0 + k].i)};
+      v[F][k0 + k] = y;
+      v[B][k0 + k] = {ia * (v[B][k0 + k].r + y.r), ia * (v[B][k0 + k].i + y.i)};
+    }
+  }
+}
+
 // ------------------------------------------------------------------ per-site finish
 // EPI 0: store Dhop(in); EPI 1: store M(in); EPI 2 / 3 / 4: r -= alpha M(in) with r FP32 / FP64 /
 // FP16 (the CG residual update fused into the operator's second pass; M(in) is not stored);
-// EPI 6: store the Mobius M(in), A(b, c) applied to the neighbours as they are loaded.
+// EPI 5: store D5^-1 Dhop(in) (DAG: D5^-dag DhopDag(in)); EPI 6: store the Mobius M(in), A(b, c) applied to the neighbours as they are loaded.
 // Returns |what was stored|^2 in part (FP32 outputs) or dpart (FP64 outputs and EPI 2-4).
 template <int PIN, int POUT, int DAG, int N, int EPI, bool SMEM = false, class T>
 __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, int s0, int LsE, int LsP,
@@ -670,7 +738,8 @@ __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, i
   if constexpr (EPI == 1 && DAG == 1 && N == 2) {
     if (p.mob) mobius_adj_hop(p, s0, v);
   }
-  if constexpr (EPI >= 1) dwf_epilogue<PIN, DAG, N, SMEM>(p, site, s0, v, rows);
+  if constexpr (EPI == 5) m5inv_lanes<DAG>(p, s0, v);
+  else if constexpr (EPI >= 1) dwf_epilogue<PIN, DAG, N, SMEM>(p, site, s0, v, rows);
   if constexpr (EPI == 4) {
     // FP16 r: dequantise with its per-slice norms, update in FP32, store with new norms
     const float al = float(*p.alpha);
@@ -838,7 +907,7 @@ __global__ void __launch_bounds__(MINB > 0 ? MAXT : 256, MINB > 0 ? MINB : 1) k_
     }
     cpx<T> acc[N][12];
     dhop_thread<PIN, GP, DAG, N, EPI == 6>(p, site, s0, acc);
-    if constexpr (EPI <= 1 || EPI == 6) dep_release();
+    if constexpr (EPI <= 1 || EPI >= 5) dep_release();
     finish_site<PIN, POUT, DAG, N, EPI>(p, site, s0, p.LsE, p.LsP, acc, part, dpart);
   }
   if (p.partials) {

@@ -129,11 +129,35 @@ int by_shape(const DhopParams& p, DhopLaunch L) {
   return GBDW_ERR_INVALID;
 }
 
+// D5^-1 after the hopping term (epi 5): form 3
+template <int PIN, int POUT, int GP, int DAG>
+int go_m5inv(const DhopParams& p, DhopLaunch L) {
+  if (L.mode == 3 && L.spt == 2 && p.LsE == 16 && p.LsP == 16) {
+    constexpr int MB = PIN == GBDW_F16 ? 8 : 6;
+    launch_after(k_dhop<PIN, POUT, GP, DAG, 2, 5, MB, 16, 64>, unsigned((p.nsite * 8 + 63) / 64), 64, 0, p);
+    GBDW_LAUNCHED();
+    return GBDW_OK;
+  }
+  if constexpr (PIN == GBDW_F32) {
+    if (L.mode == 3 && L.spt == 2) {
+      launch_after(k_dhop<PIN, POUT, GP, DAG, 2, 5, 6, 0, 64>, unsigned((p.nsite * (p.LsE / 2) + 63) / 64), 64, 0, p);
+      GBDW_LAUNCHED();
+      return GBDW_OK;
+    }
+  }
+  set_error("hopping kernel: D5^-1 in the epilogue needs form 3 or the t-sweep");
+  return GBDW_ERR_INVALID;
+}
+
 // epi 0 Dhop, 1 M; the CG residual epilogues exist for the adjoint pass only: 2 (FP32 r, FP32
 // and FP16 spinors), 3 (FP64 r, FP32 spinors) and 4 (FP16 r, FP16 spinors with FP16 links);
 // 6 the forward Mobius M (FP32).
 template <int PIN, int POUT, int GP, int S1, int S2>
 int dispatch(const DhopParams& p, int dag, int epi, DhopLaunch L) {
+  if (epi == 5) {
+    if constexpr (PIN == GBDW_F32 || PIN == GBDW_F16)
+      return dag ? go_m5inv<PIN, POUT, GP, 1>(p, L) : go_m5inv<PIN, POUT, GP, 0>(p, L);
+  }
   if (epi == 6) {
     // the forward Mobius M (A(b, c) on the loaded neighbours): FP32 slice pairs only
     if constexpr (PIN == GBDW_F32) {

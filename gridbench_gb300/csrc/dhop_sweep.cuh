@@ -124,8 +124,10 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
   dep_wait();
   constexpr int NS = 8, G = TE / 2, SS = sweep_site_bytes(TE), ROW = TE * 8;
   extern __shared__ __align__(16) char sw_smem[];
-  const int tid = threadIdx.x;
-  const int sl = tid / G, lg = tid - sl * G;
+  // a site's slice pairs are lanes of one warp: eight sites of four pairs, four of six or eight
+  constexpr int SPW = G <= 4 ? 8 : 4;
+  const int lane = threadIdx.x & 31;
+  const int sl = int(threadIdx.x >> 5) * SPW + lane / G, lg = lane % G;
   const int xl = sl & 1, yl = (sl >> 1) & 1, zl = sl >> 2;
   const int Lx = q.L[0], Ly = q.L[1], Lz = q.L[2], Lt = q.L[3];
   const int vol3 = Lx * Ly * Lz;
@@ -142,7 +144,7 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
   b /= q.nby;
   const int z = int(b % q.nbz) * 2 + zl;
   const int ta = int(b / q.nbz) * q.nt, tb = min(ta + q.nt, Lt);
-  const bool active = sl < NS;  // whole warps are launched
+  const bool active = lane < SPW * G;  // whole warps are launched
   const int col = active ? x + Lx * (y + Ly * z) : 0;
   const int e0 = tile * TE + 2 * lg;
   const char* const gcol = reinterpret_cast<const char*>(p.in) + int64_t(e0) * 8 + col * site_bytes;
@@ -237,7 +239,7 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
       float pt = 0.f;
       double dt = 0.0;
       const int64_t site = int64_t(t) * vol3 + col;
-      if ((EPI <= 1 || EPI == 6) && !more) dep_release();
+      if ((EPI <= 1 || EPI >= 5) && !more) dep_release();
       if (!EO && EPI >= 1 && !p.cen)  // the diagonal part reads this site's plane t, in shared memory
         finish_site<GBDW_F32, GBDW_F32, DAG, 2, EPI, !EO && EPI >= 1>(p, site, e0, p.LsE, p.LsP, v, pt, dt, sc - lg * 16);
       else

@@ -27,6 +27,12 @@ int sweep_by_epi(const DhopParams& p, const SweepParams& q, unsigned blocks, int
     case 3: return go_sweep<1, 1, TE, EO>(p, q, blocks);
     case 5: return go_sweep<1, 2, TE, EO>(p, q, blocks);
     case 7: return go_sweep<1, 3, TE, EO>(p, q, blocks);
+    case 10:
+      if constexpr (EO) return go_sweep<0, 5, TE, EO>(p, q, blocks);
+      break;
+    case 11:
+      if constexpr (EO) return go_sweep<1, 5, TE, EO>(p, q, blocks);
+      break;
     case 12:
       if constexpr (pow2 && !EO) return go_sweep<0, 6, TE, EO>(p, q, blocks);
       break;

@@ -222,6 +222,23 @@ __global__ void __launch_bounds__(192) k_m5inv(const M5InvParams p) {
   }
 }
 
+// 1 / a5 and 1 / (a5 (1 + mf a5^-Ls))
+int m5inv_coefficients(int Ls, double M5, double mf, double* ia5, double* g) {
+  const double a5 = 5.0 - M5;
+  if (Ls > kMaxLsInv || !(std::fabs(a5) > 1e-6)) {
+    set_error("D5^-1: needs Ls <= 64 and M5 != 5");
+    return GBDW_ERR_INVALID;
+  }
+  const double den = a5 * (1.0 + mf * std::pow(a5, -double(Ls)));
+  if (!(std::fabs(den) > 0.0) || !std::isfinite(den)) {
+    set_error("D5^-1: singular 5th-dimension operator for these M5, mf");
+    return GBDW_ERR_INVALID;
+  }
+  *ia5 = 1.0 / a5;
+  *g = 1.0 / den;
+  return GBDW_OK;
+}
+
 bool is_half(const gbdw_lattice* l) { return l && l->parity >= 0 && l->cbsite; }
 
 }  // namespace
@@ -232,12 +249,8 @@ int m5inv(gbdw_field* out, const gbdw_field* in, double M5, double mf, int dag) 
     return GBDW_ERR_INVALID;
   }
   const int Ls = in->lat->Ls;
-  const double a5 = 5.0 - M5;
-  if (Ls > kMaxLsInv || !(std::fabs(a5) > 1e-6)) {
-    set_error("D5^-1: needs Ls <= 64 and M5 != 5");
-    return GBDW_ERR_INVALID;
-  }
   M5InvParams p;
+  if (int st = m5inv_coefficients(Ls, M5, mf, &p.ia5, &p.g)) return st;
   p.in = in->d;
   p.in_norm = in->norm;
   p.out = out->d;
@@ -246,13 +259,6 @@ int m5inv(gbdw_field* out, const gbdw_field* in, double M5, double mf, int dag) 
   p.Ls = Ls;
   p.LsP = in->LsP;
   p.mf = mf;
-  p.ia5 = 1.0 / a5;
-  const double den = a5 * (1.0 + mf * std::pow(a5, -double(Ls)));
-  if (!(std::fabs(den) > 0.0) || !std::isfinite(den)) {
-    set_error("D5^-1: singular 5th-dimension operator for these M5, mf");
-    return GBDW_ERR_INVALID;
-  }
-  p.g = 1.0 / den;
   if (int st = ensure_device()) return st;
   const size_t per_site = 12 * size_t(Ls | 1) * (in->prec == GBDW_F64 ? 16 : 8);
   p.nsb = int(std::min<size_t>(16, 49152 / per_site));
@@ -310,6 +316,22 @@ int hop_eo(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag, 
   return run_dhop(g, out, in, dag ? 1 : 0, cen ? 1 : 0, 5.0 - M5, mf, norm2, fetch, cen, khop, ex);
 }
 
+// out = D5^-1 Dhop in (dag: D5^-dag DhopDag in) on g's half: in one pass where the hopping kernel can, with
+// tmp = Dhop in in between otherwise
+int hop_m5inv(const gbdw_gauge* g, gbdw_field* out, gbdw_field* tmp, const gbdw_field* in, double M5, double mf,
+              int dag) {
+  if (int st = check_eo(g, tmp, in)) return st;
+  if (int st = check_eo(g, out, in)) return st;
+  if (m5inv_fusable(g, in)) {
+    DhopExtra ex;
+    ex.m5inv = true;
+    if (int st = m5inv_coefficients(in->lat->Ls, M5, mf, &ex.mb, &ex.mc)) return st;
+    return run_dhop(g, out, in, dag ? 1 : 0, 0, 0.0, mf, nullptr, true, nullptr, 0.5, &ex);
+  }
+  if (int st = hop_eo(g, tmp, in, dag, nullptr, M5, mf, 0.5, nullptr, true)) return st;
+  return m5inv(out, tmp, M5, mf, dag);
+}
+
 int mpc(const gbdw_gauge* gp, const gbdw_gauge* gq, gbdw_field* out, gbdw_field* tq1, gbdw_field* tq2,
         const gbdw_field* in, double M5, double mf, int dag, double* norm2, bool fetch) {
   if (!gp || !gq || gq->lat != gp->lat->partner) {
@@ -320,8 +342,7 @@ int mpc(const gbdw_gauge* gp, const gbdw_gauge* gq, gbdw_field* out, gbdw_field*
     set_error("Schur operator: two distinct temporaries on the other half, out != in");
     return GBDW_ERR_INVALID;
   }
-  if (int st = hop_eo(gq, tq1, in, dag, nullptr, M5, mf, 0.5, nullptr, true)) return st;
-  if (int st = m5inv(tq2, tq1, M5, mf, dag)) return st;
+  if (int st = hop_m5inv(gq, tq2, tq1, in, M5, mf, dag)) return st;
   return hop_eo(gp, out, tq2, dag, in, M5, mf, 0.25, norm2, fetch);
 }
 
@@ -358,16 +379,14 @@ int mpcdagmpc_residual(const gbdw_gauge* gp, const gbdw_gauge* gq, gbdw_field* s
   e1.sum_to = s + CG_PAP;
   e1.num = rule.rr;
   e1.alpha_to = s + CG_ALPHA;
-  if (int st = hop_eo(gq, tq1, in, 0, nullptr, M5, mf, 0.5, nullptr, true)) return st;
-  if (int st = m5inv(tq2, tq1, M5, mf, 0)) return st;
+  if (int st = hop_m5inv(gq, tq2, tq1, in, M5, mf, 0)) return st;
   if (int st = hop_eo(gp, tp, tq2, 0, in, M5, mf, 0.25, nullptr, false, &e1)) return st;
   DhopExtra e2;
   e2.r = r;
   e2.alpha = s + CG_ALPHA;
   e2.sum_to = s + CG_RR;
   e2.rule = &rule;
-  if (int st = hop_eo(gq, tq1, tp, 1, nullptr, M5, mf, 0.5, nullptr, true)) return st;
-  if (int st = m5inv(tq2, tq1, M5, mf, 1)) return st;
+  if (int st = hop_m5inv(gq, tq2, tq1, tp, M5, mf, 1)) return st;
   return hop_eo(gp, sink, tq2, 1, tp, M5, mf, 0.25, nullptr, false, &e2);
 }
 

@@ -19,6 +19,9 @@ struct DhopExtra {
   // on DhopDag in before the epilogue (dag 1); epi 1, one right-hand side, Ls a power of two <= 64
   bool mobius = false;
   double mb = 1.0, mc = 0.0;
+  // D5^-1 of the hopping term (dag: D5^-dag) in one pass, with mb = 1 / a5 and mc = 1 / (a5 (1 + mf a5^-Ls));
+  // epi 0 on a half lattice, where m5inv_fusable
+  bool m5inv = false;
   // a tune-cache key to take the launch shape from when it holds one (else the epilogue's own)
   int tune_key = -1;
 };
@@ -58,5 +61,8 @@ int tile_extent(int LsE, const DhopLaunch& L, bool whole_sites);
 int brick_extent(const gbdw_lattice* lat, const DhopLaunch& L);
 // the Mobius operator (dag 0) or its adjoint (dag 1) can be fused into the hopping pass for these
 // operands (DhopExtra::mobius)
+bool m5inv_fusable(const gbdw_gauge* g, const gbdw_field* in);
+// the shape run_dhop takes for epilogue key epi with this gauge field
+DhopLaunch lookup(const gbdw_gauge* g, const gbdw_field* in, int epi);
 bool mobius_fusable(const gbdw_gauge* g, const gbdw_field* in, int dag);
 }  // namespace gbdw
