@@ -11,13 +11,17 @@
 //
 // 2 x 2 x 2 because each thread then has exactly one outside neighbour per direction, in every
 // warp; four CTAs of 64 threads fit an SM (34 KB and 246 registers a thread).  Hopping term, us,
-// this form / the best of the others (TMA warp rings or form 3) / all bytes once at the copy rate:
-//   16^4 x 8    37 / 49 / 20      24^4 x 8   160 / 215 / 104     24^4 x 12  247 / 287 / 141
-//   16^4 x 16   60 / 59 / 35      24^4 x 16  268 / 303 / 179     32^4 x 16  847 / 1016 / 565
-//   24^4 x 32  540 / 618 / 329    half of 32^4 x 16  404 / 506 / 283
+// this form / the best of the others (TMA warp rings or form 3, before launches overlapped) / all bytes once
+// at the copy rate:
+//   16^4 x 8    34 / 49 / 20      24^4 x 8   152 / 215 / 104     24^4 x 12  247 / 287 / 141
+//   16^4 x 16   56 / 59 / 35      24^4 x 16  264 / 303 / 179     32^4 x 16  847 / 1016 / 565
+//   24^4 x 32  521 / 618 / 329    half of 32^4 x 16  404 / 506 / 283
 // With the planes, links and stores taken away the 32^4 case still takes 528 us: the FMA pipes are
-// busy for 390 us of it, and two warps per scheduler don't hide all of the rest.  Lattices of a few
-// waves of CTAs (16^4 x 16) lose what they gain to the last wave.
+// busy for 390 us of it, and two warps per scheduler don't hide all of the rest (37 % of the issue slots
+// used; a third of the stalls wait for L2).  Three, at 168 registers with 24 to 64 bytes spilled, are slower
+// at every size: the loads move back towards their use (16^4 x 16 62 us, 32^4 x 16 961).  Lattices of a few
+// waves of CTAs (16^4 x 16) lose what they gain to the last wave; sweep_slices (tune.cu) looks for the
+// cheapest waves.
 // Tried and slower: 4 x 2 x 2 and 4 x 4 x 2 columns with 2.5 / 2 loads from L2 a site, waited for
 // at once (72 / 80 us at 16^4); two threads per slice pair, one per spin pair (12 to 16 warps but
 // 46 % more instructions: 64 us, 971 us at 32^4); one persistent CTA per slot (the columns drift
