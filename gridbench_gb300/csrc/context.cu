@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict_
   if (threadIdx.x == 0) {
     result[0] = v[0];
     if (alpha_out) alpha_out[0] = num / v[0];
-    if (rule.rr > 0.0) {
+    if (host) {  // a rule was given: all five are written, whatever rr is (NaN after a broken residual)
       double* s = result - CG_RR;
       s[CG_BETA] = v[0] / rule.rr;
       const bool go = s[CG_PAP] > 0.0 && isfinite(s[CG_PAP]) && isfinite(v[0]) && !(v[0] < rule.update) && !(v[0] <= rule.stop);
@@ -259,7 +259,7 @@ int sum_partials(const double* partials, int64_t n, double* result, double num, 
   const int threads = n >= 4096 ? 1024 : 256;
   launch_after(k_sum_partials, unsigned(ctas), threads, 0, partials, n, (double*)(s + 1024), (unsigned*)(s + 1536),
                                                            result, num, alpha_out, rule ? *rule : CgRule{0.0, 0.0, 0.0},
-                                                           g_pinned + 32);
+                                                           rule ? g_pinned + 32 : nullptr);
   GBDW_LAUNCHED();
   return GBDW_OK;
 }
