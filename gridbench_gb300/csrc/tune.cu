@@ -137,6 +137,22 @@ void pin_launch(const gbdw_gauge* g, const gbdw_field* in, const DhopLaunch& L) 
   for (int rp : cg_residual_precs(g->prec, in->prec)) set_tuned_launch(g->prec, in->prec, in->LsE, cg_step_key(rp), L);
 }
 
+// Where a pin of the tile split or of the t-brick starts: the tuned or pinned shape, and for a field without
+// one a direct form on every lattice size (the rules may choose the sweep or the rings, which have neither):
+// form 3, or form 0 where `takes` says that form 3's slice pairs don't fit the number.
+template <class TAKES>
+DhopLaunch pin_base(const gbdw_gauge* g, const gbdw_field* in, const TAKES& takes) {
+  const int ko = g->lat->parity >= 0 ? EO_KEY : 0;
+  DhopLaunch L;
+  const DhopLaunch now = lookup(g, in, 0);
+  if (find_tuned_launch(g->prec, in->prec, in->LsE, 0, &L) || find_tuned_launch(g->prec, in->prec, in->LsE, ko, &L))
+    return now;
+  L = now.mode == 0 || now.mode == 3 ? now : DhopLaunch{64, 2, 3};
+  if (takes(L)) return L;
+  const int spt = in->prec == GBDW_F64 || in->LsE % 2 ? 1 : in->prec == GBDW_F16 && in->LsE % 4 == 0 ? 4 : 2;
+  return DhopLaunch{128, spt};
+}
+
 bool same_launch(const DhopLaunch& a, const DhopLaunch& b) {
   return a.threads == b.threads && a.spt == b.spt && a.mode == b.mode && a.stages == b.stages && a.split == b.split &&
          a.brick == b.brick;
@@ -444,9 +460,13 @@ int gbdw_tune_split(const gbdw_gauge* g, const gbdw_field* in, int* split) {
 
 int gbdw_tune_set_split(const gbdw_gauge* g, const gbdw_field* in, int split) {
   if (!g || !in) return GBDW_ERR_INVALID;
-  DhopLaunch L = lookup(g, in, 0);
+  auto takes = [&](DhopLaunch q) {
+    q.split = split;
+    return split == 1 || (split > 1 && tile_extent(in->LsE, q, false) > 0);
+  };
+  DhopLaunch L = pin_base(g, in, takes);
   L.split = split;
-  if (split < 1 || (split > 1 && tile_extent(in->LsE, L, false) == 0)) {
+  if (!takes(L)) {
     set_error("gbdw_tune_set_split: the chosen form must be direct (0 or 3) and Ls*nrhs must split into whole "
               "slice groups");
     return GBDW_ERR_INVALID;
@@ -463,9 +483,14 @@ int gbdw_tune_brick(const gbdw_gauge* g, const gbdw_field* in, int* brick) {
 
 int gbdw_tune_set_brick(const gbdw_gauge* g, const gbdw_field* in, int brick) {
   if (!g || !in) return GBDW_ERR_INVALID;
-  DhopLaunch L = lookup(g, in, 0);
+  auto takes = [&](DhopLaunch q) {
+    q.brick = brick;
+    if (q.mode == 4 && in->prec == GBDW_F32) return brick >= 1 && brick <= 64;
+    return brick == 1 || (brick > 1 && brick_extent(g->lat, q) > 0);
+  };
+  DhopLaunch L = pin_base(g, in, takes);
   L.brick = brick;
-  if (brick < 1 || (L.mode == 4 && in->prec == GBDW_F32 ? brick > 64 : brick > 1 && brick_extent(g->lat, L) == 0)) {
+  if (!takes(L)) {
     set_error("gbdw_tune_set_brick: the chosen form must be direct (0 or 3) on a periodic lattice whose Lt the "
               "brick divides");
     return GBDW_ERR_INVALID;

@@ -367,7 +367,8 @@ int gbdw_tune_set(const gbdw_gauge* g, const gbdw_field* in, int threads, int sp
  * site's spinor is reused by its neighbours within a shorter stretch of the sweep.  The tuner
  * chooses among the splits 1, 2, 3, 4, 6, 8, 12, 16 that cut whole slice groups;
  * gbdw_tune_split reads the choice for fields like `in`, gbdw_tune_set_split pins it (1 = whole
- * sites; gbdw_tune_set resets it to 1). */
+ * sites; gbdw_tune_set resets it to 1).  On a field that nothing was tuned or pinned for, the pin of
+ * a split (and of a brick, below) takes a direct form with it, whichever form the field runs untuned. */
 int gbdw_tune_split(const gbdw_gauge* g, const gbdw_field* in, int* split);
 int gbdw_tune_set_split(const gbdw_gauge* g, const gbdw_field* in, int split);
 /* t-brick sweep order of the direct forms on periodic lattices: sites are visited as (t brick,
@@ -375,7 +376,7 @@ int gbdw_tune_set_split(const gbdw_gauge* g, const gbdw_field* in, int split);
  * of a whole 3D volume apart (what lets a site's spinor leave L2 before its next reader when a
  * site holds many slices, e.g. many right-hand sides).  The tuner chooses among 1 (natural order),
  * 2, 4, 8; gbdw_tune_brick reads the choice, gbdw_tune_set_brick pins it (Lt must be a multiple).
- * For FP32 in form 4 the number is the slices of t one CTA walks (1: the built-in 8). */
+ * For FP32 tuned to or pinned at form 4 the number is the slices of t one CTA walks (1: the built-in 8). */
 int gbdw_tune_brick(const gbdw_gauge* g, const gbdw_field* in, int* brick);
 int gbdw_tune_set_brick(const gbdw_gauge* g, const gbdw_field* in, int brick);
 /* The shape of the Shamir M pass (and of the CG passes built on it) for fields like `in` with one
