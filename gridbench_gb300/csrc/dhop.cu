@@ -214,8 +214,11 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
   if (!slices_ok(in, epi, L.spt, L.mode)) L.spt = 1;
   int NS = 0, tthreads = 0;
   size_t smem = 0;
-  const bool staged = L.mode == 1 || L.mode == 2;
-  if (staged && !tma_shape(in->prec, in->LsE, L, &NS, &tthreads, &smem)) L.mode = 0;
+  bool staged = L.mode == 1 || L.mode == 2;
+  if (staged && !tma_shape(in->prec, in->LsE, L, &NS, &tthreads, &smem)) {
+    L.mode = 0;
+    staged = false;
+  }
   // fall back before fixing the CTA size: the block count below must match the launch
   if (L.mode == 3 && !form3_ok(in, epi, L.spt)) L.mode = 0;
   if (L.mode == 3) L.threads = 64;
