@@ -234,11 +234,17 @@ __device__ __forceinline__ cp2 hproj(uint2 x, uint2 y) {
 struct MobLeg {
   float b, c, clo, chi;  // clo: coefficient of slice s0's s-1 term, chi: of slice s0+1's s+1 term
   int G, from_lo, from_hi;
+  unsigned mask;
 };
+// The G consecutive lanes of a warp, from `base`, that hold one site's slice pairs: the lanes an exchange
+// inside the site takes part with.  They are active or inactive together in every form that exchanges;
+// which other lanes of the warp stand at the same place is the compiler's business (__activemask() would ask).
+__device__ __forceinline__ unsigned site_lanes(int base, int G) { return (0xffffffffu >> (32 - G)) << base; }
 __device__ __forceinline__ MobLeg make_mobleg(int Ls, double b, double c, double mf, int s0) {
   MobLeg m;
   m.G = Ls >> 1;
   const int lg = int(threadIdx.x) & (m.G - 1);
+  m.mask = site_lanes((int(threadIdx.x) & 31) - lg, m.G);
   m.from_lo = (lg + m.G - 1) & (m.G - 1);
   m.from_hi = (lg + 1) & (m.G - 1);
   m.b = float(b);
@@ -249,15 +255,13 @@ __device__ __forceinline__ MobLeg make_mobleg(int Ls, double b, double c, double
 }
 // spins 0, 1 (P+): slice s0 takes psi(s0-1) from the lane below, slice s0+1 takes psi(s0)
 __device__ __forceinline__ void mob_lower(cp2& a, const MobLeg& m) {
-  const unsigned mask = __activemask();
-  const float mr = __shfl_sync(mask, a.r.y, m.from_lo, m.G), mi = __shfl_sync(mask, a.i.y, m.from_lo, m.G);
+  const float mr = __shfl_sync(m.mask, a.r.y, m.from_lo, m.G), mi = __shfl_sync(m.mask, a.i.y, m.from_lo, m.G);
   a.r = __ffma2_rn(make_float2(m.b, m.b), a.r, make_float2(m.clo * mr, m.c * a.r.x));
   a.i = __ffma2_rn(make_float2(m.b, m.b), a.i, make_float2(m.clo * mi, m.c * a.i.x));
 }
 // spins 2, 3 (P-): slice s0 takes psi(s0+1), slice s0+1 takes psi(s0+2) from the lane above
 __device__ __forceinline__ void mob_upper(cp2& a, const MobLeg& m) {
-  const unsigned mask = __activemask();
-  const float qr = __shfl_sync(mask, a.r.x, m.from_hi, m.G), qi = __shfl_sync(mask, a.i.x, m.from_hi, m.G);
+  const float qr = __shfl_sync(m.mask, a.r.x, m.from_hi, m.G), qi = __shfl_sync(m.mask, a.i.x, m.from_hi, m.G);
   a.r = __ffma2_rn(make_float2(m.b, m.b), a.r, make_float2(m.c * a.r.y, m.chi * qr));
   a.i = __ffma2_rn(make_float2(m.b, m.b), a.i, make_float2(m.c * a.i.y, m.chi * qi));
 }
@@ -630,8 +634,8 @@ __device__ __forceinline__ void dwf_epilogue(const DhopParams& p, int64_t site, 
 template <class T>
 __device__ __forceinline__ void mobius_adj_hop(const DhopParams& p, int s0, cpx<T> (&v)[2][12]) {
   const int G = p.Ls >> 1, lg = s0 >> 1;  // lanes per site, this one's place among them
-  const unsigned mask = __activemask();
   const int base = int(threadIdx.x & 31) - lg;
+  const unsigned mask = site_lanes(base, G);
   const int from_lo = base + (lg == 0 ? G - 1 : lg - 1), from_hi = base + (lg == G - 1 ? 0 : lg + 1);
   cpx<T> vm[6], vp[6];
 #pragma unroll
@@ -670,7 +674,7 @@ __device__ __forceinline__ void mobius_adj_hop(const DhopParams& p, int s0, cpx<
 template <int DAG>
 __device__ __forceinline__ void m5inv_lanes(const DhopParams& p, int s0, cpx<float> (&v)[2][12]) {
   const int G = p.LsE >> 1, lg = s0 >> 1, base = int(threadIdx.x & 31) - lg;
-  const unsigned mask = __activemask();
+  const unsigned mask = site_lanes(base, G);
   const float ia = float(p.mb), g = float(p.mc), wall = float(-p.mf);
 #pragma unroll
   for (int ch = 0; ch < 2; ++ch) {
