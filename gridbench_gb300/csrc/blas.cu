@@ -27,7 +27,7 @@ struct Calc<GBDW_F64> {
 
 template <int P, class T>
 __device__ __forceinline__ void ld24(const void* d, const float* nrm, int64_t site, int e, int LsE, int LsP, T (&v)[24]) {
-  const float n = (P == GBDW_F16) ? __ldg(nrm + site * LsE + e) : 1.f;
+  const float n = (P == GBDW_F16) ? nrm[site * LsE + e] : 1.f;
 #pragma unroll
   for (int k = 0; k < 12; ++k) {
     const auto a = Elem<P>::ld(d, site * 12 + k, e, LsP);
@@ -116,9 +116,12 @@ __global__ void k_dot(FieldRef x, FieldRef y, int64_t nsite, int LsE, Reduce red
   grid_sum<2>(acc, red.partials, red.counter, red.result);
 }
 
-// y = a x + b y
+constexpr int kThreads = 256;
+
+// y = a x + b y (FP16: 64 registers; left alone the loads ahead of the stores take 72, and 24^4 x 12 174 us for 171)
 template <int PX, int PY>
-__global__ void k_axpby(double a, FieldRef x, double b, FieldOut y, int64_t nsite, int LsE) {
+__global__ void __launch_bounds__(kThreads, PY == GBDW_F16 ? 4 : 0)
+    k_axpby(double a, FieldRef x, double b, FieldOut y, int64_t nsite, int LsE) {
   using T = typename Calc<(PX == GBDW_F64 || PY == GBDW_F64) ? GBDW_F64 : GBDW_F32>::T;
   const int64_t n = nsite * LsE;
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
@@ -178,16 +181,17 @@ struct CgStep {
   const double* dev;
   __device__ __forceinline__ bool go() {
     if (!dev) return true;
-    alpha = __ldg(dev + CG_ALPHA);
-    beta = __ldg(dev + CG_BETA);
-    return __ldg(dev + CG_GO) != 0.0;
+    alpha = dev[CG_ALPHA];
+    beta = dev[CG_BETA];
+    return dev[CG_GO] != 0.0;
   }
 };
 
-// x += alpha p ; p = r + beta p (both with the old p) ; optionally q = p
+// x += alpha p ; p = r + beta p (both with the old p) ; optionally q = p.  Two CTAs per SM: three fields' rows
+// loaded ahead of the stores would take 168 registers
 template <int PX, int PP, int PR, int PQ>
-__global__ void k_cg_xp(CgStep cg, FieldOut x, FieldOut p, FieldRef r, FieldOut q, int64_t nsite,
-                        int LsE) {
+__global__ void __launch_bounds__(kThreads, 2)
+    k_cg_xp(CgStep cg, FieldOut x, FieldOut p, FieldRef r, FieldOut q, int64_t nsite, int LsE) {
   using T = typename Calc<(PX == GBDW_F64 || PR == GBDW_F64) ? GBDW_F64 : GBDW_F32>::T;
   const int64_t n = nsite * LsE;
   if (!cg.go()) return;
@@ -231,7 +235,6 @@ __global__ void k_cg_p(double beta, FieldRef r, FieldOut p, FieldOut q, int64_t 
 FieldRef ref(const gbdw_field* f) { return FieldRef{f->d, f->norm, f->LsP}; }
 FieldOut out(gbdw_field* f) { return FieldOut{f->d, f->norm, f->LsP}; }
 
-constexpr int kThreads = 256;
 int64_t grid_for(const gbdw_field* f) {
   const int64_t n = f->lat->nsite * f->LsE;
   int64_t g = (n + kThreads - 1) / kThreads;
@@ -266,7 +269,7 @@ __device__ __forceinline__ void ld_pair(const void* d, const float* nrm, int64_t
 }
 
 template <int PX, int PP, int PR>
-__global__ void k_cg_xp_pairs(CgStep cg, FieldOut x, FieldOut p, FieldRef r, int64_t nsite, int LsE) {
+__global__ void __launch_bounds__(kThreads, 2) k_cg_xp_pairs(CgStep cg, FieldOut x, FieldOut p, FieldRef r, int64_t nsite, int LsE) {
   dep_wait();
   const int G = LsE / 2;
   const int64_t n = nsite * G;
@@ -441,7 +444,7 @@ __global__ void __launch_bounds__(kSumThreads, 2) k_norm2_flat(const void* x_, i
   double acc[1] = {0.0};
   typename Arith<P>::T s[2] = {};
   V u[2 * kVec];
-  flat_loop<2 * kVec>(n, [&](int64_t i, int k) { u[k] = __ldg(x + i); },
+  flat_loop<2 * kVec>(n, [&](int64_t i, int k) { u[k] = x[i]; },
                       [&](int64_t, int k) { norm_v(u[k], s[k / kVec]); },
                       [&] {
                         acc[0] += double(s[0]);
@@ -460,7 +463,7 @@ __global__ void __launch_bounds__(kSumThreads, 2) k_dot_flat(const void* x_, con
   double acc[2] = {0.0, 0.0};
   typename Arith<P>::T re = 0, im = 0;
   V u[kVec], v[kVec];
-  flat_loop(n, [&](int64_t i, int k) { u[k] = __ldg(x + i); v[k] = __ldg(y + i); },
+  flat_loop(n, [&](int64_t i, int k) { u[k] = x[i]; v[k] = y[i]; },
             [&](int64_t, int k) { dot_v(u[k], v[k], re, im); },
             [&] {
               acc[0] += double(re);
@@ -473,12 +476,11 @@ __global__ void __launch_bounds__(kSumThreads, 2) k_dot_flat(const void* x_, con
 
 // r = b - t, |r|^2 (FP64)
 __global__ void __launch_bounds__(kSumThreads, 2)
-    k_xmy_norm_flat(const double2* __restrict__ b, const double2* __restrict__ t, double2* __restrict__ r, int64_t n,
-                    Reduce red) {
+    k_xmy_norm_flat(const double2* b, const double2* t, double2* r, int64_t n, Reduce red) {
   dep_wait();
   double acc[1] = {0.0};
   double2 u[2], v[2];
-  flat_loop<2>(n, [&](int64_t i, int k) { u[k] = __ldg(b + i); v[k] = __ldg(t + i); },
+  flat_loop<2>(n, [&](int64_t i, int k) { u[k] = b[i]; v[k] = t[i]; },
             [&](int64_t i, int k) {
               const double2 d = make_double2(u[k].x - v[k].x, u[k].y - v[k].y);
               r[i] = d;
@@ -490,23 +492,24 @@ __global__ void __launch_bounds__(kSumThreads, 2)
 }
 
 // x += alpha p ; p = r + beta p, all FP64, and q = p in the FP32 pair layout: one thread per slice
-// pair of a row, which is two FP64 vectors side by side and one FP32 vector
-__global__ void k_cg_xp_f64_pairs(CgStep cg, double2* __restrict__ x, double2* __restrict__ p,
-                                  const double2* __restrict__ r, float4* __restrict__ q, int64_t npair) {
+// pair of a row, which is two FP64 vectors side by side and one FP32 vector.  Bound by the FP64 pipe (8 FMAs
+// and 4 conversions a pair).  A grid-stride loop of up to four pairs a thread took 30.8 us at 12^4 x 8 and 178
+// at 16^4 x 16, one pair a thread 28.7 and 163.
+__global__ void k_cg_xp_f64_pairs(CgStep cg, double2* x, double2* p, const double2* r, float4* q, int64_t npair) {
   dep_wait();
   if (!cg.go()) return;
   const double alpha = cg.alpha, beta = cg.beta;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < npair; i += int64_t(gridDim.x) * blockDim.x) {
-    const double2 p0 = p[2 * i], p1 = p[2 * i + 1], x0 = x[2 * i], x1 = x[2 * i + 1];
-    const double2 r0 = __ldg(r + 2 * i), r1 = __ldg(r + 2 * i + 1);
-    x[2 * i] = make_double2(fma(alpha, p0.x, x0.x), fma(alpha, p0.y, x0.y));
-    x[2 * i + 1] = make_double2(fma(alpha, p1.x, x1.x), fma(alpha, p1.y, x1.y));
-    const double2 n0 = make_double2(fma(beta, p0.x, r0.x), fma(beta, p0.y, r0.y));
-    const double2 n1 = make_double2(fma(beta, p1.x, r1.x), fma(beta, p1.y, r1.y));
-    p[2 * i] = n0;
-    p[2 * i + 1] = n1;
-    if (q) q[i] = make_float4(float(n0.x), float(n1.x), float(n0.y), float(n1.y));
-  }
+  const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i >= npair) return;
+  const double2 p0 = p[2 * i], p1 = p[2 * i + 1], x0 = x[2 * i], x1 = x[2 * i + 1];
+  const double2 r0 = r[2 * i], r1 = r[2 * i + 1];
+  const double2 n0 = make_double2(fma(beta, p0.x, r0.x), fma(beta, p0.y, r0.y));
+  const double2 n1 = make_double2(fma(beta, p1.x, r1.x), fma(beta, p1.y, r1.y));
+  x[2 * i] = make_double2(fma(alpha, p0.x, x0.x), fma(alpha, p0.y, x0.y));
+  x[2 * i + 1] = make_double2(fma(alpha, p1.x, x1.x), fma(alpha, p1.y, x1.y));
+  p[2 * i] = n0;
+  p[2 * i + 1] = n1;
+  if (q) q[i] = make_float4(float(n0.x), float(n1.x), float(n0.y), float(n1.y));
 }
 
 bool flat_ok(const gbdw_field* f) { return f->prec != GBDW_F16 && f->LsP == f->LsE; }
@@ -654,7 +657,7 @@ int blas_cg_xp(double alpha, double beta, gbdw_field* x, gbdw_field* p, const gb
   if (x->prec == GBDW_F64 && p->prec == GBDW_F64 && r->prec == GBDW_F64 && L % 2 == 0 && x != p && x != r && p != r &&
       (!q || q->prec == GBDW_F32)) {
     const int64_t npair = ns * 12 * int64_t(L / 2);
-    launch_after(k_cg_xp_f64_pairs, unsigned(grid_flat(npair)), kThreads, 0,
+    launch_after(k_cg_xp_f64_pairs, unsigned((npair + kThreads - 1) / kThreads), kThreads, 0,
         cg, (double2*)x->d, (double2*)p->d, (const double2*)r->d, q ? (float4*)q->d : nullptr, npair);
     GBDW_LAUNCHED();
     return GBDW_OK;

@@ -64,7 +64,10 @@ size_t max_dynamic_smem();      // opt-in dynamic shared memory per CTA, minus r
 // before it on the stream still drains; its first statement is dep_wait(), which returns when that launch
 // is complete and its writes are visible (and at once in a kernel started the ordinary way).  dep_release()
 // lets the next such launch come up; it stands behind a kernel's dep_wait and behind its loads of anything
-// it writes, so no line that an SM's L1 keeps across a release can be stale.
+// it writes, so no line that an SM's L1 keeps across a release can be stale.  Such a kernel is resident while
+// the launch before it still writes, so its loads are ordinary ones: a read-only load (__ldg, ld.global.nc, a
+// pointer marked __restrict__) promises that nobody writes during the kernel's whole life, and the compiler may
+// move it above the wait.  Here dep_wait's memory clobber holds them back.
 // Hopping terms of 4^4 x 8 in a row 5.2 -> 2.7 us each; 16^4 x 16 57.5 -> 54; a Lanczos step's 38 launches at
 // 12^4 x 8 569 -> 482.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -205,7 +205,7 @@ namespace {
 // and with several CTAs the last one to finish adds the CTA sums.  One CTA per kSumShare partials: a
 // single CTA walked the 131072 partials of 32^4 x 16 in 43 us, the shares take 4.
 constexpr int kSumShare = 4096;
-__global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict__ partials, int64_t n, double* sums,
+__global__ void __launch_bounds__(1024) k_sum_partials(const double* partials, int64_t n, double* sums,
                                                        unsigned* counter, double* result, double num,
                                                        double* alpha_out, CgRule rule, double* host) {
   dep_wait();

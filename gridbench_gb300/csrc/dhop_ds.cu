@@ -135,7 +135,7 @@ __device__ __forceinline__ ds2 times(const Unit2& c, ds2 y) {
 
 // One leg, its direction and side known at run time (and the same for the whole CTA): spins 0 and 1
 // take c0 and c1 times spins A and B.
-__device__ __forceinline__ void ds_leg(const float4* __restrict__ u, const double2* __restrict__ in, int64_t row0,
+__device__ __forceinline__ void ds_leg(const float4* u, const double2* in, int64_t row0,
                                        int LsE, int leg, ds2 (&acc)[12]) {
   const int d = leg & 3, back = leg >> 2;
   const int spin_a = d < 2 ? 3 : 2, spin_b = d < 2 ? 2 : 3;
@@ -144,8 +144,8 @@ __device__ __forceinline__ void ds_leg(const float4* __restrict__ u, const doubl
   ds2 h0[3], h1[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    h0[c] = split2(__ldg(in + (row0 + c) * LsE)) + times(c0, split2(__ldg(in + (row0 + spin_a * 3 + c) * LsE)));
-    h1[c] = split2(__ldg(in + (row0 + 3 + c) * LsE)) + times(c1, split2(__ldg(in + (row0 + spin_b * 3 + c) * LsE)));
+    h0[c] = split2(in[(row0 + c) * LsE]) + times(c0, split2(in[(row0 + spin_a * 3 + c) * LsE]));
+    h1[c] = split2(in[(row0 + 3 + c) * LsE]) + times(c1, split2(in[(row0 + spin_b * 3 + c) * LsE]));
   }
   const Unit2 q0 = unit_of(k0 >= 2 ? k0 ^ 1 : k0), q1 = unit_of(k1 >= 2 ? k1 ^ 1 : k1);
 #pragma unroll
@@ -153,7 +153,7 @@ __device__ __forceinline__ void ds_leg(const float4* __restrict__ u, const doubl
     float2 s0 = make_float2(0.f, 0.f), e0 = s0, s1 = s0, e1 = s0;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const float4 a = __ldg(u + r * 3 + c);  // re h, re l, im h, im l
+      const float4 a = u[r * 3 + c];  // re h, re l, im h, im l
       const float2 rh = make_float2(a.x, a.x), rl = make_float2(a.y, a.y);
       const float2 ih = make_float2(-a.z, a.z), il = make_float2(-a.w, a.w);
       dot2(rh, rl, h0[c], s0, e0);
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(DS_THREADS, MINB) k_dhop_ds(const DhopParams p
 #pragma unroll 1
     for (int k = 0; k < 8; ++k) {
       const int leg = (k >> 1) + 4 * (k & 1);
-      ds_leg(u + 9 * leg, in, int64_t(__ldg(nb + leg)) * 12, p.LsE, DAG ? leg ^ 4 : leg, acc);
+      ds_leg(u + 9 * leg, in, int64_t(nb[leg]) * 12, p.LsE, DAG ? leg ^ 4 : leg, acc);
     }
     cpx<double> v[1][12];
 #pragma unroll

@@ -36,15 +36,15 @@ struct Arith<GBDW_F64> {
 template <int N>
 __device__ __forceinline__ void load_norms(const float* nrm, int64_t e, float (&v)[N]) {
   if constexpr (N == 1) {
-    v[0] = __ldg(nrm + e);
+    v[0] = nrm[e];
   } else if constexpr (N == 2) {
-    const float2 a = __ldg((const float2*)nrm + (e >> 1));
+    const float2 a = ((const float2*)nrm)[e >> 1];
     v[0] = a.x;
     v[1] = a.y;
   } else {
 #pragma unroll
     for (int k = 0; k < N / 4; ++k) {
-      const float4 a = __ldg((const float4*)nrm + (e >> 2) + k);
+      const float4 a = ((const float4*)nrm)[(e >> 2) + k];
       v[4 * k] = a.x;
       v[4 * k + 1] = a.y;
       v[4 * k + 2] = a.z;
@@ -97,12 +97,11 @@ struct LinkIO;
 template <>
 struct LinkIO<GBDW_F32> {
   static constexpr unsigned bytes = 72;
-  template <bool SMEM = false>
   static __device__ __forceinline__ void load(const void* U, size_t link, cpx<float> (&u)[3][3]) {
     const float2* p = (const float2*)U + link * 9;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-      const float2 a = ldv<SMEM>(p + k);
+      const float2 a = p[k];
       u[k / 3][k % 3] = {a.x, a.y};
     }
   }
@@ -110,12 +109,11 @@ struct LinkIO<GBDW_F32> {
 template <>
 struct LinkIO<GBDW_F64> {
   static constexpr unsigned bytes = 144;
-  template <bool SMEM = false>
   static __device__ __forceinline__ void load(const void* U, size_t link, cpx<double> (&u)[3][3]) {
     const double2* p = (const double2*)U + link * 9;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-      const double2 a = ldv<SMEM>(p + k);
+      const double2 a = p[k];
       u[k / 3][k % 3] = {a.x, a.y};
     }
   }
@@ -123,12 +121,11 @@ struct LinkIO<GBDW_F64> {
 template <>
 struct LinkIO<GBDW_F16> {
   static constexpr unsigned bytes = 24;
-  template <bool SMEM = false>
   static __device__ __forceinline__ void load(const void* U, size_t link, cpx<float> (&u)[3][3]) {
     const uint2* p = (const uint2*)U + link * 3;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const uint2 a = ldv<SMEM>(p + k);
+      const uint2 a = p[k];
       u[(2 * k) / 3][(2 * k) % 3] = h2c(a.x);
       u[(2 * k + 1) / 3][(2 * k + 1) % 3] = h2c(a.y);
     }
@@ -138,12 +135,11 @@ struct LinkIO<GBDW_F16> {
 template <>
 struct LinkIO<GBDW_BF16> {
   static constexpr unsigned bytes = 24;
-  template <bool SMEM = false>
   static __device__ __forceinline__ void load(const void* U, size_t link, cpx<float> (&u)[3][3]) {
     const uint2* p = (const uint2*)U + link * 3;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const uint2 a = ldv<SMEM>(p + k);
+      const uint2 a = p[k];
       u[(2 * k) / 3][(2 * k) % 3] = b2c(a.x);
       u[(2 * k + 1) / 3][(2 * k + 1) % 3] = b2c(a.y);
     }
@@ -240,11 +236,13 @@ struct MobLeg {
 // inside the site takes part with.  They are active or inactive together in every form that exchanges;
 // which other lanes of the warp stand at the same place is the compiler's business (__activemask() would ask).
 __device__ __forceinline__ unsigned site_lanes(int base, int G) { return (0xffffffffu >> (32 - G)) << base; }
+// WARP: every lane of the warp holds a slice pair, so that whole warps exchange
+template <bool WARP = false>
 __device__ __forceinline__ MobLeg make_mobleg(int Ls, double b, double c, double mf, int s0) {
   MobLeg m;
   m.G = Ls >> 1;
   const int lg = int(threadIdx.x) & (m.G - 1);
-  m.mask = site_lanes((int(threadIdx.x) & 31) - lg, m.G);
+  m.mask = WARP ? 0xffffffffu : site_lanes((int(threadIdx.x) & 31) - lg, m.G);
   m.from_lo = (lg + m.G - 1) & (m.G - 1);
   m.from_hi = (lg + 1) & (m.G - 1);
   m.b = float(b);
@@ -309,7 +307,7 @@ __device__ __forceinline__ void hop_leg_pairs(const cpx<float> (&u)[3][3], const
     // accumulated (FFMA2 in place of FADD2) instead of every projected component
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
-      const float2 nr = ldv<SMEM>(reinterpret_cast<const float2*>(nrm) + q);
+      const float2 nr = reinterpret_cast<const float2*>(nrm)[q];
       const float2 nn = neg2(nr);
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
@@ -360,7 +358,7 @@ __device__ __forceinline__ void hop_leg_scalar(const cpx<T> (&u)[3][3], const vo
   if constexpr (PIN == GBDW_F16) {
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      const float nr = ldv<SMEM>(nrm + j);
+      const float nr = nrm[j];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         h0[j][c].r *= nr;
@@ -596,8 +594,8 @@ __device__ __forceinline__ void dwf_epilogue(const DhopParams& p, int64_t site, 
         cen[j][k].r *= nc[j];
         cen[j][k].i *= nc[j];
       }
-    nlo *= __ldg(cnorm + site * Ls + slo);
-    nhi *= __ldg(cnorm + site * Ls + shi);
+    nlo *= cnorm[site * Ls + slo];
+    nhi *= cnorm[site * Ls + shi];
   }
   const T a5 = T(p.a5), kh = T(p.khop), c5 = T(p.c5);
 #pragma unroll
@@ -768,20 +766,25 @@ __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, i
     // FP32 rows are added exactly in two floats instead, and widened once.
     TR sr[N] = {}, si[N] = {};
     float hi = 0.f, lo = 0.f;
+    // rows are loaded six ahead of their stores, over which the compiler may not move a load
+    constexpr int B = 6;
+    cpx<TR> rv[12][N];
+#pragma unroll
+    for (int k = 0; k < B; ++k) Vec<RP, N>::load(p.r, site * 12 + k, s0, p.rLsP, rv[k]);
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
-      cpx<TR> rv[N];
-      Vec<RP, N>::load(p.r, site * 12 + k, s0, p.rLsP, rv);
+      if (k + B < 12) Vec<RP, N>::load(p.r, site * 12 + k + B, s0, p.rLsP, rv[k + B]);
       TR ks = TR(0);
 #pragma unroll
       for (int j = 0; j < N; ++j) {
-        rv[j].r -= al * TR(v[j][k].r);
-        rv[j].i -= al * TR(v[j][k].i);
+        cpx<TR>& x = rv[k][j];
+        x.r -= al * TR(v[j][k].r);
+        x.i -= al * TR(v[j][k].i);
         if constexpr (RP == GBDW_F64) {
-          sr[j] += rv[j].r * rv[j].r;
-          si[j] += rv[j].i * rv[j].i;
+          sr[j] += x.r * x.r;
+          si[j] += x.i * x.i;
         } else {
-          ks += rv[j].r * rv[j].r + rv[j].i * rv[j].i;
+          ks += x.r * x.r + x.i * x.i;
         }
       }
       if constexpr (RP == GBDW_F32) {
@@ -789,7 +792,7 @@ __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, i
         lo += (hi - (t - part_of)) + (ks - part_of);
         hi = t;
       }
-      Vec<RP, N>::store(p.r, site * 12 + k, s0, p.rLsP, rv);
+      Vec<RP, N>::store(p.r, site * 12 + k, s0, p.rLsP, rv[k]);
     }
     double s = double(hi) + double(lo);
     if constexpr (RP == GBDW_F64) {
@@ -817,7 +820,7 @@ __device__ __forceinline__ void dhop_thread(const DhopParams& p, unsigned site, 
   if constexpr (MOB) ml = make_mobleg(p.Ls, p.mb, p.mc, p.mf, s0);
 #define GBDW_LEG(L)                                                                                    \
   {                                                                                                    \
-    const int64_t n = __ldg(nb + L);                                                                   \
+    const int64_t n = nb[L];                                                                           \
     cpx<T> u[3][3];                                                                                    \
     LinkIO<GP>::load(p.U, size_t(site) * 8 + L, u);                                                    \
     hop_leg<PIN, DAG, N, L, false, MOB>(u, p.in, n * 12, s0, p.LsP, p.in_norm + n * p.LsE + s0, acc, &ml); \
@@ -934,7 +937,7 @@ __global__ void __launch_bounds__(256) k_dhop_general(const DhopParams p) {
   const int64_t Ls = p.Ls;
 #define GBDW_LEG(L)                                                                            \
   {                                                                                            \
-    const int64_t n5 = __ldg(nb + L);                                                          \
+    const int64_t n5 = nb[L];                                                                  \
     const int64_t ns = n5 / Ls;                                                                \
     const int sn = int(n5 - ns * Ls);                                                          \
     cpx<T> u[3][3];                                                                            \

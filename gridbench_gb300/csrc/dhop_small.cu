@@ -17,7 +17,7 @@ constexpr int SMALL_ITEMS = 32;
 template <int D, int DAG>
 __device__ __forceinline__ void small_direction(const DhopParams& p, unsigned site, int e0, cp2 (&acc)[12]) {
   const uint32_t* nb = p.nbr4 + size_t(site) * 8;
-  const uint32_t n0 = __ldg(nb + D), n1 = __ldg(nb + D + 4);
+  const uint32_t n0 = nb[D], n1 = nb[D + 4];
   cpx<float> u0[3][3], u1[3][3];
   RawSpinor x0, x1;
   const uint32_t row_bytes = uint32_t(p.LsP) * 8;

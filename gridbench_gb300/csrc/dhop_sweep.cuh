@@ -74,7 +74,7 @@ struct RawSpinor {
 __device__ __forceinline__ void sweep_issue(RawSpinor& w, const char* base, uint32_t stride) {
 #pragma unroll
   for (int r = 0; r < 12; ++r)
-    asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];"
+    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];"
                  : "=f"(w.v[r].r.x), "=f"(w.v[r].r.y), "=f"(w.v[r].i.x), "=f"(w.v[r].i.y)
                  : "l"(base + uint32_t(r) * stride));
 }
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
   auto x_outside = [&](int bd) { return int64_t(outside(x, bd, Lx)) * site_bytes; };
 
   MobLeg ml;
-  if constexpr (EPI == 6) ml = make_mobleg(p.Ls, p.mb, p.mc, p.mf, e0);
+  if constexpr (EPI == 6) ml = make_mobleg<SPW * G == 32>(p.Ls, p.mb, p.mc, p.mf, e0);
   cpx<float> u[3][3];
   RawSpinor ra, rb;
   Acc<GBDW_F32, 2> acc;

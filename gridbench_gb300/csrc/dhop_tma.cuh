@@ -71,8 +71,9 @@ struct ESz {
 
 // Shared memory: STAGES rings of NS neighbour blocks (+ norms), then the NS sites' links,
 // then STAGES+1 mbarriers (the last one for the links).
+// (M on FP32 pairs with two stages is kept at 128 registers, where 145 cost it a CTA: 16^4 x 16 78.3 -> 72.1 us)
 template <int PIN, int POUT, int GP, int DAG, int N, int EPI, int STAGES>
-__global__ void __launch_bounds__(256) k_dhop_tma(const DhopParams p, int NS) {
+__global__ void __launch_bounds__(256, PIN == GBDW_F32 && EPI == 1 && N == 2 && STAGES == 2 ? 2 : 0) k_dhop_tma(const DhopParams p, int NS) {
   dep_wait();
   using T = typename Arith<PIN>::T;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(256) k_dhop_tma(const DhopParams p, int NS) {
   uint32_t nb[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (tid < nvalid) {
     const uint4* q = reinterpret_cast<const uint4*>(p.nbr4 + (site0 + tid) * 8);
-    const uint4 a = __ldg(q), b = __ldg(q + 1);
+    const uint4 a = q[0], b = q[1];
     nb[0] = a.x; nb[1] = a.y; nb[2] = a.z; nb[3] = a.w;
     nb[4] = b.x; nb[5] = b.y; nb[6] = b.z; nb[7] = b.w;
   }
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(256) k_dhop_tma(const DhopParams p, int NS) {
       const unsigned char* base = smem + st * stage;                                                        \
       if (active) {                                                                                         \
         cpx<T> u[3][3];                                                                                     \
-        LinkIO<GP>::template load<true>(my_links, (L), u);                                                  \
+        LinkIO<GP>::load(my_links, (L), u);                                                  \
         hop_leg<PIN, DAG, N, L, true, EPI == 6>(u, base + sl * blk, 0, s0, LsP,                             \
                                       reinterpret_cast<const float*>(base + NS * blk + sl * nblk) + s0, acc, &ml); \
       }                                                                                                     \
@@ -239,7 +240,7 @@ __global__ void __launch_bounds__(256) k_dhop_tmaw(const DhopParams p_) {
     uint32_t nb[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (lane < nvalid) {
       const uint4* q = reinterpret_cast<const uint4*>(p.nbr4 + (site0 + lane) * 8);
-      const uint4 a = __ldg(q), b = __ldg(q + 1);
+      const uint4 a = q[0], b = q[1];
       nb[0] = a.x; nb[1] = a.y; nb[2] = a.z; nb[3] = a.w;
       nb[4] = b.x; nb[5] = b.y; nb[6] = b.z; nb[7] = b.w;
     }
@@ -271,7 +272,7 @@ __global__ void __launch_bounds__(256) k_dhop_tmaw(const DhopParams p_) {
       const unsigned char* base = wbase + st * stage;                                                      \
       if (active) {                                                                                        \
         cpx<T> u[3][3];                                                                                    \
-        LinkIO<GP>::template load<true>(my_links, (L), u);                                                 \
+        LinkIO<GP>::load(my_links, (L), u);                                                 \
         hop_leg<PIN, DAG, N, L, true, EPI == 6>(u, base + sl * blk, 0, s0, LsP,                            \
                                       reinterpret_cast<const float*>(base + NSW * blk + sl * nblk) + s0, acc, &ml); \
       }                                                                                                    \

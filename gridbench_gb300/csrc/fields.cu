@@ -284,8 +284,8 @@ __global__ void k_import_sites(const SRC* __restrict__ src, int64_t nsite, int L
 }
 
 template <class DST, int P, bool SINGLE>
-__global__ void k_export_sites(const void* __restrict__ srcd, const float* __restrict__ norm, int64_t nsite, int Ls,
-                               int LsE, int e0, DST* __restrict__ dst, int LsP) {
+__global__ void k_export_sites(const void* srcd, const float* norm, int64_t nsite, int Ls, int LsE, int e0, DST* dst,
+                               int LsP) {
   dep_wait();
   extern __shared__ __align__(16) unsigned char sm[];
   constexpr int TS = kTile<DST>, V = 16 / sizeof(DST);
@@ -295,7 +295,7 @@ __global__ void k_export_sites(const void* __restrict__ srcd, const float* __res
   DST* buf = reinterpret_cast<DST*>(sm) + size_t(warp) * TS * Ls;
   auto put = [&](int row, int s, float re, float im) {
     if constexpr (P == GBDW_F16) {
-      const float n = __ldg(norm + site * LsE + e0 + s);
+      const float n = norm[site * LsE + e0 + s];
       re *= n;
       im *= n;
     }
@@ -305,22 +305,31 @@ __global__ void k_export_sites(const void* __restrict__ srcd, const float* __res
   };
   if constexpr (P == GBDW_F64) {
     const double2* d = reinterpret_cast<const double2*>(srcd) + site * 12 * LsP;
-    for (int i = lane; i < 12 * Ls; i += 32) {
-      const int row = i / Ls, s = i - row * Ls;
-      const double2 a = __ldg(d + row * LsP + e0 + s);
-      DST* b = buf + s * TS + 2 * row;
-      b[0] = DST(a.x);
-      b[1] = DST(a.y);
+    for (int i0 = lane; i0 < 12 * Ls; i0 += 128) {  // four loads ahead of the first use
+      double2 a[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int i = i0 + 32 * j, row = i / Ls;
+        if (i < 12 * Ls) a[j] = d[row * LsP + e0 + i - row * Ls];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int i = i0 + 32 * j, row = i / Ls, s = i - row * Ls;
+        if (i >= 12 * Ls) break;
+        DST* b = buf + s * TS + 2 * row;
+        b[0] = DST(a[j].x);
+        b[1] = DST(a[j].y);
+      }
     }
   } else {
     auto group = [&](int row, int e) -> float4 {  // (Re, Re, Im, Im) of the stored pair of slice e
       const int64_t g = ((site * 12 + row) * LsP + e) >> 1;
       if constexpr (P == GBDW_F16) {
-        const uint2 h = __ldg(reinterpret_cast<const uint2*>(srcd) + g);
+        const uint2 h = reinterpret_cast<const uint2*>(srcd)[g];
         const float2 r = h2f(h.x), m = h2f(h.y);
         return make_float4(r.x, r.y, m.x, m.y);
       } else {
-        return __ldg(reinterpret_cast<const float4*>(srcd) + g);
+        return reinterpret_cast<const float4*>(srcd)[g];
       }
     };
     if constexpr (SINGLE) {

@@ -114,7 +114,7 @@ __device__ __forceinline__ void pack_face(const HaloParams& p, const HaloFace& F
     float n[N], m[N], sc[N];
     if constexpr (FROM) {
 #pragma unroll
-      for (int j = 0; j < N; ++j) n[j] = __ldg(p.in_norm + site * p.LsE + from(e0 + j));
+      for (int j = 0; j < N; ++j) n[j] = p.in_norm[site * p.LsE + from(e0 + j)];
     } else {
       load_norms<N>(p.in_norm, site * p.LsE + e0, n);
     }

@@ -28,12 +28,6 @@ struct cp2 {
   float2 r, i;
 };
 
-template <bool SMEM, class V>
-__device__ __forceinline__ V ldv(const V* p) {
-  if constexpr (SMEM) return *p;
-  else return __ldg(p);
-}
-
 __device__ __forceinline__ float2 h2f(unsigned w) {
   __half2 h = *reinterpret_cast<__half2*>(&w);
   return __half22float2(h);
@@ -48,9 +42,8 @@ template <int P>
 struct Elem;
 template <>
 struct Elem<GBDW_F64> {
-  template <bool SMEM = false>
   __device__ static cpx<double> ld(const void* b, int64_t row, int e, int LsP) {
-    const double2 a = ldv<SMEM>((const double2*)b + row * LsP + e);
+    const double2 a = ((const double2*)b)[row * LsP + e];
     return {a.x, a.y};
   }
   __device__ static void st(void* b, int64_t row, int e, int LsP, double re, double im) {
@@ -59,10 +52,9 @@ struct Elem<GBDW_F64> {
 };
 template <>
 struct Elem<GBDW_F32> {
-  template <bool SMEM = false>
   __device__ static cpx<float> ld(const void* b, int64_t row, int e, int LsP) {
     const float* f = (const float*)b + re_index(row, e, LsP);
-    return {ldv<SMEM>(f), ldv<SMEM>(f + 2)};
+    return {f[0], f[2]};
   }
   __device__ static void st(void* b, int64_t row, int e, int LsP, float re, float im) {
     float* f = (float*)b + re_index(row, e, LsP);
@@ -73,10 +65,9 @@ struct Elem<GBDW_F32> {
 // F16: returns / takes the stored (norm-scaled) values.
 template <>
 struct Elem<GBDW_F16> {
-  template <bool SMEM = false>
   __device__ static cpx<float> ld(const void* b, int64_t row, int e, int LsP) {
     const unsigned short* h = (const unsigned short*)b + re_index(row, e, LsP);
-    const unsigned short a = ldv<SMEM>(h), c = ldv<SMEM>(h + 2);
+    const unsigned short a = h[0], c = h[2];
     return {__half2float(__ushort_as_half(a)), __half2float(__ushort_as_half(c))};
   }
   __device__ static void st(void* b, int64_t row, int e, int LsP, float re, float im) {
@@ -95,7 +86,7 @@ struct Vec {
   __device__ static void load(const void* b, int64_t row, int e0, int LsP, cpx<T> (&v)[N]) {
     if constexpr (P == GBDW_F64 || N == 1) {
 #pragma unroll
-      for (int j = 0; j < N; ++j) v[j] = Elem<P>::template ld<SMEM>(b, row, e0 + j, LsP);
+      for (int j = 0; j < N; ++j) v[j] = Elem<P>::ld(b, row, e0 + j, LsP);
     } else {
       cp2 q[N / 2];
       load_pairs(b, row, e0, LsP, q);
@@ -111,7 +102,7 @@ struct Vec {
   // the line is in L1, the wider access costs more (M at 16^4 x 16 in form 3: 64.3 -> 66.6 us).
   __device__ static cpx<T> one(const void* b, int64_t row, int e, int second, int LsP) {
     if constexpr (P == GBDW_F64 || N == 1 || !SMEM) {
-      return Elem<P>::template ld<SMEM>(b, row, e, LsP);
+      return Elem<P>::ld(b, row, e, LsP);
     } else {
       cp2 q[1];
       Vec<P, 2, SMEM>::load_pairs(b, row, e - second, LsP, q);
@@ -124,14 +115,14 @@ struct Vec {
       const float4* f = reinterpret_cast<const float4*>((const float*)b + row * 2 * int64_t(LsP) + 2 * e0);
 #pragma unroll
       for (int k = 0; k < N / 2; ++k) {
-        const float4 a = ldv<SMEM>(f + k);
+        const float4 a = f[k];
         q[k] = {make_float2(a.x, a.y), make_float2(a.z, a.w)};
       }
     } else if constexpr (P == GBDW_F16) {
       const uint2* h = reinterpret_cast<const uint2*>((const unsigned short*)b + row * 2 * int64_t(LsP) + 2 * e0);
 #pragma unroll
       for (int k = 0; k < N / 2; ++k) {
-        const uint2 a = ldv<SMEM>(h + k);
+        const uint2 a = h[k];
         q[k] = {h2f(a.x), h2f(a.y)};
       }
     }
@@ -140,7 +131,7 @@ struct Vec {
   __device__ static void load_pairs_raw(const void* b, int64_t row, int e0, int LsP, uint2 (&q)[N / 2]) {
     const uint2* h = reinterpret_cast<const uint2*>((const unsigned short*)b + row * 2 * int64_t(LsP) + 2 * e0);
 #pragma unroll
-    for (int k = 0; k < N / 2; ++k) q[k] = ldv<SMEM>(h + k);
+    for (int k = 0; k < N / 2; ++k) q[k] = h[k];
   }
   // F64 / F32 stores
   __device__ static void store(void* b, int64_t row, int e0, int LsP, const cpx<T> (&v)[N]) {

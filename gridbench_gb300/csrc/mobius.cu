@@ -97,7 +97,7 @@ __device__ __forceinline__ void apply5(const Coef5& c, const void* v, const floa
     for (int j = 0; j < N; ++j)
 #pragma unroll
       for (int k = 0; k < 12; ++k) cen[j][k] = {cen[j][k].r * nc[j], cen[j][k].i * nc[j]};
-    const float nl = __ldg(vn + site * Ls + slo), nh = __ldg(vn + site * Ls + shi);
+    const float nl = vn[site * Ls + slo], nh = vn[site * Ls + shi];
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
       lo[k] = {lo[k].r * nl, lo[k].i * nl};
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(192) k_m5d_inv(const __grid_constant__ M5DInvP
       auto x = [&](int t) -> cpx<T> {
         cpx<T> e = Elem<P>::ld(p.in, r, t, p.LsP);
         if constexpr (P == GBDW_F16) {
-          const float n = __ldg(p.in_norm + site * Ls + t);
+          const float n = p.in_norm[site * Ls + t];
           e = {e.r * n, e.i * n};
         }
         return e;
@@ -299,7 +299,9 @@ int m5d(gbdw_field* out, const gbdw_field* x, const Coef5& a, const gbdw_field* 
   p.LsP = x->LsP;
   p.a = a;
   if (b) p.b = *b;
-  const bool pair = Ls % 2 == 0;
+  // pairs share their inner neighbours; an FP64 pair with all its rows loaded ahead of the stores would take
+  // 168 registers (254 with two operands) and is slower than single slices: 16^4 x 16 97.8 us against 95.0
+  const bool pair = Ls % 2 == 0 && x->prec != GBDW_F64;
   const int64_t n = p.nsite * (pair ? Ls / 2 : Ls);
   const unsigned g = nblk(n, 128);
 #define GBDW_M5D_N(P, N)                                                          \
@@ -317,7 +319,7 @@ int m5d(gbdw_field* out, const gbdw_field* x, const Coef5& a, const gbdw_field* 
     GBDW_M5D_N(P, 1)     \
   }
   if (x->prec == GBDW_F64) {
-    GBDW_M5D(GBDW_F64)
+    GBDW_M5D_N(GBDW_F64, 1)
   } else if (x->prec == GBDW_F32) {
     GBDW_M5D(GBDW_F32)
   } else {
