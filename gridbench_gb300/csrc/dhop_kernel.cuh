@@ -670,9 +670,9 @@ __device__ __forceinline__ void mobius_adj_hop(const DhopParams& p, int s0, cpx<
 // work of the other warps, in place of a pass of its own (k_m5inv).  Hopping term and D5^-1, us: FP16 on half
 // of 16^4 x 16 27.5 + 15.8 -> 30.6, FP32 on half of 16^3 x 32 x 12 58.6 + 33.2 -> 73.
 template <int DAG>
-__device__ __forceinline__ void m5inv_lanes(const DhopParams& p, int s0, cpx<float> (&v)[2][12]) {
+__device__ __forceinline__ void m5inv_lanes(const DhopParams& p, int s0, cpx<float> (&v)[2][12], unsigned lanes) {
   const int G = p.LsE >> 1, lg = s0 >> 1, base = int(threadIdx.x & 31) - lg;
-  const unsigned mask = site_lanes(base, G);
+  const unsigned mask = lanes ? lanes : site_lanes(base, G);
   const float ia = float(p.mb), g = float(p.mc), wall = float(-p.mf);
 #pragma unroll
   for (int ch = 0; ch < 2; ++ch) {
@@ -732,15 +732,16 @@ __device__ __forceinline__ void m5inv_lanes(const DhopParams& p, int s0, cpx<flo
 // EPI 0: store Dhop(in); EPI 1: store M(in); EPI 2 / 3 / 4: r -= alpha M(in) with r FP32 / FP64 /
 // FP16 (the CG residual update fused into the operator's second pass; M(in) is not stored);
 // EPI 5: store D5^-1 Dhop(in) (DAG: D5^-dag DhopDag(in)); EPI 6: store the Mobius M(in), A(b, c) applied to the neighbours as they are loaded.
+// lanes: the lanes of the warp that are here together, if the form knows them (0: the site's).
 // Returns |what was stored|^2 in part (FP32 outputs) or dpart (FP64 outputs and EPI 2-4).
 template <int PIN, int POUT, int DAG, int N, int EPI, bool SMEM = false, class T>
 __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, int s0, int LsE, int LsP,
                                             cpx<T> (&v)[N][12], float& part, double& dpart,
-                                            const void* rows = nullptr) {
+                                            const void* rows = nullptr, unsigned lanes = 0) {
   if constexpr (EPI == 1 && DAG == 1 && N == 2) {
     if (p.mob) mobius_adj_hop(p, s0, v);
   }
-  if constexpr (EPI == 5) m5inv_lanes<DAG>(p, s0, v);
+  if constexpr (EPI == 5) m5inv_lanes<DAG>(p, s0, v, lanes);
   else if constexpr (EPI >= 1) dwf_epilogue<PIN, DAG, N, SMEM>(p, site, s0, v, rows);
   if constexpr (EPI == 4) {
     // FP16 r: dequantise with its per-slice norms, update in FP32, store with new norms

@@ -149,6 +149,7 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
   const int z = int(b % q.nbz) * 2 + zl;
   const int ta = int(b / q.nbz) * q.nt, tb = min(ta + q.nt, Lt);
   const bool active = lane < SPW * G;  // whole warps are launched
+  constexpr unsigned lanes = 0xffffffffu >> (32 - SPW * G);  // the active ones, in every warp
   const int col = active ? x + Lx * (y + Ly * z) : 0;
   const int e0 = tile * TE + 2 * lg;
   const char* const gcol = reinterpret_cast<const char*>(p.in) + int64_t(e0) * 8 + col * site_bytes;
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
       if (!EO && EPI >= 1 && !p.cen)  // the diagonal part reads this site's plane t, in shared memory
         finish_site<GBDW_F32, GBDW_F32, DAG, 2, EPI, !EO && EPI >= 1>(p, site, e0, p.LsE, p.LsP, v, pt, dt, sc - lg * 16);
       else
-        finish_site<GBDW_F32, GBDW_F32, DAG, 2, EPI>(p, site, e0, p.LsE, p.LsP, v, pt, dt);
+        finish_site<GBDW_F32, GBDW_F32, DAG, 2, EPI>(p, site, e0, p.LsE, p.LsP, v, pt, dt, nullptr, lanes);
       part += pt;
       dpart += dt;
     }
