@@ -155,7 +155,6 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
   const char* const gcol = reinterpret_cast<const char*>(p.in) + int64_t(e0) * 8 + col * site_bytes;
   char* const own = sw_smem + sl * SS + lg * 16;            // this thread's rows in plane slot 0
   char* const ulk = sw_smem + 2 * NS * SS + sl * SWEEP_LS;  // its site's links in buffer 0
-  float part = 0.f;
   double dpart = 0.0;
   const float fl = DAG ? -1.f : 1.f;
   auto fetch_plane = [&](int t, int slot) {
@@ -249,8 +248,8 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
         finish_site<GBDW_F32, GBDW_F32, DAG, 2, EPI, !EO && EPI >= 1>(p, site, e0, p.LsE, p.LsP, v, pt, dt, sc - lg * 16);
       else
         finish_site<GBDW_F32, GBDW_F32, DAG, 2, EPI>(p, site, e0, p.LsE, p.LsP, v, pt, dt, nullptr, lanes);
-      part += pt;
-      dpart += dt;
+      // |M in|^2 is FP64 above one site's 48 squares, as in the other forms, however far this walk goes
+      if (p.partials) dpart += (EPI >= 2 && EPI <= 4) ? dt : double(pt);
     }
     if (!more) break;
     cp_async_wait<0>();
@@ -269,7 +268,7 @@ __global__ void __launch_bounds__((4 * TE + 31) / 32 * 32, 256 / ((4 * TE + 31) 
   }
   cp_async_wait<0>();
   if (p.partials) {
-    double v[1] = {(EPI >= 2 && EPI <= 4) ? dpart : double(part)};
+    double v[1] = {dpart};
     block_partial<1>(v, p.partials);
   }
 }
