@@ -729,6 +729,14 @@ __device__ __forceinline__ void m5inv_lanes(const DhopParams& p, int s0, cpx<flo
 }
 
 // ------------------------------------------------------------------ per-site finish
+// s += x, and what s could not hold of it (Knuth's two-sum)
+__device__ __forceinline__ float add_into(float& s, float x) {
+  const float t = s + x, part_of = t - s;
+  const float rest = (s - (t - part_of)) + (x - part_of);
+  s = t;
+  return rest;
+}
+
 // EPI 0: store Dhop(in); EPI 1: store M(in); EPI 2 / 3 / 4: r -= alpha M(in) with r FP32 / FP64 /
 // FP16 (the CG residual update fused into the operator's second pass; M(in) is not stored);
 // EPI 5: store D5^-1 Dhop(in) (DAG: D5^-dag DhopDag(in)); EPI 6: store the Mobius M(in), A(b, c) applied to the neighbours as they are loaded.
@@ -764,11 +772,13 @@ __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, i
     const TR al = TR(*p.alpha);
     // The FP64 pipe takes some 90 clocks a warp instruction and scheduler, and an FP64 r costs it one FMA a
     // component for the update and one for the sum; each component of the slices keeps a sum of its own.
-    // FP32 rows are added exactly in two floats instead, and widened once.
+    // An FP32 r's rows are added in three floats, which hold their sum to 2^-65 where FP64 adds would to 2^-49,
+    // and widened once (twelve FP64 adds and conversions a thread: a mixed FP32 solve at 16^4 x 16 16.2 -> 17.4 ms).
     TR sr[N] = {}, si[N] = {};
-    float hi = 0.f, lo = 0.f;
-    // rows are loaded six ahead of their stores, over which the compiler may not move a load
-    constexpr int B = 6;
+    float hi = 0.f, lo = 0.f, least = 0.f;
+    // Rows are loaded ahead of their stores, over which the compiler may not move a load: all of an FP32 r (six:
+    // M^dag with the update at 16^4 x 16 86 us in place of 78), six of an FP64 r.
+    constexpr int B = RP == GBDW_F32 ? 12 : 6;
     cpx<TR> rv[12][N];
 #pragma unroll
     for (int k = 0; k < B; ++k) Vec<RP, N>::load(p.r, site * 12 + k, s0, p.rLsP, rv[k]);
@@ -788,14 +798,10 @@ __device__ __forceinline__ void finish_site(const DhopParams& p, int64_t site, i
           ks += x.r * x.r + x.i * x.i;
         }
       }
-      if constexpr (RP == GBDW_F32) {
-        const float t = hi + ks, part_of = t - hi;
-        lo += (hi - (t - part_of)) + (ks - part_of);
-        hi = t;
-      }
+      if constexpr (RP == GBDW_F32) least += add_into(lo, add_into(hi, ks));
       Vec<RP, N>::store(p.r, site * 12 + k, s0, p.rLsP, rv[k]);
     }
-    double s = double(hi) + double(lo);
+    double s = double(hi) + (double(lo) + double(least));
     if constexpr (RP == GBDW_F64) {
       s = sr[0] + si[0];
 #pragma unroll
