@@ -195,10 +195,10 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
   // and no Shamir epilogue: it runs on the hopping term's shape
   const int key_epi = (p.mob && epi == 6) ? 0 : tune_epi;  // (tune_epi is 0 for D5^-1 after the hopping term)
   DhopLaunch L;
-  bool tuned = find_tuned_launch(g->prec, in->prec, in->LsE, key_epi, &L);
+  bool tuned = find_tuned_launch(g->prec, in->prec, in->LsE, key_epi, g->lat->nsite, &L);
   if (!tuned) L = untuned_launch(g, in, epi);
-  if (g->lat->parity >= 0) tuned |= find_tuned_launch(g->prec, in->prec, in->LsE, key_epi + EO_KEY, &L);
-  if (ex && ex->tune_key >= 0) tuned |= find_tuned_launch(g->prec, in->prec, in->LsE, ex->tune_key, &L);
+  if (g->lat->parity >= 0) tuned |= find_tuned_launch(g->prec, in->prec, in->LsE, key_epi + EO_KEY, g->lat->nsite, &L);
+  if (ex && ex->tune_key >= 0) tuned |= find_tuned_launch(g->prec, in->prec, in->LsE, ex->tune_key, g->lat->nsite, &L);
   if (epi == 5) L = m5inv_launch(L);
   if (p.mob) L.spt = 2;  // the fused adjoint works on slice pairs, one site's pairs in consecutive lanes
   if (p.mob && (in->lat->Ls & (in->lat->Ls - 1))) L = DhopLaunch{64, 2, 2, 2};  // whole sites in a warp
@@ -260,7 +260,7 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
     // tuned register cap and t-brick order
     if (int s2 = ds_links(g, &p.U)) return s2;
     DhopLaunch D{DS_THREADS, 1, 0, 4};  // stages: register cap as CTAs per SM
-    find_tuned_launch(g->prec, in->prec, in->LsE, tune_epi + DS_KEY, &D);
+    find_tuned_launch(g->prec, in->prec, in->LsE, tune_epi + DS_KEY, g->lat->nsite, &D);
     p.TE = 0;
     p.brick = brick_extent(g->lat, DhopLaunch{DS_THREADS, 1, 0, 4, 1, D.brick});
     const int64_t blocks_ds = (p.nsite * p.LsE + DS_THREADS - 1) / DS_THREADS;

@@ -970,6 +970,7 @@ struct DhopLaunch {
   int stages = 4;  // staged kernels: depth of the leg ring
   int split = 1;   // forms 0 and 3: each site's Ls*nrhs slices cut into this many tiles
   int brick = 1;   // forms 0 and 3 on periodic lattices: t-brick sweep order (1: natural order)
+  int64_t sites = 0;  // 4D sites of the lattice the tuner chose it on; 0: pinned, for every lattice
 };
 
 // The t-sweep form's geometry (dhop_sweep.cuh).

@@ -96,11 +96,15 @@ DhopLaunch untuned_launch(const gbdw_gauge* g, const gbdw_field* in, int epi) {
   return DhopLaunch{64, 2, 3};
 }
 
-bool find_tuned_launch(int gprec, int sprec, int LsE, int epi, DhopLaunch* L) {
+// Tuned at 16^4 x 8, the sweep took 14.0 us a hopping term on 8^4 x 8 and 10.8 on 6^4 x 8, where the rules by size
+// take 5.4 and 3.5.  Other forms hold their own on other volumes (rings tuned at 16^4 x 20: 8.1 on 8^4, rules 7.3).
+bool find_tuned_launch(int gprec, int sprec, int LsE, int epi, int64_t sites, DhopLaunch* L) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   auto it = g_tuned.find(key_of(gprec, sprec, LsE, epi));
   if (it == g_tuned.end()) return false;
-  *L = it->second;
+  const DhopLaunch& T = it->second;
+  if (T.mode == 4 && sprec == GBDW_F32 && T.sites && T.sites != sites) return false;
+  *L = T;
   return true;
 }
 
@@ -121,14 +125,15 @@ std::vector<int> cg_residual_precs(int gprec, int sprec) {
 // entry if one exists)
 DhopLaunch lookup(const gbdw_gauge* g, const gbdw_field* in, int epi) {
   DhopLaunch L;
-  if (!find_tuned_launch(g->prec, in->prec, in->LsE, epi, &L)) L = untuned_launch(g, in, epi);
-  if (g->lat->parity >= 0) find_tuned_launch(g->prec, in->prec, in->LsE, epi + EO_KEY, &L);
+  if (!find_tuned_launch(g->prec, in->prec, in->LsE, epi, g->lat->nsite, &L)) L = untuned_launch(g, in, epi);
+  if (g->lat->parity >= 0) find_tuned_launch(g->prec, in->prec, in->LsE, epi + EO_KEY, g->lat->nsite, &L);
   return L;
 }
 
-// a pinned shape applies to the hopping term and, with one right-hand side, to M and the CG steps
-// (on a half-lattice gauge field: to the even-odd hopping term and its Schur epilogue)
-void pin_launch(const gbdw_gauge* g, const gbdw_field* in, const DhopLaunch& L) {
+// a pinned shape applies, on every lattice, to the hopping term and, with one right-hand side, to M and the CG
+// steps (on a half-lattice gauge field: to the even-odd hopping term and its Schur epilogue)
+void pin_launch(const gbdw_gauge* g, const gbdw_field* in, DhopLaunch L) {
+  L.sites = 0;
   const int ko = g->lat->parity >= 0 ? EO_KEY : 0;
   set_tuned_launch(g->prec, in->prec, in->LsE, ko, L);
   if (in->nrhs != 1) return;
@@ -145,8 +150,8 @@ DhopLaunch pin_base(const gbdw_gauge* g, const gbdw_field* in, const TAKES& take
   const int ko = g->lat->parity >= 0 ? EO_KEY : 0;
   DhopLaunch L;
   const DhopLaunch now = lookup(g, in, 0);
-  if (find_tuned_launch(g->prec, in->prec, in->LsE, 0, &L) || find_tuned_launch(g->prec, in->prec, in->LsE, ko, &L))
-    return now;
+  for (int key : {0, ko})
+    if (find_tuned_launch(g->prec, in->prec, in->LsE, key, g->lat->nsite, &L)) return now;
   L = now.mode == 0 || now.mode == 3 ? now : DhopLaunch{64, 2, 3};
   if (takes(L)) return L;
   const int spt = in->prec == GBDW_F64 || in->LsE % 2 ? 1 : in->prec == GBDW_F16 && in->LsE % 4 == 0 ? 4 : 2;
@@ -237,7 +242,7 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
     }
   }
   DhopLaunch saved = lookup(g, in, 0);
-  if (eo) find_tuned_launch(g->prec, in->prec, in->LsE, ko, &saved);
+  if (eo) find_tuned_launch(g->prec, in->prec, in->LsE, ko, g->lat->nsite, &saved);
   DhopLaunch best = saved, best_m = saved;
   float best_ms = 1e30f, best_m_ms = 1e30f;
   int status = GBDW_OK;
@@ -263,7 +268,7 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
   // M (one right-hand side) is timed over the same shapes on its own: its epilogue reads the
   // centre site and its 5th-dimension neighbours besides the hopping term's gather.
   DhopLaunch saved_m = lookup(g, in, 1);
-  if (eo) find_tuned_launch(g->prec, in->prec, in->LsE, 1 + ko, &saved_m);
+  if (eo) find_tuned_launch(g->prec, in->prec, in->LsE, 1 + ko, g->lat->nsite, &saved_m);
   std::vector<std::pair<float, DhopLaunch>> m_times;
   for (const DhopLaunch& L : cands) {
     float ms = 0.f;
@@ -280,9 +285,14 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
       best_m = L;
     }
   }
+  // what it chose holds a t-sweep's volume; while it times, a candidate holds everywhere
+  auto chosen = [&](DhopLaunch L) {
+    L.sites = g->lat->nsite;
+    return L;
+  };
   if (!ds_only) {
-    set_tuned_launch(g->prec, in->prec, in->LsE, ko, status ? saved : best);
-    if (in->nrhs == 1) set_tuned_launch(g->prec, in->prec, in->LsE, 1 + ko, status ? saved_m : best_m);
+    set_tuned_launch(g->prec, in->prec, in->LsE, ko, status ? saved : chosen(best));
+    if (in->nrhs == 1) set_tuned_launch(g->prec, in->prec, in->LsE, 1 + ko, status ? saved_m : chosen(best_m));
   }
   // FP64 fields: the double-single form's register cap (three or four CTAs per SM) and t-brick
   // order, for Dhop and M, timed with that form forced
@@ -360,7 +370,7 @@ int gbdw_tune_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, i
           best_cg = L;
         }
       }
-      set_tuned_launch(g->prec, in->prec, in->LsE, key, status ? best_m : best_cg);
+      set_tuned_launch(g->prec, in->prec, in->LsE, key, chosen(status ? best_m : best_cg));
       gbdw_field_destroy(r);
       if (status) break;
     }
@@ -391,7 +401,7 @@ int gbdw_tune_query_m(const gbdw_gauge* g, const gbdw_field* in, int cfg[6]) {
 int gbdw_tune_query_cg(const gbdw_gauge* g, const gbdw_field* in, int rprec, int cfg[6]) {
   if (!g || !in || !cfg || rprec < GBDW_F64 || rprec > GBDW_F16) return GBDW_ERR_INVALID;
   DhopLaunch L = lookup(g, in, 1);
-  if (g->lat->parity < 0) find_tuned_launch(g->prec, in->prec, in->LsE, cg_step_key(rprec), &L);
+  if (g->lat->parity < 0) find_tuned_launch(g->prec, in->prec, in->LsE, cg_step_key(rprec), g->lat->nsite, &L);
   const int v[6] = {L.threads, L.spt, L.mode, L.stages, L.split, L.brick};
   for (int i = 0; i < 6; ++i) cfg[i] = v[i];
   return GBDW_OK;
@@ -400,7 +410,7 @@ int gbdw_tune_query_cg(const gbdw_gauge* g, const gbdw_field* in, int rprec, int
 int gbdw_tune_query_ds(const gbdw_gauge* g, const gbdw_field* in, int epi, int cfg[2]) {
   if (!g || !in || !cfg || epi < 0 || epi > 1) return GBDW_ERR_INVALID;
   DhopLaunch L{DS_THREADS, 1, 0, 4};
-  find_tuned_launch(g->prec, in->prec, in->LsE, epi + DS_KEY, &L);
+  find_tuned_launch(g->prec, in->prec, in->LsE, epi + DS_KEY, g->lat->nsite, &L);
   cfg[0] = L.stages;
   cfg[1] = L.brick;
   return GBDW_OK;
@@ -512,8 +522,10 @@ int gbdw_tune_save(const char* path) {
   std::map<std::string, DhopLaunch> text;  // in the order of the keys' text
   for (auto& kv : g_tuned) text[key_text(kv.first)] = kv.second;
   for (auto& kv : text) {
-    fprintf(f, "%s\n  \"%s\": [%d, %d, %d, %d, %d, %d]", first ? "" : ",", kv.first.c_str(), kv.second.threads,
+    fprintf(f, "%s\n  \"%s\": [%d, %d, %d, %d, %d, %d", first ? "" : ",", kv.first.c_str(), kv.second.threads,
             kv.second.spt, kv.second.mode, kv.second.stages, kv.second.split, kv.second.brick);
+    if (kv.second.sites) fprintf(f, ", %lld", (long long)kv.second.sites);
+    fprintf(f, "]");
     first = false;
   }
   fprintf(f, "\n}\n");
@@ -534,7 +546,8 @@ int gbdw_tune_load(const char* path) {
   while ((n = fread(buf, 1, sizeof buf, f)) > 0) text.append(buf, n);
   fclose(f);
   // Entries look like "g1_s1_L16_e0": [128, 2, 0, 4, 1, 1] (threads, slices per thread, form,
-  // stages, tile split, t-brick; shorter entries keep the defaults of the missing numbers)
+  // stages, tile split, t-brick and, for a tuned shape, the sites of its lattice; shorter entries keep the
+  // defaults of the missing numbers)
   size_t pos = 0;
   int loaded = 0;
   while ((pos = text.find('"', pos)) != std::string::npos) {
@@ -542,15 +555,17 @@ int gbdw_tune_load(const char* path) {
     if (end == std::string::npos) break;
     const std::string key = text.substr(pos + 1, end - pos - 1);
     int gp, sp, LsE, epi, th, spt, mode = 0, stages = 4, split = 1, brick = 1;
+    long long sites = 0;
     const size_t lb = text.find('[', end);
     if (lb == std::string::npos) break;
     if (sscanf(key.c_str(), "g%d_s%d_L%d_e%d", &gp, &sp, &LsE, &epi) == 4 &&
-        sscanf(text.c_str() + lb, "[%d , %d , %d , %d , %d , %d]", &th, &spt, &mode, &stages, &split, &brick) >= 2 &&
+        sscanf(text.c_str() + lb, "[%d , %d , %d , %d , %d , %d , %lld]", &th, &spt, &mode, &stages, &split, &brick,
+               &sites) >= 2 &&
         th > 0 && th <= 256 && th % 32 == 0 && (spt == 1 || spt == 2 || spt == 4) && mode >= 0 && mode <= 4 &&
         // the double-single keys hold their register cap (CTAs per SM, 3 or 4) in `stages`
         (stages == 2 || stages == 4 || (epi >= DS_KEY && stages == 3)) && split >= 1 && split <= 64 && brick >= 1 &&
-        brick <= 64) {
-      set_tuned_launch(gp, sp, LsE, epi, DhopLaunch{th, spt, mode, stages, split, brick});
+        brick <= 64 && sites >= 0) {
+      set_tuned_launch(gp, sp, LsE, epi, DhopLaunch{th, spt, mode, stages, split, brick, sites});
       ++loaded;
     }
     pos = text.find(']', lb);

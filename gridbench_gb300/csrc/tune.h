@@ -31,7 +31,8 @@ constexpr int EO_KEY = 32;
 // tune-cache key of the fused CG step (both passes of mdagm_residual) with a residual of precision rprec
 inline int cg_step_key(int rprec) { return 16 + rprec; }
 // the cached shape for the key, if one was tuned or pinned
-bool find_tuned_launch(int gprec, int sprec, int LsE, int epi, DhopLaunch* L);
+// (a t-sweep that was timed on a lattice of another volume is none: its slices of t fill other waves)
+bool find_tuned_launch(int gprec, int sprec, int LsE, int epi, int64_t sites, DhopLaunch* L);
 // cen / khop: the M epilogue's diagonal field (default: in) and hopping coefficient (1/2)
 int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag, int epi, double a5, double mf,
              double* norm2, bool fetch = true, const gbdw_field* cen = nullptr, double khop = 0.5,
