@@ -4,8 +4,8 @@
 //
 // Work decomposition.  A thread owns `spt` consecutive innermost slices (e = rhs*Ls + s)
 // of one site; the slices of a site are cut into `split` contiguous tiles of TE = LsE/split
-// slices, so a tile holds whole right-hand sides (an RHS tile) or part of one's slices (an Ls tile)
-// where the cuts allow it.  Threads are ordered (tile,
+// slices, so a tile holds whole right-hand sides (an RHS tile) or a whole part of one's slices (an Ls
+// tile): batch_tile.h.  Threads are ordered (tile,
 // site, slice group), and an instance's threads are cut into work items of one warp each.  The
 // link of a (site, leg) is loaded once per thread group and reused over its tile's slices;
 // more tiles put more sites in a CTA.
@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "batch_tile.h"
 #include "common.cuh"
 #include "dhop_kernel.cuh"
 
@@ -178,18 +179,6 @@ void launch(const gbdw_batch* b, cudaStream_t s) {
     k_batch<DAG, 128, 3><<<b->grid, 128, 0, s>>>(b->d_inst, b->d_item_inst, b->d_begin, b->total, b->d_next);
 }
 
-// Tile of an instance for the batch's split: the largest split <= the batch's that cuts the
-// extent into whole slice groups and whose tile is whole values of s (a multiple of nrhs) or
-// whole sets of right-hand sides at one s (a divisor of nrhs).
-int tile_of(int LsE, int nrhs, int spt, int split) {
-  for (int sp = split; sp > 1; sp >>= 1) {
-    if (LsE % sp) continue;
-    const int TE = LsE / sp;
-    if (TE % spt == 0 && (TE % nrhs == 0 || nrhs % TE == 0)) return TE;
-  }
-  return LsE;
-}
-
 // Builds the work list for the current shape and captures [reset counter, persistent kernel].
 int build(gbdw_batch* b) {
   release_graph(b);
@@ -214,7 +203,7 @@ int build(gbdw_batch* b) {
     int spt = (I.kind == 0) ? b->spt32 : b->spt16;
     if (x->LsE % spt != 0) spt = 1;
     I.spt = spt;
-    I.TE = tile_of(x->LsE, x->nrhs, spt, b->split);
+    I.TE = batch_tile(x->LsE, g->lat->Ls, spt, b->split);
     const int L = x->LsE;
     I.lsp = (spt == 2 && L == x->LsP &&
              (L == 8 || L == 12 || L == 16 || L == 24 || L == 32 || L == 48 || L == 64)) ? L : 0;

@@ -335,8 +335,8 @@ int gbdw_batch_destroy(gbdw_batch* b);
 int gbdw_batch_info(const gbdw_batch* b, int64_t info[4]);
 /* The autotuned shape: shape[0] threads per CTA, shape[1] / shape[2] slices per thread of the
  * FP32 / FP16 instances, shape[3] tile split (each site's Ls*nrhs slices are cut into up to
- * this many contiguous tiles: an Ls tile of some values of s with every right-hand side, or an
- * RHS tile of some right-hand sides at one s). */
+ * this many contiguous tiles: an RHS tile of whole right-hand sides, or an Ls tile of some of one
+ * right-hand side's slices). */
 int gbdw_batch_shape(const gbdw_batch* b, int shape[4]);
 /* Pins a shape (same meaning; threads 64/128, slices per thread 1 or 2, split a power of two)
  * and rebuilds the graph. */
