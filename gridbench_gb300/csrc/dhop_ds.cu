@@ -5,7 +5,7 @@
 // FP64 operator (true residuals of the reliable updates, the FP64 CG) by default and any FP64
 // operator call on request (gbdw_set_fp64_arith).
 #include "dhop_kernel.cuh"
-#include "dsfloat.cuh"
+#include "dspairs.cuh"
 
 namespace gbdw {
 
@@ -60,67 +60,6 @@ int ds_links(const gbdw_gauge* g, const void** out) {
 
 namespace {
 
-// ------------------------------------------------------------------ packed double-single arithmetic
-// A complex number as two FP32 pairs: (re, im) of the leading parts in h and of the trailing parts in
-// l, so that one FADD2 / FMUL2 / FFMA2 serves both components: half the instructions of the scalar
-// form of dsfloat.cuh, the same error-free transformations step by step.
-struct ds2 {
-  float2 h, l;
-};
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }  // exact product
-__device__ __forceinline__ float2 swap2(float2 a) { return make_float2(a.y, a.x); }
-// s + e = a + b exactly (Knuth)
-__device__ __forceinline__ float2 two_sum2(float2 a, float2 b, float2& e) {
-  const float2 s = add2(a, b), bb = sub2(s, a);
-  e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
-  return s;
-}
-// the pair (s, t) renormalised (Dekker)
-__device__ __forceinline__ ds2 join2(float2 s, float2 t) {
-  const float2 h = add2(s, t);
-  return {h, sub2(t, sub2(h, s))};
-}
-// SloppyDWPlusDW
-__device__ __forceinline__ ds2 operator+(ds2 a, ds2 b) {
-  float2 e;
-  const float2 s = two_sum2(a.h, b.h, e);
-  return join2(s, add2(e, add2(a.l, b.l)));
-}
-// One step of a compensated dot product: s + e += a b with s the running sum of the leading products
-// (every rounding error of which goes into e) and e plain FP32; a is the same real for both components
-// up to sign.
-__device__ __forceinline__ void dot2(float2 ah, float2 al, ds2 b, float2& s, float2& e) {
-  const float2 p = __fmul2_rn(ah, b.h);
-  const float2 pe = __ffma2_rn(ah, b.h, make_float2(-p.x, -p.y));  // exact
-  e = __ffma2_rn(ah, b.l, e);
-  e = __ffma2_rn(al, b.h, e);
-  float2 f;
-  s = two_sum2(s, p, f);
-  e = add2(e, add2(pe, f));
-}
-// An FP64 complex number as pairs, with the bits of ds_split: h the leading 24 mantissa bits moved over
-// by integer operations, l the other 29 rounded to 24 and scaled by 2^-52 of h's exponent.
-__device__ __forceinline__ void split1(double d, float& h, float& l) {
-  const unsigned hi = unsigned(__double2hiint(d)), lo = unsigned(__double2loint(d));
-  const unsigned t = __funnelshift_l(lo, hi, 3);
-  const unsigned hb = ((t & 0x7fffffffu) ^ 0x40000000u) | (hi & 0x80000000u);
-  const unsigned ah = hi & 0x7fffffffu;
-  const float scale = __uint_as_float(hb & 0xff800000u) * 2.220446049250313e-16f;
-  h = __uint_as_float(hb);
-  l = __uint2float_rn(lo & 0x1fffffffu) * scale;
-  if (ah - 0x38100000u >= 0x0fe00000u) {  // below 2^-126 (zero) or beyond FP32 (infinity)
-    h = __uint_as_float((hi & 0x80000000u) | (ah < 0x38100000u ? 0u : 0x7f800000u));
-    l = 0.f;
-  }
-}
-__device__ __forceinline__ ds2 split2(double2 a) {
-  float2 h, l;
-  split1(a.x, h.x, l.x);
-  split1(a.y, h.y, l.y);
-  return join2(h, l);
-}
-
 // c y for a unit c known at run time: the components exchanged or not, times a pair of signs
 struct Unit2 {
   bool swap;
@@ -130,7 +69,7 @@ __device__ __forceinline__ Unit2 unit_of(int code) {  // codes of LegSpin
   return {code >= 2, make_float2(code == 1 || code == 2 ? -1.f : 1.f, code == 1 || code == 3 ? -1.f : 1.f)};
 }
 __device__ __forceinline__ ds2 times(const Unit2& c, ds2 y) {
-  return {__fmul2_rn(c.swap ? swap2(y.h) : y.h, c.sign), __fmul2_rn(c.swap ? swap2(y.l) : y.l, c.sign)};
+  return {mul2(c.swap ? swap2(y.h) : y.h, c.sign), mul2(c.swap ? swap2(y.l) : y.l, c.sign)};
 }
 
 // One leg, its direction and side known at run time (and the same for the whole CTA): spins 0 and 1

@@ -1,9 +1,10 @@
 // Double-word ("double-single") arithmetic on pairs of FP32 numbers: a value is h + l with
 // |l| <= ulp(h) / 2, about 48 significant bits (relative rounding ~2^-47), computed on the FP32
 // pipe.  GB300 executes FP64 at 1/64 of its FP32 rate, so the FP64-accurate hopping operator
-// (the solvers' true residuals and the FP64 CG) runs its arithmetic in this form instead of in
-// FP64: FP64 fields are split into pairs as they are loaded and joined back to FP64 as they are
-// stored.
+// (the solvers' true residuals and the FP64 CG) computes with pairs instead of in FP64: FP64 fields
+// are split into pairs as they are loaded and joined back to FP64 as they are stored.  This is the
+// scalar form: the operator's links are split with it, and its sums and products are what the
+// packed form that the operator runs (dspairs.cuh) does for two components at once.
 //
 // The building blocks are the published error-free transformations and double-word
 // algorithms:
