@@ -752,7 +752,7 @@ def run_ours(args, D: Dist) -> dict | None:
         "parallelism": "replicas" if D.world > 1 else "single",
         "launch": {"threads": cfg[0], "slices_per_thread": cfg[1],
                    "form": {0: "direct", 1: "tma-staged (CTA ring)", 2: "tma-staged (warp rings)",
-                            3: "direct (Ls=16 specialised)", 4: "t-sweep over 2x2x2 columns"}[cfg[2]],
+                            3: "direct (registers capped)", 4: "t-sweep over 2x2x2 columns"}[cfg[2]],
                    "stages": cfg[3], "tile_split": gb.tune_split(g, xA), "t_brick": gb.tune_brick(g, xA)},
         "rel_err_vs_fp64": rel,
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",

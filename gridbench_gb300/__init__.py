@@ -481,7 +481,7 @@ def tune_dhop(g: Gauge, out: Field, inp: Field, dag: int = 0) -> tuple:
 
 def tune_query(g: Gauge, inp: Field) -> tuple:
     """(threads per CTA, slices per thread, form, stages); form 0 direct loads, 1 TMA-staged
-    CTA ring, 2 TMA-staged ring per warp, 3 direct FP32/FP16 kernel specialised for Ls*nrhs = 16, 4 site blocks:
+    CTA ring, 2 TMA-staged ring per warp, 3 direct with registers capped (FP32; FP16 with Ls*nrhs = 16), 4 site blocks:
     FP32 2x2x2 columns swept along t (tune_brick: t-slices per CTA), FP16 form 3 over 2x2x2x2 blocks."""
     cfg = (C.c_int * 4)()
     check(load().gbdw_tune_query(g.h, inp.h, cfg))

@@ -331,8 +331,6 @@ struct CgRule {
 // cg_scalars() + CG_RR, the scalars after it are set and all of them copied to the host
 int sum_partials(const double* partials, int64_t n, double* result, double num = 0.0, double* alpha_out = nullptr,
                  const CgRule* rule = nullptr);
-// copies n <= 8 device doubles to the host (synchronising the library stream)
-int fetch_doubles(const double* dev, int n, double* host);
 // the host's copy of a step's scalars in two halves, the first behind the step: work queued between
 // them runs while the host waits
 int cg_scalars_mark();

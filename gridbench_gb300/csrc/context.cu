@@ -266,13 +266,6 @@ int sum_partials(const double* partials, int64_t n, double* result, double num, 
 
 double* cg_scalars() { return (double*)scratch(64, 9); }
 
-int fetch_doubles(const double* dev, int n, double* host) {
-  GBDW_CUDA(cudaMemcpyAsync(g_pinned, dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost, stream()));
-  GBDW_CUDA(cudaStreamSynchronize(stream()));
-  for (int k = 0; k < n; ++k) host[k] = g_pinned[k];
-  return GBDW_OK;
-}
-
 int cg_scalars_mark() {
   if (!g_scalars) GBDW_CUDA(cudaEventCreateWithFlags(&g_scalars, cudaEventDisableTiming));
   GBDW_CUDA(cudaEventRecord(g_scalars, stream()));

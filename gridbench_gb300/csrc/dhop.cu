@@ -86,7 +86,11 @@ bool mobius_fusable(const gbdw_gauge* g, const gbdw_field* in, int dag) {
   const int Ls = g->lat->Ls;
   // the adjoint (A^dag in the epilogue) in every precision; the forward operator (A on the loaded
   // neighbours) on FP32 slice pairs.  Other even Ls: the FP32 adjoint on the warp rings, where a warp
-  // holds whole sites.
+  // holds whole sites, in a shape of its own whatever is tuned or pinned for M: no other form keeps a site's
+  // lanes in one warp there.  It is faster than the hopping term in its best form and the two-operand m5d pass
+  // at every Ls measured, also where lanes idle.  16^4, us, two passes / this: Ls 6 73 / 50, 10 96 / 66, 12 98 /
+  // 69, 14 121 / 81, 18 146 / 96, 20 146 / 94, 22 164 / 119, 24 181 / 119, 30 208 / 131, 34 (17 lanes) 240 / 221,
+  // 36 267 / 222, 48 316 / 226, 62 419 / 248; 8^4 11 to 35 / 9 to 17.
   if (!g->lat->fast || in->nrhs != 1 || in->LsE != in->LsP || Ls < 2 || Ls > 64 || Ls % 2) return false;
   if ((Ls & (Ls - 1)) == 0) return dag || in->prec == GBDW_F32;
   int ns, threads;
@@ -158,8 +162,8 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
   if (ex) p.c5 = ex->c5;
   if (ex && ex->mobius) {
     if (epi != 1 || ex->r || !mobius_fusable(g, in, dag)) {
-      set_error("fused Mobius operator: the M epilogue, one right-hand side, Ls a power of two <= 64, FP32 for "
-                "the forward operator");
+      set_error("fused Mobius operator: the M epilogue, one right-hand side, Ls a power of two <= 64 (FP32 for the "
+                "forward operator) or, for the FP32 adjoint, any even Ls <= 64");
       return GBDW_ERR_INVALID;
     }
     p.mob = 1;
@@ -275,7 +279,7 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
     if (reduce) {
       double* to = (ex && ex->sum_to) ? ex->sum_to : red.result;
       if (int s2 = sum_partials(red.partials, blocks_ds, to, ex ? ex->num : 0.0, ex ? ex->alpha_to : nullptr, ex ? ex->rule : nullptr)) return s2;
-      if (norm2 && fetch) return ex && ex->sum_to ? fetch_doubles(to, 1, norm2) : reduce_fetch(red, 1, norm2);
+      if (norm2 && fetch) return reduce_fetch(red, 1, norm2);
     }
     return GBDW_OK;
   }
@@ -290,7 +294,7 @@ int run_dhop(const gbdw_gauge* g, gbdw_field* out, const gbdw_field* in, int dag
     // the kernel leaves one partial per CTA; one CTA sums them in a fixed order
     double* to = (ex && ex->sum_to) ? ex->sum_to : red.result;
     if (int s2 = sum_partials(red.partials, blocks, to, ex ? ex->num : 0.0, ex ? ex->alpha_to : nullptr, ex ? ex->rule : nullptr)) return s2;
-    if (norm2 && fetch) return ex && ex->sum_to ? fetch_doubles(to, 1, norm2) : reduce_fetch(red, 1, norm2);
+    if (norm2 && fetch) return reduce_fetch(red, 1, norm2);
   }
   return GBDW_OK;
 }

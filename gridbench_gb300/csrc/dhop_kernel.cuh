@@ -473,7 +473,7 @@ struct DhopParams {
   float* r_norm = nullptr;  // EPI 4: FP16 r with per-slice norms
   int rLsP = 0;
   const double* alpha = nullptr;
-  // Mobius operator in one pass (one right-hand side, Ls a power of two <= 64, two slices per
+  // Mobius operator in one pass (mobius_fusable; one right-hand side, two slices per
   // thread): with EPI 1 and DhopDag the hopping result v is replaced by A(mb, mc)^dag v before the
   // M epilogue (Mooee^dag in - khop A(b, c)^dag DhopDag in); with EPI 6 (FP32) A(mb, mc) is
   // applied to the neighbours as they are loaded (Mooee in - khop Dhop A(b, c) in)

@@ -10,7 +10,7 @@
 // (their broadcast 64-bit loads are 43 % of the direct form's L1 wavefronts).
 //
 // 2 x 2 x 2 because each thread then has exactly one outside neighbour per direction, in every
-// warp; four CTAs of 64 threads fit an SM (34 KB and 246 registers a thread).  Hopping term, us,
+// warp; four CTAs of 64 threads fit an SM (34 KB and, at 16 slices, 212 to 255 registers a thread).  Hopping term, us,
 // this form / the best of the others (TMA warp rings or form 3, before launches overlapped) / all bytes once
 // at the copy rate:
 //   16^4 x 8    34 / 49 / 20      24^4 x 8   152 / 215 / 104     24^4 x 12  247 / 287 / 141

@@ -23,9 +23,10 @@
 // Kernels: k_m5d (out = A x [+ B y], one thread per 4D site and N slices, every operand read
 // once: HBM bound, 2 spinors per 5D site per operand) and k_m5d_inv (A^-1 as two cyclic
 // bidiagonal solves per chirality, O(Ls) per row, the same two-phase shared-memory tile as the
-// Shamir D5^-1 in eo.cu).  With one right-hand side and Ls a power of two, M^dag is a single
-// hopping pass in every precision (A(b, c)^dag applied to the hopping result in the epilogue),
-// and so is M for FP32 fields (A(b, c) applied to the neighbours' slices as they are loaded);
+// Shamir D5^-1 in eo.cu).  With one right-hand side and Ls a power of two (FP32: any even Ls), M^dag
+// is a single hopping pass in every precision (A(b, c)^dag applied to the hopping result in the
+// epilogue), and for a power of two so is M for FP32 fields (A(b, c) applied to the neighbours' slices
+// as they are loaded);
 // the neighbouring slices are taken by shuffles from the lanes of the same site (dhop_kernel.cuh).
 #include <cmath>
 #include <string>

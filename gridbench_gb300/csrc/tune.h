@@ -10,13 +10,13 @@ void set_tuned_launch(int gprec, int sprec, int LsE, int epi, DhopLaunch L);
 struct DhopExtra {
   gbdw_field* r = nullptr;          // with epi 1: r -= (*alpha) M(in) instead of storing M(in)
   const double* alpha = nullptr;    // device
-  double* sum_to = nullptr;         // device: where the fused |.|^2 goes (default: the reduce result)
+  double* sum_to = nullptr;         // device: where the fused |.|^2 goes (default: the reduce result, for norm2)
   double num = 0.0;                 // with alpha_to: alpha_to = num / sum
   double* alpha_to = nullptr;       // device
   const CgRule* rule = nullptr;     // with sum_to = cg_scalars() + CG_RR
   double c5 = 1.0;                  // the epilogue's 5th-dimension hopping coefficient
   // Mobius operator in one pass: A(mb, mc) on the loaded neighbours (dag 0, FP32) or A(mb, mc)^dag
-  // on DhopDag in before the epilogue (dag 1); epi 1, one right-hand side, Ls a power of two <= 64
+  // on DhopDag in before the epilogue (dag 1); epi 1, where mobius_fusable
   bool mobius = false;
   double mb = 1.0, mc = 0.0;
   // D5^-1 of the hopping term (dag: D5^-dag) in one pass, with mb = 1 / a5 and mc = 1 / (a5 (1 + mf a5^-Ls));

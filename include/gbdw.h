@@ -356,12 +356,16 @@ int gbdw_tune_load(const char* path);
 int gbdw_tune_save(const char* path);
 /* Writes the chosen shape for a field into cfg[4]: threads per CTA, slices per thread,
  * form (0 direct loads, 1 TMA-staged neighbour blocks with one ring per CTA, 2 the same with
- * one ring per warp, 3 the direct form specialised for FP32/FP16 with Ls*nrhs = 16, 4 site blocks on
+ * one ring per warp, 3 the direct form with registers capped for more CTAs (FP32, any Ls*nrhs, odd
+ * ones in pairs with a padded last one; FP16 with Ls*nrhs = 16), 4 site blocks on
  * periodic lattices: for FP32 2x2x2 columns swept along t (Ls*nrhs a multiple of 8 or 12, even x, y
  * and z), for FP16 form 3 over 2x2x2x2 blocks (even extents)) and stages of the staged forms. */
 int gbdw_tune_query(const gbdw_gauge* g, const gbdw_field* in, int cfg[4]);
 /* Pins the shape for fields like `in` (threads a multiple of 32 up to 256; slices per thread
- * 1, 2 or 4 dividing Ls*nrhs, at most 2 for F64; form 0..4; stages 2/4). */
+ * 1, 2 or 4 dividing Ls*nrhs (2 also for an odd FP32 Ls*nrhs in forms 0 and 3), at most 2 for F64;
+ * form 0..4; stages 2/4).  Two fused passes run shapes of their own where they need a site's lanes in one
+ * warp: the FP32 Mobius adjoint for an even Ls that is no power of two (warp rings), and D5^-1 after the
+ * even-odd hopping term (form 3, unless the t-sweep is chosen). */
 int gbdw_tune_set(const gbdw_gauge* g, const gbdw_field* in, int threads, int spt, int form, int stages);
 /* Ls / RHS tiles of the direct forms (0 and 3): each site's Ls*nrhs slices are cut into `split`
  * contiguous tiles, threads ordered (tile, site, slice group), so each tile is one sweep over all
